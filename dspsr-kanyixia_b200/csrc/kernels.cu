@@ -1,1708 +1,14 @@
-// kernels.cu -- sm_100a kernels of the B200 baseband hot path.
-//
-// Overlap-save coherent dedispersion (Signal/General/Convolution.C:724-803 is
-// the CPU algorithm; CUDA::ConvolutionEngine runs it as cuFFT + 3 kernels per
-// batch) is restructured here as a four-step FFT of length N = n1 * n2:
-//
-//   K1 (columns)  unpack the int8/int16/float input on load, n1-point DFTs in
-//                 registers across the n1 chunks of n2 samples, store rows k1.
-//   K2 (rows)     twiddle w_N^{k1 n2}, n2-point Stockham FFT in shared memory,
-//                 multiply by the response (stored in four-step order), inverse
-//                 n2-point FFT, conjugate twiddle -- one read and one write.
-//   K3 (columns)  inverse n1-point DFTs in registers, overlap discard, and then
-//                 either write the voltages (Engine::perform) or detect and
-//                 fold in the same pass (warp-segmented reduction by bin).
-//
-// For n1 == 1 a single kernel does load, FFT, multiply, inverse FFT and the
-// epilogue entirely in shared memory: one HBM round trip per part.
-//
-// FFT sign conventions are FFTW's (forward -1, backward +1, unnormalised); the
-// 1/sqrt(N) normaliser is folded into the response, as Convolution::prepare
-// does (Convolution.C:401-414).
+// kernels.cu -- response construction and the standalone engines: filterbank,
+// SpectralKurtosis, unpackers, detection, fold (sm_100a)
 
-#include "kernels.cuh"
-#include "fft_core.cuh"
-
-#include <cuda_runtime.h>
-
-#include <algorithm>
-#include <atomic>
+#include "device_common.cuh"
+#include "group_fft.cuh"
 
 namespace b200 {
 
-namespace {
-
-constexpr unsigned FULL = 0xffffffffu;
-
 std::atomic<uint64_t> g_launches {0};
 
-struct ClockScope
-{
-  const KernelClock* c;
-  int kind;
-  cudaStream_t st;
-  ClockScope (const KernelClock* c_, int k, cudaStream_t s) : c (c_), kind (k), st (s)
-  {
-    g_launches++;
-    if (c) c->mark (c->self, kind, 0, st);
-  }
-  ~ClockScope ()
-  {
-    if (c) c->mark (c->self, kind, 1, st);
-  }
-};
-
-// --------------------------------------------------------------------------
-// input fetch (unpack fused into the load)
-// --------------------------------------------------------------------------
-
-template <int KIND>
-__device__ __forceinline__ float2 fetch (const InputView& in, const float* s_lut,
-                                         unsigned c, unsigned p, uint64_t t)
-{
-  const void* base = in.main;
-  uint64_t span = in.main_span;
-  if (t < in.npre)
-    base = in.pre, span = in.pre_span;
-  else
-    t -= in.npre;
-  if constexpr (KIND == IN_INT8)
-  {
-    const uint8_t* b = static_cast<const uint8_t*> (base)
-                       + ((t * in.nchan + c) * in.npol + p) * 2;
-    const unsigned short w = __ldg (reinterpret_cast<const unsigned short*> (b));
-    return make_float2 (s_lut[w & 0xff], s_lut[w >> 8]);
-  }
-  else if constexpr (KIND == IN_INT16)
-  {
-    const int16_t* q = static_cast<const int16_t*> (base)
-                       + ((t * in.nchan + c) * in.npol + p) * 2;
-    const unsigned w = __ldg (reinterpret_cast<const unsigned*> (q));
-    short re = short (w & 0xffff), im = short (w >> 16);
-    if (in.offset_binary)
-    {
-      re = short (re ^ 0x8000);
-      im = short (im ^ 0x8000);
-    }
-    // SixteenBitUnpacker.C:69: float(x) + 0.5 (the double 0.5 rounds to float)
-    return make_float2 (__fadd_rn (float (re), 0.5f), __fadd_rn (float (im), 0.5f));
-  }
-  else
-  {
-    const float2* f = static_cast<const float2*> (base);
-    return __ldg (f + (uint64_t (c) * in.npol + p) * span + t);
-  }
-}
-
-__device__ __forceinline__ void load_lut (const InputView& in, const float* lut, float* s_lut)
-{
-  if (in.kind == IN_INT8)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-      s_lut[i] = lut[i];
-}
-
-// --------------------------------------------------------------------------
-// detection (Detection.C:253-301 Intensity/PPQQ order, cross_detect.ic:38-41,
-// stokes_detect.ic:40-43); explicit _rn arithmetic so that no product is
-// fused into an FMA and every value rounds as the reference's CPU code does.
-// --------------------------------------------------------------------------
-
-__device__ __forceinline__ void detect_values (int state, unsigned npol, float2 p, float2 q,
-                                               float* o)
-{
-  if (state == 0)
-  {
-    float v = __fmul_rn (p.x, p.x);
-    v = __fadd_rn (v, __fmul_rn (p.y, p.y));
-    if (npol == 2)
-    {
-      v = __fadd_rn (v, __fmul_rn (q.x, q.x));
-      v = __fadd_rn (v, __fmul_rn (q.y, q.y));
-    }
-    o[0] = v;
-    return;
-  }
-  const float pp = __fadd_rn (__fmul_rn (p.x, p.x), __fmul_rn (p.y, p.y));
-  const float qq = __fadd_rn (__fmul_rn (q.x, q.x), __fmul_rn (q.y, q.y));
-  if (state == 1)
-  {
-    o[0] = pp;
-    o[1] = qq;
-    return;
-  }
-  const float re = __fadd_rn (__fmul_rn (p.x, q.x), __fmul_rn (p.y, q.y));
-  const float im = __fsub_rn (__fmul_rn (p.x, q.y), __fmul_rn (p.y, q.x));
-  if (state == 2)
-  {
-    o[0] = pp;
-    o[1] = qq;
-    o[2] = re;
-    o[3] = im;
-    return;
-  }
-  o[0] = __fadd_rn (pp, qq);
-  o[1] = __fsub_rn (pp, qq);
-  o[2] = __fmul_rn (2.0f, re);
-  o[3] = __fmul_rn (2.0f, im);
-}
-
-// --------------------------------------------------------------------------
-// fold
-// --------------------------------------------------------------------------
-
-// Index of the plan segment holding sample t (segments are sorted by start).
-__device__ __forceinline__ int seg_search (const FoldSegment* __restrict__ segs, int nseg,
-                                           uint64_t t)
-{
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi)
-  {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg (&segs[mid].start) <= t) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-// Exact bin of plan sample t in segment s (see host_rules.cpp for the algebra):
-// y = (m0 + j*dm) * g in integer arithmetic, then one rounded multiply by nbin.
-__device__ __forceinline__ unsigned seg_bin (const FoldSegment* __restrict__ segs, int s,
-                                             uint64_t t, unsigned nbin)
-{
-  const uint64_t start = __ldg (&segs[s].start);
-  const int64_t m0 = __ldg (&segs[s].m0);
-  const int64_t dm = __ldg (&segs[s].dm);
-  const double g = __ldg (&segs[s].g);
-  const double y = __dmul_rn (double (m0 + int64_t (t - start) * dm), g);
-  return __double2uint_rz (__dmul_rn (y, double (nbin)));
-}
-
-__device__ __forceinline__ unsigned fold_bin (const FoldSegment* __restrict__ segs, int nseg,
-                                              uint64_t t, unsigned nbin)
-{
-  return seg_bin (segs, seg_search (segs, nseg, t), t, nbin);
-}
-
-// Profile columns of a warp whose active lanes hold increasing sample
-// indices: one binary search by the first active lane, then each lane steps
-// forward over the (few) segment boundaries between it and that lane.  The
-// column is the segment's base plus the bin; NO_COLUMN for skipped samples
-// and bins outside [0, nbin).  All 32 lanes call this.
-constexpr unsigned NO_COLUMN = 0xffffffffu;
-__device__ __forceinline__ unsigned warp_fold_bin (const FoldSegment* __restrict__ segs,
-                                                   int nseg, bool ok, uint64_t t, unsigned nbin)
-{
-  const unsigned act = __ballot_sync (FULL, ok);
-  if (!act) return NO_COLUMN;
-  const int leader = __ffs (act) - 1;
-  int s = 0;
-  if ((threadIdx.x & 31) == leader) s = seg_search (segs, nseg, t);
-  s = __shfl_sync (FULL, s, leader);
-  if (!ok) return NO_COLUMN;
-  while (s + 1 < nseg && __ldg (&segs[s + 1].start) <= t) s++;
-  const unsigned base = __ldg (&segs[s].base);
-  const unsigned bin = seg_bin (segs, s, t, nbin);
-  return (base == FOLD_SKIP || bin >= nbin) ? NO_COLUMN : base + bin;
-}
-
-// All 32 lanes call this together.  Lanes holding consecutive time samples
-// with equal bins form runs; each run is summed by a segmented shuffle
-// reduction and added to the profile by its first lane with one atomic.
-template <int NOUT, bool HITS>
-__device__ __forceinline__ void warp_fold_t (bool ok, unsigned bin, const float* v,
-                                             float* prof, unsigned nbin, unsigned* hits)
-{
-  const int lane = threadIdx.x & 31;
-  const unsigned key = ok ? bin : 0xffffffffu;
-  const unsigned prev = __shfl_up_sync (FULL, key, 1);
-  const bool head = (lane == 0) || (prev != key);
-  const unsigned hm = __ballot_sync (FULL, head);
-  const int rid = __popc (hm & (FULL >> (31 - lane)));
-  float acc[NOUT];
-#pragma unroll
-  for (int k = 0; k < NOUT; k++) acc[k] = ok ? v[k] : 0.0f;
-  int cnt = ok ? 1 : 0;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1)
-  {
-    const int orid = __shfl_down_sync (FULL, rid, off);
-    const bool take = (lane + off < 32) && (orid == rid);
-#pragma unroll
-    for (int k = 0; k < NOUT; k++)
-    {
-      const float o = __shfl_down_sync (FULL, acc[k], off);
-      if (take) acc[k] += o;
-    }
-    if constexpr (HITS)
-    {
-      const int oc = __shfl_down_sync (FULL, cnt, off);
-      if (take) cnt += oc;
-    }
-  }
-  if (head && ok)
-  {
-#pragma unroll
-    for (int k = 0; k < NOUT; k++)
-      atomicAdd (prof + uint64_t (k) * nbin + bin, acc[k]);
-    if constexpr (HITS) atomicAdd (hits + bin, unsigned (cnt));
-  }
-}
-
-// Only the warps that count hits (one channel's) reduce the counts; hits is
-// the same pointer in every lane, so the choice is warp-uniform.
-template <int NOUT>
-__device__ __forceinline__ void warp_fold (bool ok, unsigned bin, const float* v,
-                                           float* prof, unsigned nbin, unsigned* hits)
-{
-  if (hits)
-    warp_fold_t<NOUT, true> (ok, bin, v, prof, nbin, hits);
-  else
-    warp_fold_t<NOUT, false> (ok, bin, v, prof, nbin, hits);
-}
-
-template <int NOUT>
-__device__ __forceinline__ void emit_fold (const FoldView& fv, unsigned c, unsigned npol, bool ok,
-                                           uint64_t t, float2 p, float2 q)
-{
-  // a warp whose samples all fall in the overlap discard has nothing to add
-  // (all 32 lanes are here, so the vote and the return are warp-uniform)
-  if (!__any_sync (FULL, ok)) return;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-  unsigned bin = fv.cols ? (ok ? __ldg (fv.cols + t) : NO_COLUMN)
-                         : warp_fold_bin (fv.segs, fv.nseg, ok, t, fv.nbin);
-  if (ok)
-  {
-    detect_values (fv.state, npol, p, q, v);
-    ok = bin < fv.stride;
-  }
-  warp_fold<NOUT> (ok, bin, v, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride,
-                   c == 0 ? fv.hits : nullptr);
-}
-
-// --------------------------------------------------------------------------
-// shared-memory Stockham FFT
-// --------------------------------------------------------------------------
-
-template <int N, int T, int D, int P>
-__device__ __forceinline__ void smem_pass (float2* s, float2* v, const float2* tw)
-{
-  if constexpr (P < stockham_npass (N))
-  {
-    constexpr int R = stockham_radix (N, P);
-    constexpr int Ns = stockham_ns (N, P);
-    StockhamPass<N, R, T, D>::load (threadIdx.x, s, v);
-    __syncthreads ();
-    StockhamPass<N, R, T, D>::compute_store (threadIdx.x, Ns, v, s, tw);
-    __syncthreads ();
-    smem_pass<N, T, D, P + 1> (s, v, tw);
-  }
-}
-
-// N-point FFT of s[spad(0..N-1)] in place; the caller has synchronised after
-// writing s.  Returns synchronised.
-template <int N, int T, int D>
-__device__ __forceinline__ void smem_fft (float2* s, const float2* tw)
-{
-  float2 v[N / T];
-  smem_pass<N, T, D, 0> (s, v, tw);
-}
-
-// --------------------------------------------------------------------------
-// K1: forward column DFTs with the unpack fused into the load
-// --------------------------------------------------------------------------
-
-// columns per 128-thread block: one thread per column, two at n1 = 32
-template <int N1>
-constexpr unsigned fwd_cols_per_block ()
-{
-  return N1 == 32 ? 64u : 128u;
-}
-
-template <int N1, int KIND>
-__global__ void __launch_bounds__ (128, 2)
-k_fwd_cols (const InputView in, const float* __restrict__ lut, const uint64_t nkeep,
-            const uint64_t part0, const unsigned n2, const float2* __restrict__ tw4,
-            float2* __restrict__ scratch, const float* __restrict__ apod)
-{
-  __shared__ float s_lut[256];
-  load_lut (in, lut, s_lut);
-  __syncthreads ();
-  const unsigned b = blockIdx.y;
-  const unsigned c = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * n2;
-  if constexpr (N1 == 32)
-  {
-    // Two threads per column (a 32-point DFT in one thread's registers
-    // spills): thread h of the pair takes rows 2m + h, a 16-point DFT of
-    // them gives E (h = 0) or O (h = 1), thread 1 applies w32^j, and one
-    // exchange gives X[j] = E[j] + w32^j O[j] to thread 0 and
-    // X[j + 16] = E[j] - w32^j O[j] to thread 1.
-    const unsigned h = threadIdx.x & 1;
-    const unsigned i2 = blockIdx.x * 64 + (threadIdx.x >> 1);
-    const uint64_t t0 = (part0 + b) * nkeep + i2;
-    for (unsigned p = 0; p < in.npol; p++)
-    {
-      float2 v[16];
-#pragma unroll
-      for (int m = 0; m < 16; m++)
-        v[m] = fetch<KIND> (in, s_lut, c, p, t0 + uint64_t (2 * m + h) * n2);
-      if (apod)
-      {
-        // Apodization::operate on the part before the forward FFT (Convolution.C:739-743)
-#pragma unroll
-        for (int m = 0; m < 16; m++)
-        {
-          const float w = __ldg (apod + uint64_t (2 * m + h) * n2 + i2);
-          v[m] = make_float2 (__fmul_rn (v[m].x, w), __fmul_rn (v[m].y, w));
-        }
-      }
-      RegDFT<16, -1>::run (v);
-#pragma unroll
-      for (int j = 0; j < 16; j++)
-      {
-        const float2 mine = h ? tw_mul<32, -1> (j, v[j]) : v[j];
-        const float2 other = make_float2 (__shfl_xor_sync (0xffffffffu, mine.x, 1),
-                                          __shfl_xor_sync (0xffffffffu, mine.y, 1));
-        // thread 0: E + O'; thread 1: E - O' (E is the partner's value)
-        v[j] = h ? csub (other, mine) : cadd (mine, other);
-      }
-      const unsigned k0 = 16 * h;
-      float2* dst = scratch + ((uint64_t (b) * in.nchan + c) * in.npol + p) * N + i2;
-#pragma unroll
-      for (int j = 0; j < 16; j++)
-      {
-        const unsigned k1 = k0 + j;
-        float2 y = v[j];
-        // four-step twiddle w_N^{k1 n2} (row k1 of the [n1][n2] table)
-        if (k1) y = cmul (y, __ldg (tw4 + uint64_t (k1) * n2 + i2));
-        dst[uint64_t (k1) * n2] = y;
-      }
-    }
-    return;
-  }
-  const unsigned i2 = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t t0 = (part0 + b) * nkeep + i2;
-  for (unsigned p = 0; p < in.npol; p++)
-  {
-    float2 v[N1];
-#pragma unroll
-    for (int k = 0; k < N1; k++)
-      v[k] = fetch<KIND> (in, s_lut, c, p, t0 + uint64_t (k) * n2);
-    if (apod)
-    {
-      // Apodization::operate on the part before the forward FFT (Convolution.C:739-743)
-#pragma unroll
-      for (int k = 0; k < N1; k++)
-      {
-        const float w = __ldg (apod + uint64_t (k) * n2 + i2);
-        v[k] = make_float2 (__fmul_rn (v[k].x, w), __fmul_rn (v[k].y, w));
-      }
-    }
-    RegDFT<N1, -1>::run (v);
-    // four-step twiddle w_N^{k1 n2} (row k1 of the [n1][n2] table; coalesced)
-#pragma unroll
-    for (int k = 1; k < N1; k++)
-      v[k] = cmul (v[k], __ldg (tw4 + uint64_t (k) * n2 + i2));
-    float2* dst = scratch + ((uint64_t (b) * in.nchan + c) * in.npol + p) * N + i2;
-#pragma unroll
-    for (int k = 0; k < N1; k++)
-      dst[uint64_t (k) * n2] = v[k];
-  }
-}
-
-// --------------------------------------------------------------------------
-// K1 with the filterbank in front (Filterbank with freq_res 1 and 64 channels,
-// FilterbankEngineCPU.C:379-535, then the first four-step pass of each
-// channel's convolution), for raw TFPD input of one channel and two
-// polarisations and n1 = 8.  The filterbank's own output never reaches
-// memory: a warp takes one column i2 of one part and computes, for the eight
-// filterbank samples t0 + j*n2 of that column, all 64 channels of both
-// polarisations, then each channel's 8-point column DFT.
-//
-// Lane (j, q), j = lane/4, q = lane%4, reads raw samples s = q + 4m (m < 16)
-// of filterbank sample j: a 16-point DFT over m and the twiddle w64^(q ka)
-// give Y[q][ka] (ka < 16).  One transpose through the warp's shared buffer
-// hands lane 2 ka + pol the 32 values Y[q][ka] of every (q, j): 4-point DFTs
-// over q give channels c = ka + 16 kb (kb < 4) of each filterbank sample,
-// and 8-point DFTs over j the four channels' column DFTs, all in registers
-// (64-point DFT as 16 x 4, X[ka + 16 kb] = sum_q w4^(q kb) w64^(q ka)
-// Y[q][ka]).  The block's four warps (four consecutive
-// columns) stage their outputs in shared memory and write each scratch row
-// in runs of one 32-byte sector (blocks of two or eight warps measured
-// slower).  The transpose's rows are 34 float2 apart, so its stores (one row,
-// 32 lanes) and 16-byte loads (32 rows) are free of bank conflicts.  The staging is column-major with the even and odd rows in two
-// halves (row -> row/2 + (row odd) FBC_SODD, column stride FBC_SP = 2 mod 16):
-// the 16 rows a half-warp stores (two apart) and the 4 x 4 (row, column)
-// pairs it loads for the write-out then fall in 16 distinct bank pairs.
-// --------------------------------------------------------------------------
-
-constexpr int FBC_THREADS = 128;
-constexpr int FBC_COLS = FBC_THREADS / 32;      // columns per block, one per warp
-constexpr int FBC_XROW = 34;                    // exchange row stride (float2; 16-byte reads)
-constexpr int FBC_XSTRIDE = 32 * FBC_XROW;      // float2 per warp exchange buffer
-constexpr int FBC_SODD = 520;                   // staging offset of the odd rows (8 mod 16)
-constexpr int FBC_SP = 1042;                    // staging column stride (2 mod 16)
-constexpr size_t FBC_SMEM =
-    (size_t (FBC_SP) * FBC_COLS > size_t (FBC_COLS) * FBC_XSTRIDE ? size_t (FBC_SP) * FBC_COLS
-                                                                  : size_t (FBC_COLS) * FBC_XSTRIDE)
-    * sizeof (float2);
-
-__host__ __device__ constexpr int fbc_stage (int row, int col)
-{
-  return col * FBC_SP + (row >> 1) + (row & 1) * FBC_SODD;
-}
-
-// (float(x) + 0.5f) * scale for the two's-complement byte x, bit for bit:
-// 2^22 + (x + 128) has its last mantissa bit worth 0.5, so subtracting
-// 2^22 + 127.5 leaves x + 0.5 exactly; no int -> float conversion
-__device__ __forceinline__ float unpack_affine (unsigned byte, float scale)
-{
-  const float big = __int_as_float (0x4a800000u | (((byte & 0xffu) ^ 0x80u) << 1));
-  return __fmul_rn (__fsub_rn (big, 4194431.5f), scale);
-}
-
-// The 8-bit table of the fused filterbank pass is one 1 KB copy in shared
-// memory.  Eight interleaved copies (lane l reading copy l % 8, so a warp's
-// random lookups spread over all banks) measured 10 % slower on the C2 pass:
-// the 8 KB table costs more in occupancy than the bank conflicts it removes.
-
-template <int KIND, bool AFFINE>
-__device__ __forceinline__ void fetch_raw2 (const InputView& in, const float* s_lut, uint64_t r,
-                                            float2& p0, float2& p1)
-{
-  const void* base = in.main;
-  const uint64_t npre = in.npre * 64;
-  if (r < npre)
-    base = in.pre;
-  else
-    r -= npre;
-  if constexpr (KIND == IN_INT8)
-  {
-    const unsigned w = __ldg (static_cast<const unsigned*> (base) + r);
-    if constexpr (AFFINE)
-    {
-      const float sc = in.lut_scale;
-      p0 = make_float2 (unpack_affine (w, sc), unpack_affine (w >> 8, sc));
-      p1 = make_float2 (unpack_affine (w >> 16, sc), unpack_affine (w >> 24, sc));
-    }
-    else
-    {
-      p0 = make_float2 (s_lut[w & 0xff], s_lut[(w >> 8) & 0xff]);
-      p1 = make_float2 (s_lut[(w >> 16) & 0xff], s_lut[w >> 24]);
-    }
-  }
-  else
-  {
-    const uint2 w = __ldg (static_cast<const uint2*> (base) + r);
-    short a = short (w.x & 0xffff), b = short (w.x >> 16);
-    short c = short (w.y & 0xffff), d = short (w.y >> 16);
-    if (in.offset_binary)
-    {
-      a = short (a ^ 0x8000);
-      b = short (b ^ 0x8000);
-      c = short (c ^ 0x8000);
-      d = short (d ^ 0x8000);
-    }
-    p0 = make_float2 (__fadd_rn (float (a), 0.5f), __fadd_rn (float (b), 0.5f));
-    p1 = make_float2 (__fadd_rn (float (c), 0.5f), __fadd_rn (float (d), 0.5f));
-  }
-}
-
-template <int KIND, bool AFFINE>
-__global__ void __launch_bounds__ (FBC_THREADS, 768 / FBC_THREADS)
-k_fwd_cols_fb64 (const InputView in, const float* __restrict__ lut, const uint64_t nkeep,
-                 const uint64_t part0, const unsigned n2, const float2* __restrict__ tw4,
-                 float2* __restrict__ scratch)
-{
-  extern __shared__ __align__ (16) float2 s_fbc[];
-  __shared__ float s_lut[AFFINE ? 1 : 256];
-  __shared__ float2 s_tw64[64];
-  if (!AFFINE && in.kind == IN_INT8)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-      s_lut[i] = lut[i];
-  if (threadIdx.x < 64)
-    s_tw64[threadIdx.x] = make_float2 (cos64 (int (threadIdx.x)), -sin64 (int (threadIdx.x)));
-  __syncthreads ();
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned j = lane >> 2, q = lane & 3;
-  const unsigned i0 = blockIdx.x * FBC_COLS;
-  const unsigned i2 = i0 + warp;
-  const unsigned b = blockIdx.y;
-  const uint64_t N = 8ull * n2;
-  float2* xb = s_fbc + warp * FBC_XSTRIDE;
-
-  // raw samples q + 4m of filterbank sample t, both polarisations
-  const uint64_t t = (part0 + b) * nkeep + i2 + uint64_t (j) * n2;
-  float2 x0[16], x1[16];
-#pragma unroll
-  for (int m = 0; m < 16; m++)
-    fetch_raw2<KIND, AFFINE> (in, s_lut, t * 64 + q + 4 * m, x0[m], x1[m]);
-  RegDFT<16, -1>::run (x0);
-  RegDFT<16, -1>::run (x1);
-  // twiddle w64^(q ka); lane (j, q) then hands Y[q][ka] of both
-  // polarisations to lane 2 ka + pol through the warp's buffer (row 2 ka + pol,
-  // column 4 j + q, rows FBC_XROW float2 apart)
-#pragma unroll
-  for (int ka = 0; ka < 16; ka++)
-  {
-    const float2 w = s_tw64[(q * ka) & 63];
-    xb[(2 * ka) * FBC_XROW + lane] = cmul (x0[ka], w);
-    xb[(2 * ka + 1) * FBC_XROW + lane] = cmul (x1[ka], w);
-  }
-  __syncwarp ();
-  // lane 2 ka + pol reads its row in 16-byte pairs: z[jj][qq] = Y[qq][ka] of
-  // filterbank sample jj
-  float2 z[8][4];
-#pragma unroll
-  for (int jj = 0; jj < 8; jj++)
-#pragma unroll
-    for (int qq = 0; qq < 4; qq += 2)
-    {
-      const float4 t = *reinterpret_cast<const float4*> (xb + lane * FBC_XROW + 4 * jj + qq);
-      z[jj][qq] = make_float2 (t.x, t.y);
-      z[jj][qq + 1] = make_float2 (t.z, t.w);
-    }
-  // 4-point DFTs over q: z[jj][kb] = channel ka + 16 kb of filterbank sample jj
-#pragma unroll
-  for (int jj = 0; jj < 8; jj++) RegDFT<4, -1>::run (z[jj]);
-  // the column DFTs over the eight filterbank samples, per channel
-  float2 col[4][8];
-#pragma unroll
-  for (int kb = 0; kb < 4; kb++)
-  {
-#pragma unroll
-    for (int jj = 0; jj < 8; jj++) col[kb][jj] = z[jj][kb];
-    RegDFT<8, -1>::run (col[kb]);
-  }
-  // four-step twiddle w_N^(k1 n2) of column i2, and the filterbank
-  // normaliser 1/sqrt(64) (exact)
-  float2 tw[8];
-  tw[0] = make_float2 (1.f, 0.f);
-#pragma unroll
-  for (int k1 = 1; k1 < 8; k1++) tw[k1] = __ldg (tw4 + uint64_t (k1) * n2 + i2);
-  __syncthreads ();                    // every warp is done with its exchange buffer
-  // channel c = ka + 16 kb, pol of lane 2 ka + pol; staging row
-  // k1*128 + c*2 + pol, column = warp
-  {
-    const unsigned ka = lane >> 1, pol = lane & 1;
-#pragma unroll
-    for (int kb = 0; kb < 4; kb++)
-    {
-      const unsigned c = ka + 16 * kb;
-#pragma unroll
-      for (int k1 = 0; k1 < 8; k1++)
-      {
-        float2 o = k1 ? cmul (col[kb][k1], tw[k1]) : col[kb][k1];
-        o = make_float2 (__fmul_rn (o.x, 0.125f), __fmul_rn (o.y, 0.125f));
-        s_fbc[fbc_stage (k1 * 128 + c * 2 + pol, warp)] = o;
-      }
-    }
-  }
-  __syncthreads ();
-  // scratch row ((b*64 + c)*2 + pol)*N + k1*n2, columns i0 .. i0+FBC_COLS-1
-#pragma unroll 4
-  for (unsigned idx = threadIdx.x; idx < 1024 * FBC_COLS; idx += FBC_THREADS)
-  {
-    const unsigned row = idx / FBC_COLS, w = idx % FBC_COLS;
-    const unsigned k1 = row >> 7, c = (row & 127) >> 1, pol = row & 1;
-    scratch[((uint64_t (b) * 64 + c) * 2 + pol) * N + uint64_t (k1) * n2 + i0 + w] =
-        s_fbc[fbc_stage (row, w)];
-  }
-}
-
-// --------------------------------------------------------------------------
-// K2 (persistent): the rows.  Row r holds n2 contiguous values,
-// r = ((b*nchan + c)*npol + p)*n1 + k1.
-// --------------------------------------------------------------------------
-
-template <int N, int D, int P, bool PI, bool PO>
-__device__ __forceinline__ void tpass (const float2* src, float2* dst, float2* v,
-                                       const float2* tab)
-{
-  if constexpr (P < stockham_npass (N))
-  {
-    constexpr int T = stockham_threads (N);
-    constexpr int R = stockham_radix (N, P);
-    constexpr int Ns = stockham_ns (N, P);
-    StockhamPassT<N, R, T, D, PI, PO>::load (threadIdx.x, src, v);
-    __syncthreads ();
-    StockhamPassT<N, R, T, D, PI, PO>::compute_store (
-        threadIdx.x, Ns, v, dst, P ? tab + pass_table_offset (N, P) : nullptr);
-    __syncthreads ();
-  }
-}
-
-// read-only load kept in L1 ahead of other lines (reused by later rows)
-__device__ __forceinline__ float2 ldg_evict_last (const float2* p)
-{
-  float2 v;
-  asm volatile ("ld.global.nc.L1::evict_last.v2.f32 {%0, %1}, [%2];"
-                : "=f"(v.x), "=f"(v.y)
-                : "l"(p));
-  return v;
-}
-
-// L2 prefetch of a global range (16-byte aligned, multiple of 16 bytes)
-__device__ __forceinline__ void prefetch_l2 (const void* p, unsigned bytes)
-{
-  asm volatile ("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-template <int N2>
-constexpr size_t rows32_smem_bytes ()
-{
-  return size_t (spad_size (N2) + Row32<N2>::TABN) * sizeof (float2);
-}
-
-// CTAs of k_rows32 resident per SM: at 8192 shared memory (one padded row +
-// 10 KB of twiddles) and 128 registers per thread allow two; at 4096 three
-// (four would cap the registers at 128, where the 4096-point schedule spills).
-// A 30 KB pass-2 table shared by a thread's two butterflies (fewer
-// instructions) measured slower: 208 KB of shared memory per SM leaves too
-// little L1 for the rows' global loads.  So did one CTA per SM running two
-// row groups with named barriers on alternate rows of one run (sharing one
-// response row in L1): 1.91 against 1.78 ms per C2 step.
-template <int N2>
-constexpr unsigned rows32_ctas_per_sm ()
-{
-  return N2 == 8192 ? 2u : 3u;
-}
-
-// The convolution row (CONV: forward FFT, x H, inverse FFT; otherwise the
-// inverse FFT alone, for the inverse filterbank's stitched spectra) with 32
-// points per thread in three radix passes each way (Row32): pass 0 reads the
-// row straight from the scratch in natural order, the forward pass 2, the
-// response multiply and the inverse pass 0 run in registers, the last pass
-// writes the row back in natural order.  One padded row of shared memory per
-// CTA, used in place; several CTAs per SM overlap one another's
-// barrier-separated phases.  The next row (and its response) is prefetched
-// into L2 while this one is transformed.
-template <int N2, bool CONV>
-__global__ void __launch_bounds__ (Row32<N2>::T, rows32_ctas_per_sm<N2> ())
-k_rows32 (float2* scratch, const float2* __restrict__ H, const unsigned n1,
-          const unsigned nchan, const unsigned npol, const unsigned nrows, const unsigned inner)
-{
-  using RS = Row32<N2>;
-  constexpr unsigned ROW_BYTES = N2 * sizeof (float2);
-  constexpr unsigned CHUNK = 16384;
-  extern __shared__ __align__ (16) float2 s_row32[];
-  float2* work = s_row32;
-  float2* tab1 = work + spad_size (N2);
-  float2* th = tab1 + RS::TAB1;
-  float2* tl = th + RS::TABH;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < RS::TABN; i += RS::T) tab1[i] = RS::table_entry (i);
-
-  // Rows are walked with their response row (channel, k1) outermost and the
-  // parts and polarisations innermost (inner = parts x polarisations), and
-  // each CTA takes a contiguous run of that order: the rows of one response
-  // row follow each other on one SM, which keeps the response in its L1
-  // (loaded evict-last, the streamed rows evict-first).
-  const auto row_of = [=] (unsigned idx, unsigned& hrow) {
-    hrow = idx / inner;                             // c * n1 + k1
-    const unsigned bp = idx % inner;
-    return ((bp / npol) * nchan * n1 + hrow / n1 * n1) * npol + (bp % npol) * n1 + hrow % n1;
-  };
-  float2 v[32];
-  const unsigned run = (nrows + gridDim.x - 1) / gridDim.x;
-  const unsigned idx_end = min (nrows, (blockIdx.x + 1) * run);
-  for (unsigned idx = blockIdx.x * run; idx < idx_end; idx++)
-  {
-    unsigned hrow = 0;
-    const unsigned row = CONV ? row_of (idx, hrow) : idx;
-    float2* grow = scratch + uint64_t (row) * N2;
-    const unsigned next = idx + 1;
-    if (tid == 0 && next < idx_end)
-    {
-      unsigned nh = 0;
-      const unsigned nrow = CONV ? row_of (next, nh) : next;
-      const char* nr = reinterpret_cast<const char*> (scratch + uint64_t (nrow) * N2);
-      for (unsigned o = 0; o < ROW_BYTES; o += CHUNK) prefetch_l2 (nr + o, CHUNK);
-      if (CONV && nh != hrow)
-      {
-        const char* hp = reinterpret_cast<const char*> (H + uint64_t (nh) * N2);
-        for (unsigned o = 0; o < ROW_BYTES; o += CHUNK) prefetch_l2 (hp + o, CHUNK);
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < 2; b++)
-#pragma unroll
-      for (int r = 0; r < 16; r++) v[16 * b + r] = __ldcs (grow + tid + b * RS::T + r * RS::NS2);
-    __syncthreads ();     // the previous row's last shared-memory reads are done
-    if constexpr (CONV)
-    {
-      RS::template p0_compute_store<-1> (tid, v, work);
-      __syncthreads ();
-      RS::p1_load (tid, work, v);
-      __syncthreads ();
-      RS::template p1_compute_store<-1> (tid, v, work, tab1);
-      __syncthreads ();
-      RS::p2_load (tid, work, v);
-      __syncthreads ();
-      RS::template p2_compute<-1> (tid, v, th, tl);
-      // Response::operate (Response.C:662-726): (f_r d_r - f_i d_i, f_i d_r + f_r d_i)
-      const float2* h = H + uint64_t (hrow) * N2;
-#pragma unroll
-      for (int b = 0; b < 2; b++)
-#pragma unroll
-        for (int r = 0; r < 16; r++)
-        {
-          const float2 d = v[16 * b + r];
-          const float2 f = ldg_evict_last (h + tid + b * RS::T + r * RS::NS2);
-          v[16 * b + r] = make_float2 (d.x * f.x - d.y * f.y, d.x * f.y + d.y * f.x);
-        }
-    }
-    RS::template p0_compute_store<+1> (tid, v, work);
-    __syncthreads ();
-    RS::p1_load (tid, work, v);
-    __syncthreads ();
-    RS::template p1_compute_store<+1> (tid, v, work, tab1);
-    __syncthreads ();
-    RS::p2_load (tid, work, v);
-    RS::template p2_compute<+1> (tid, v, th, tl);
-    RS::p2_store (tid, v, grow);
-  }
-}
-
-// --------------------------------------------------------------------------
-// K3: inverse column DFTs, overlap discard, voltage out or detect + fold
-// --------------------------------------------------------------------------
-
-// One column of an inverse four-step pass: N1 values stride apart, the
-// conjugate twiddles tw[k*tw_stride], then the N1-point inverse DFT.
-template <int N1>
-__device__ __forceinline__ void inv_column (const float2* __restrict__ src, uint64_t stride,
-                                            const float2* __restrict__ tw, unsigned tw_stride,
-                                            float2* v)
-{
-#pragma unroll
-  for (int k = 0; k < N1; k++)
-    v[k] = src[uint64_t (k) * stride];
-#pragma unroll
-  for (int k = 1; k < N1; k++)
-    v[k] = cmulc (v[k], __ldg (tw + uint64_t (k) * tw_stride));
-  RegDFT<N1, +1>::run (v);
-}
-
-// Two polarisations of 16 or 32 values each do not fit in registers beside
-// the DFT's temporaries: the first waits in shared memory (one slot per
-// thread, so no barrier) while the second is transformed.
-template <int N1, int NPOL>
-__host__ __device__ constexpr bool stage_first_pol () { return NPOL == 2 && N1 >= 16; }
-
-template <int N1, int NPOL, int MODE, int NOUT>
-__global__ void __launch_bounds__ (128, N1 >= 32 ? 3 : 4)
-k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigned nchan,
-            const uint64_t nkeep, const unsigned nfilt_pos, const uint64_t part0,
-            const float2* __restrict__ tw4, const FoldView fv, const VoltView vv)
-{
-  const unsigned b = blockIdx.y;
-  const unsigned c = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * n2;
-  const uint64_t tbase0 = (part0 + b) * nkeep;
-  if constexpr (N1 == 32)
-  {
-    // Two threads per column (16 columns per warp): thread h = lane & 1 of a
-    // pair takes rows 2m + h, a 16-point inverse DFT of them gives E (h = 0)
-    // or O (h = 1), thread 1 applies w32^j, one exchange leaves
-    // X[j] = E[j] + w32^j O[j] with thread 0 and X[j + 16] = E[j] - w32^j O[j]
-    // with thread 1; a second shuffle moves them so that lanes 0..15 hold
-    // X[j] of the warp's 16 columns and lanes 16..31 X[j + 16] (runs of
-    // consecutive samples for the fold).
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned h = lane & 1;
-    const unsigned colw = blockIdx.x * 64 + (threadIdx.x >> 5) * 16;
-    const unsigned i2 = colw + (lane >> 1);
-    float2 v[NPOL][16];
-#pragma unroll
-    for (int m = 0; m < 16; m++)
-    {
-      const unsigned k = 2 * m + h;
-      const float2 w = __ldg (tw4 + uint64_t (k) * n2 + i2);
-#pragma unroll
-      for (int p = 0; p < NPOL; p++)
-      {
-        const float2 x = scratch[((uint64_t (b) * nchan + c) * NPOL + p) * N + uint64_t (k) * n2 + i2];
-        v[p][m] = k ? cmulc (x, w) : x;
-      }
-    }
-    const int srcl = lane < 16 ? 2 * int (lane) : 2 * (int (lane) - 16) + 1;
-#pragma unroll
-    for (int p = 0; p < NPOL; p++)
-    {
-      RegDFT<16, +1>::run (v[p]);
-#pragma unroll
-      for (int j = 0; j < 16; j++)
-      {
-        const float2 mine = h ? tw_mul<32, +1> (j, v[p][j]) : v[p][j];
-        const float2 other = make_float2 (__shfl_xor_sync (FULL, mine.x, 1),
-                                          __shfl_xor_sync (FULL, mine.y, 1));
-        const float2 x = h ? csub (other, mine) : cadd (mine, other);
-        v[p][j] = make_float2 (__shfl_sync (FULL, x.x, srcl), __shfl_sync (FULL, x.y, srcl));
-      }
-    }
-    const unsigned ocol = colw + (lane & 15), koff = 16 * (lane >> 4);
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-    {
-      const uint64_t tl = uint64_t (koff + j) * n2 + ocol;
-      const bool ok = tl >= nfilt_pos && tl < nfilt_pos + nkeep;
-      const uint64_t t = tbase0 + (tl - nfilt_pos);
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        if (ok)
-        {
-#pragma unroll
-          for (int p = 0; p < NPOL; p++)
-            vv.out[(uint64_t (c) * NPOL + p) * vv.span + t] = v[p][j];
-        }
-      }
-      else
-        emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][j], v[NPOL - 1][j]);
-    }
-    return;
-  }
-  const unsigned i2 = blockIdx.x * blockDim.x + threadIdx.x;
-  if constexpr (stage_first_pol<N1, NPOL> ())
-
-  {
-    __shared__ float2 s0[N1 * 128];
-    const float2* src = scratch + (uint64_t (b) * nchan + c) * 2 * N + i2;
-    {
-      float2 v[N1];
-      inv_column<N1> (src, n2, tw4 + i2, n2, v);
-#pragma unroll
-      for (int k = 0; k < N1; k++) s0[k * 128 + threadIdx.x] = v[k];
-    }
-    float2 q[N1];
-    inv_column<N1> (src + N, n2, tw4 + i2, n2, q);
-#pragma unroll (N1 >= 32 ? 2 : N1)
-    for (int k = 0; k < N1; k++)
-    {
-      const uint64_t tl = uint64_t (k) * n2 + i2;
-      const bool ok = tl >= nfilt_pos && tl < nfilt_pos + nkeep;
-      const uint64_t t = tbase0 + (tl - nfilt_pos);
-      const float2 p = s0[k * 128 + threadIdx.x];
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        if (ok)
-        {
-          vv.out[(uint64_t (c) * 2) * vv.span + t] = p;
-          vv.out[(uint64_t (c) * 2 + 1) * vv.span + t] = q[k];
-        }
-      }
-      else
-        emit_fold<NOUT> (fv, c, 2, ok, t, p, q[k]);
-    }
-    return;
-  }
-  float2 w[N1];
-#pragma unroll
-  for (int k = 1; k < N1; k++)
-    w[k] = __ldg (tw4 + uint64_t (k) * n2 + i2);
-  float2 v[NPOL][N1];
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
-  {
-    const float2* src = scratch + ((uint64_t (b) * nchan + c) * NPOL + p) * N + i2;
-#pragma unroll
-    for (int k = 0; k < N1; k++)
-      v[p][k] = src[uint64_t (k) * n2];
-    // conjugate four-step twiddle, then the inverse n1-point DFT
-#pragma unroll
-    for (int k = 1; k < N1; k++)
-      v[p][k] = cmulc (v[p][k], w[k]);
-    RegDFT<N1, +1>::run (v[p]);
-  }
-  const uint64_t tbase = (part0 + b) * nkeep;
-#pragma unroll
-  for (int k = 0; k < N1; k++)
-  {
-    const uint64_t tl = uint64_t (k) * n2 + i2;
-    const bool ok = tl >= nfilt_pos && tl < nfilt_pos + nkeep;
-    const uint64_t t = tbase + (tl - nfilt_pos);
-    if constexpr (MODE == OUT_VOLTAGE)
-    {
-      if (ok)
-      {
-#pragma unroll
-        for (int p = 0; p < NPOL; p++)
-          vv.out[(uint64_t (c) * NPOL + p) * vv.span + t] = v[p][k];
-      }
-    }
-    else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][k], v[NPOL - 1][k]);
-  }
-}
-
-// --------------------------------------------------------------------------
-// single-kernel path (n1 == 1): everything in shared memory
-// --------------------------------------------------------------------------
-
-template <int N, int T, int KIND, int MODE, int NOUT>
-__global__ void __launch_bounds__ (T, 512 / T)
-k_fused (const InputView in, const float* __restrict__ lut, const float2* __restrict__ tw,
-         const float2* __restrict__ H, const uint64_t nkeep, const unsigned nfilt_pos,
-         const uint64_t part0, const FoldView fv, const VoltView vv,
-         const float* __restrict__ apod)
-{
-  extern __shared__ float2 s[];
-  __shared__ float s_lut[256];
-  constexpr int SP = spad_size (N);
-  const unsigned b = blockIdx.x;
-  const unsigned c = blockIdx.y;
-  const uint64_t part = part0 + b;
-  const unsigned npol = in.npol;
-  load_lut (in, lut, s_lut);
-  __syncthreads ();
-  for (unsigned p = 0; p < npol; p++)
-    for (int i = threadIdx.x; i < N; i += T)
-    {
-      float2 x = fetch<KIND> (in, s_lut, c, p, part * nkeep + i);
-      if (apod)
-      {
-        const float w = __ldg (apod + i);
-        x = make_float2 (__fmul_rn (x.x, w), __fmul_rn (x.y, w));
-      }
-      s[p * SP + spad (i)] = x;
-    }
-  __syncthreads ();
-  const float2* h = H + uint64_t (c) * N;
-  for (unsigned p = 0; p < npol; p++)
-  {
-    float2* sp = s + p * SP;
-    smem_fft<N, T, -1> (sp, tw);
-    for (int i = threadIdx.x; i < N; i += T)
-    {
-      const float2 d = sp[spad (i)];
-      const float2 f = __ldg (h + i);
-      sp[spad (i)] = make_float2 (d.x * f.x - d.y * f.y, d.x * f.y + d.y * f.x);
-    }
-    __syncthreads ();
-    smem_fft<N, T, +1> (sp, tw);
-  }
-  const uint64_t tbase = part * nkeep;
-  const unsigned rounds = unsigned ((nkeep + T - 1) / T);
-  for (unsigned r = 0; r < rounds; r++)
-  {
-    const uint64_t j = uint64_t (r) * T + threadIdx.x;
-    const bool ok = j < nkeep;
-    const int tl = ok ? int (nfilt_pos + j) : 0;
-    const float2 pv = s[spad (tl)];
-    const float2 qv = npol > 1 ? s[SP + spad (tl)] : make_float2 (0.f, 0.f);
-    if (MODE == OUT_VOLTAGE)
-    {
-      if (ok)
-      {
-        vv.out[(uint64_t (c) * npol) * vv.span + tbase + j] = pv;
-        if (npol > 1) vv.out[(uint64_t (c) * npol + 1) * vv.span + tbase + j] = qv;
-      }
-    }
-    else
-      emit_fold<NOUT> (fv, c, npol, ok, tbase + j, pv, qv);
-  }
-}
-
-// --------------------------------------------------------------------------
-// inverse filterbank (InverseFilterbankEngineCPU.C:309-779 restructured)
-// --------------------------------------------------------------------------
-
-// Stockham FFT of N points run by a group of T = N/16 threads (tid within the
-// group) on the group's own shared-memory array; every group of the CTA runs
-// the same passes, so the CTA-wide barriers line up.
-// Twiddles come from the per-pass tables (pass_table_offset layout) that the
-// caller holds in shared memory.
-template <int N, int T, int D, int P>
-__device__ __forceinline__ void group_fft_pass (float2* s, float2* v, const float2* tab, int tid)
-{
-  if constexpr (P < stockham_npass (N))
-  {
-    constexpr int R = stockham_radix (N, P);
-    constexpr int Ns = stockham_ns (N, P);
-    StockhamPassT<N, R, T, D, true, true>::load (tid, s, v);
-    __syncthreads ();
-    StockhamPassT<N, R, T, D, true, true>::compute_store (
-        tid, Ns, v, s, P ? tab + pass_table_offset (N, P) : nullptr);
-    __syncthreads ();
-    group_fft_pass<N, T, D, P + 1> (s, v, tab, tid);
-  }
-}
-
-// A CTA of IFB_THREADS threads transforms F = 8192/LIN (channel, pol) slots of
-// one part: CG = F/npol consecutive fine channels, both pols.  The input tile
-// is read so that consecutive threads touch consecutive bytes (for TFPD input
-// the slots of one time sample are contiguous; for FPT input the samples of
-// one slot are), unpacked and windowed (Apodization::operate) into shared
-// memory; each group of LIN/16 threads runs the forward FFT of its slot; then
-// the kept bins of both halves -- stitch_one's placement, precomputed per
-// channel on the host -- times the response and the spectral window go to the
-// output channel's spectrum in four-step order (bin k at row k mod n1, column
-// k div n1) for the row kernel.
-constexpr int IFB_THREADS = 512;
-
-template <int LIN, int KIND>
-__global__ void __launch_bounds__ (IFB_THREADS)
-k_ifb_stitch (const InputView in, const IfbShape sh, const IfbTables tb, const uint64_t part0,
-              float2* __restrict__ scratch)
-{
-  constexpr int TF = stockham_threads (LIN);     // threads per transform
-  constexpr int F = IFB_THREADS / TF;             // slots per CTA
-  // slot stride: the padded transform plus 32 bytes, so that the slots of one
-  // time sample written together fall on different banks
-  constexpr int SP = spad_size (LIN) + 4;
-  constexpr int TABN = pass_tables_size (LIN);
-  extern __shared__ float2 s_ifb[];               // [F][SP], then the pass tables
-  float2* s_tab = s_ifb + F * SP;
-  __shared__ float s_lut[256];
-  const unsigned npol = sh.npol;
-  const unsigned cg = F / npol;                   // channels per CTA
-  const unsigned c0 = blockIdx.x * cg;
-  const unsigned b = blockIdx.y;
-  load_lut (in, tb.lut, s_lut);
-  for (int i = threadIdx.x; i < TABN; i += IFB_THREADS) s_tab[i] = __ldg (tb.ptab_lin + i);
-  __syncthreads ();
-  const uint64_t t0 = (part0 + b) * sh.in_step;
-  // all PER loads of a thread are issued before any is used
-  constexpr int PER = F * LIN / IFB_THREADS;
-  const unsigned nslot = min (unsigned (F), (sh.nin - c0) * npol);   // live slots
-  const uint64_t row = uint64_t (sh.nin) * npol;                       // TFPD values per sample
-  uint32_t word[PER];
-  float2 fv[KIND == IN_FLOAT ? PER : 1];
-#pragma unroll
-  for (int k = 0; k < PER; k++)
-  {
-    const unsigned e = threadIdx.x + k * IFB_THREADS;
-    if constexpr (KIND == IN_FLOAT)
-    {
-      const unsigned slot = e / LIN, t = e % LIN;
-      fv[k] = slot < nslot ? __ldg (static_cast<const float2*> (in.main)
-                                    + (uint64_t (c0) * npol + slot) * in.main_span + t0 + t)
-                           : make_float2 (0.f, 0.f);
-    }
-    else
-    {
-      const unsigned slot = e % F, t = e / F;
-      const uint64_t idx = (t0 + t) * row + uint64_t (c0) * npol + slot;
-      if constexpr (KIND == IN_INT16)
-        word[k] = slot < nslot ? __ldg (static_cast<const uint32_t*> (in.main) + idx) : 0u;
-      else
-        word[k] = slot < nslot ? __ldg (static_cast<const unsigned short*> (in.main) + idx) : 0u;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < PER; k++)
-  {
-    const unsigned e = threadIdx.x + k * IFB_THREADS;
-    unsigned slot, t;
-    float2 x;
-    if constexpr (KIND == IN_FLOAT)
-    {
-      slot = e / LIN;
-      t = e % LIN;
-      x = fv[k];
-    }
-    else
-    {
-      slot = e % F;
-      t = e / F;
-      if constexpr (KIND == IN_INT16)
-      {
-        short re = short (word[k] & 0xffff), im = short (word[k] >> 16);
-        if (in.offset_binary)
-        {
-          re = short (re ^ 0x8000);
-          im = short (im ^ 0x8000);
-        }
-        // SixteenBitUnpacker.C:69: float(x) + 0.5
-        x = make_float2 (__fadd_rn (float (re), 0.5f), __fadd_rn (float (im), 0.5f));
-      }
-      else
-        x = make_float2 (s_lut[word[k] & 0xff], s_lut[word[k] >> 8]);
-      if (slot >= nslot) x = make_float2 (0.f, 0.f);
-    }
-    if (tb.temporal)
-    {
-      const float w = __ldg (tb.temporal + t);
-      x = make_float2 (__fmul_rn (x.x, w), __fmul_rn (x.y, w));
-    }
-    s_ifb[slot * SP + spad (t)] = x;
-  }
-  __syncthreads ();
-  const unsigned group = threadIdx.x / TF, tid = threadIdx.x % TF;
-  float2* s = s_ifb + group * SP;
-  {
-    float2 v[LIN / TF];
-    group_fft_pass<LIN, TF, -1, 0> (s, v, s_tab, tid);
-  }
-  const unsigned c = c0 + group / npol, p = group % npol;
-  if (c >= sh.nin) return;
-  const int4 m = __ldg (tb.map + c);
-  const unsigned keep2 = sh.keep / 2;
-  const unsigned skip2 = (LIN - sh.keep) / 2;
-  const unsigned src_neg = sh.dual_sideband ? LIN - keep2 : skip2;
-  const unsigned src_pos = sh.dual_sideband ? 0 : skip2 + keep2;
-  if (keep2 % sh.n1 == 0)
-  {
-    // n1 divides keep/2, so every half starts on a multiple of n1 and its
-    // bins fill per_row consecutive columns of each four-step row: threads
-    // walk them row by row, consecutive threads writing consecutive columns.
-    const unsigned per_row = keep2 / sh.n1;
-    const bool pow2 = (per_row & (per_row - 1)) == 0;
-    const unsigned lg = __ffs (per_row) - 1;
-    for (int h = 0; h < 2; h++)
-    {
-      const int o = h ? m.z : m.x;
-      const int offz = h ? m.w : m.y;
-      const unsigned off = unsigned (offz & (IFB_ZERO - 1));
-      const unsigned src0 = h ? src_pos : src_neg;
-      float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout + off / sh.n1;
-      for (unsigned r = tid; r < keep2; r += TF)
-      {
-        const unsigned a = pow2 ? r >> lg : r / per_row;
-        const unsigned q = r - a * per_row;
-        const unsigned j = q * sh.n1 + a;
-        float2 y = (offz & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad (src0 + j)];
-        if (tb.response)
-        {
-          const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + off + j);
-          y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
-                           __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
-        }
-        if (tb.spectral)
-        {
-          const float w = __ldg (tb.spectral + off + j);
-          y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
-        }
-        dst[uint64_t (a) * sh.n2 + q] = y;
-      }
-    }
-    return;
-  }
-  for (unsigned i = tid; i < sh.keep; i += TF)
-  {
-    const bool neg = i < keep2;
-    const unsigned j = neg ? i : i - keep2;
-    const int o = neg ? m.x : m.z;
-    const int off = neg ? m.y : m.w;
-    const unsigned k = unsigned (off & (IFB_ZERO - 1)) + j;
-    float2 y = (off & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad ((neg ? src_neg : src_pos) + j)];
-    if (tb.response)
-    {
-      // Response::operate: (f_r d_r - f_i d_i, f_i d_r + f_r d_i)
-      const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + k);
-      y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
-                       __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
-    }
-    if (tb.spectral)
-    {
-      const float w = __ldg (tb.spectral + k);
-      y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
-    }
-    float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout;
-    dst[uint64_t (k % sh.n1) * sh.n2 + k / sh.n1] = y;
-  }
-}
-
-// Inverse column DFTs of the lout-point transforms (after the row kernel):
-// conjugate four-step twiddle, n1-point inverse DFT in registers (n1 may
-// carry a factor 3), output discard, voltages out.  Pols one after another.
-template <int N1>
-__global__ void __launch_bounds__ (128)
-k_ifb_cols (const float2* __restrict__ scratch, const IfbShape sh, const float2* __restrict__ tw4,
-            const uint64_t part0, const VoltView vv)
-{
-  const unsigned i2 = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned b = blockIdx.y;
-  const unsigned o = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * sh.n2;
-  const uint64_t tbase = (part0 + b) * sh.out_step;
-  for (unsigned p = 0; p < sh.npol; p++)
-  {
-    const float2* src = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * N + i2;
-    float2 v[N1];
-#pragma unroll
-    for (int k = 0; k < N1; k++) v[k] = src[uint64_t (k) * sh.n2];
-#pragma unroll
-    for (int k = 1; k < N1; k++) v[k] = cmulc (v[k], __ldg (tw4 + uint64_t (k) * sh.n2 + i2));
-    RegDFTm<N1, +1>::run (v);
-    float2* dst = vv.out + (uint64_t (o) * sh.npol + p) * vv.span + tbase;
-#pragma unroll
-    for (int k = 0; k < N1; k++)
-    {
-      const uint64_t tl = uint64_t (k) * sh.n2 + i2;
-      if (tl >= sh.out_discard_pos && tl < sh.out_discard_pos + sh.out_step)
-        dst[tl - sh.out_discard_pos] = v[k];
-    }
-  }
-}
-
-// --------------------------------------------------------------------------
-// Filterbank with a response ("During")
-// --------------------------------------------------------------------------
-
-// Barrier of a group of TS consecutive threads that exchange data only among
-// themselves: a warp barrier when the group lies inside one warp (TS divides
-// 32), else the block's.
-template <int TS>
-__device__ __forceinline__ void group_sync ()
-{
-  static_assert (TS <= 32 ? 32 % TS == 0 : TS % 32 == 0, "groups must tile the warps");
-  if constexpr (TS <= 32)
-    __syncwarp ();
-  else
-    __syncthreads ();
-}
-
-// One radix pass of an N-point transform run by the stockham_threads(N)
-// threads of one group (lane = index in the group), both sides in the padded
-// layout relative to the group's base, or the output unpadded (PO false).
-// Every thread of the block calls it.  Its barriers cover the group only, so
-// a caller that reads or writes the groups' buffers across groups puts a
-// block barrier between that and the passes.
-template <int N, int D, int P, bool PO>
-__device__ __forceinline__ void gpass (int lane, const float2* src, float2* dst, float2* v,
-                                       const float2* tab)
-{
-  if constexpr (P < stockham_npass (N))
-  {
-    constexpr int T = stockham_threads (N);
-    constexpr int R = stockham_radix (N, P);
-    constexpr int Ns = stockham_ns (N, P);
-    StockhamPassT<N, R, T, D, true, PO>::load (lane, src, v);
-    group_sync<T> ();
-    StockhamPassT<N, R, T, D, true, PO>::compute_store (
-        lane, Ns, v, dst, P ? tab + pass_table_offset (N, P) : nullptr);
-    group_sync<T> ();
-  }
-}
-
-constexpr int DUR_N2 = 8192;
-
-template <int SEG>
-constexpr size_t during_rows_smem ()
-{
-  return size_t (spad_size (DUR_N2) + Row32<DUR_N2>::TABN + pass_tables_size (SEG))
-         * sizeof (float2);
-}
-
-// Rows of the big transform (persistent CTAs, one row at a time, two per SM):
-// the forward n2-point FFT with 32 points per thread in three passes
-// (Row32), the response of each output channel on its segment multiplied in
-// registers (Response::operate over nchan_subband channels from
-// input_ichan*nchan_subband, FilterbankEngineCPU.C:480-484), then the
-// seg-point inverse FFT of every segment, written back in place: each group
-// of seg/16 threads takes two segments.  Row r of the scratch is row
-// k1 = r mod n1 of (part, input channel, pol).
-template <int SEG>
-__global__ void __launch_bounds__ (Row32<DUR_N2>::T, 2)
-k_rows_during (float2* __restrict__ scratch, const float2* __restrict__ ptab_seg,
-               const float2* __restrict__ H, const unsigned n1, const unsigned nsub,
-               const unsigned npol, const unsigned nchan_in, const unsigned nrows,
-               const unsigned inner)
-{
-  constexpr int N2 = DUR_N2;
-  using RS = Row32<N2>;
-  constexpr int T = RS::T;
-  constexpr int TABS = pass_tables_size (SEG);
-  constexpr int TS = stockham_threads (SEG);
-  constexpr int NPS = stockham_npass (SEG);
-  constexpr int NG = T / TS;                      // segment groups
-  constexpr unsigned ROW_BYTES = N2 * sizeof (float2);
-  constexpr unsigned CHUNK = 16384;
-  static_assert (NPS == 2 || NPS == 3, "segment transforms of 64 .. 4096 points");
-  static_assert (T % TS == 0 && (N2 / SEG) == 2 * NG, "each group takes two segments");
-  extern __shared__ __align__ (16) float2 s_dur[];
-  float2* work = s_dur;
-  float2* tab1 = work + spad_size (N2);
-  float2* th = tab1 + RS::TAB1;
-  float2* tl = th + RS::TABH;
-  float2* tabs = tab1 + RS::TABN;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < RS::TABN; i += T) tab1[i] = RS::table_entry (i);
-  for (int i = tid; i < TABS; i += T) tabs[i] = __ldg (ptab_seg + i);
-  const int g = tid / TS, lane = tid % TS;
-  // As in k_rows32: rows walked with their response rows (input channel,
-  // k1) outermost, parts and polarisations innermost (inner of them), each
-  // CTA a contiguous run, the response kept in L1 (evict-last loads) and the
-  // scratch rows streamed (evict-first).
-  const auto row_of = [=] (unsigned idx, unsigned& hrow) {
-    hrow = idx / inner;                             // cin * n1 + k1
-    const unsigned bp = idx % inner;
-    return ((bp / npol) * nchan_in * n1 + hrow / n1 * n1) * npol + (bp % npol) * n1 + hrow % n1;
-  };
-  float2 v[32];
-  const unsigned run = (nrows + gridDim.x - 1) / gridDim.x;
-  const unsigned idx_end = min (nrows, (blockIdx.x + 1) * run);
-  for (unsigned idx = blockIdx.x * run; idx < idx_end; idx++)
-  {
-    unsigned hrow = 0;
-    const unsigned row = row_of (idx, hrow);
-    const unsigned k1 = hrow % n1;
-    const unsigned cin = hrow / n1;
-    float2* grow = scratch + uint64_t (row) * N2;
-    if (tid == 0 && idx + 1 < idx_end)
-    {
-      unsigned nh = 0;
-      const char* nr = reinterpret_cast<const char*> (scratch + uint64_t (row_of (idx + 1, nh)) * N2);
-      for (unsigned o = 0; o < ROW_BYTES; o += CHUNK) prefetch_l2 (nr + o, CHUNK);
-    }
-#pragma unroll
-    for (int b = 0; b < 2; b++)
-#pragma unroll
-      for (int r = 0; r < 16; r++) v[16 * b + r] = __ldcs (grow + tid + b * T + r * RS::NS2);
-    __syncthreads ();     // the previous row's segment passes are done
-    RS::template p0_compute_store<-1> (tid, v, work);
-    __syncthreads ();
-    RS::p1_load (tid, work, v);
-    __syncthreads ();
-    RS::template p1_compute_store<-1> (tid, v, work, tab1);
-    __syncthreads ();
-    RS::p2_load (tid, work, v);
-    __syncthreads ();
-    RS::template p2_compute<-1> (tid, v, th, tl);
-    // position i = cs*SEG + f2 of row k1 is bin k1 + n1*f2 of output channel
-    // cin*nsub + cs: (f_r d_r - f_i d_i, f_i d_r + f_r d_i), Response.C:662-726
-    const float2* hc = H + (uint64_t (cin) * nsub * n1 + k1) * SEG;
-#pragma unroll
-    for (int b = 0; b < 2; b++)
-#pragma unroll
-      for (int r = 0; r < 16; r++)
-      {
-        const int i = tid + b * T + r * RS::NS2;
-        const unsigned cs = unsigned (i) / SEG, f2 = unsigned (i) % SEG;
-        const float2 f = ldg_evict_last (hc + uint64_t (cs) * n1 * SEG + f2);
-        const float2 d = v[16 * b + r];
-        work[spad (i)] = make_float2 (d.x * f.x - d.y * f.y, d.x * f.y + d.y * f.x);
-      }
-    __syncthreads ();
-    // spad(s*SEG + i) = spad(s*SEG) + spad(i) because SEG is a multiple of 16
-#pragma unroll
-    for (int s2 = 0; s2 < 2; s2++)
-    {
-      const int sg = g + s2 * NG;
-      float2* wseg = work + spad (sg * SEG);
-      float2* gseg = grow + sg * SEG;
-      if constexpr (NPS == 2)
-      {
-        gpass<SEG, +1, 0, true> (lane, wseg, wseg, v, tabs);
-        gpass<SEG, +1, 1, false> (lane, wseg, gseg, v, tabs);
-      }
-      else
-      {
-        gpass<SEG, +1, 0, true> (lane, wseg, wseg, v, tabs);
-        gpass<SEG, +1, 1, true> (lane, wseg, wseg, v, tabs);
-        gpass<SEG, +1, 2, false> (lane, wseg, gseg, v, tabs);
-      }
-    }
-  }
-}
-
-// Inverse column DFTs of the freq_res-point transforms: thread i2 holds
-// sample t2 = i2 mod seg of output channel cin*nsub + i2/seg; conjugate
-// twiddle exp(+2 pi i k1 t2 / freq_res), n1-point inverse DFT giving samples
-// t2 + seg*t1, then the discard of nfilt_pos / nfilt_neg
-// (FilterbankEngineCPU.C:516-523) and voltages out, or detection + fold.
-// seg >= 64, so the 32 lanes of a warp share one output channel.
-template <int N1, int NPOL, int MODE, int NOUT>
-__global__ void __launch_bounds__ (128, N1 >= 32 ? 3 : 4)
-k_inv_cols_during (const float2* __restrict__ scratch, const DuringShape sh, const uint64_t part0,
-                   const float2* __restrict__ twd, const FoldView fv, const VoltView vv)
-{
-  const unsigned i2 = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned b = blockIdx.y;
-  const unsigned cin = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * sh.n2;
-  const unsigned cs = i2 / sh.seg, t2 = i2 % sh.seg;
-  const unsigned c = cin * sh.nsub + cs;
-  if constexpr (stage_first_pol<N1, NPOL> ())
-  {
-    __shared__ float2 s0[N1 * 128];
-    const float2* src = scratch + (uint64_t (b) * sh.nchan_in + cin) * 2 * N + i2;
-    {
-      float2 v[N1];
-      inv_column<N1> (src, sh.n2, twd + t2, sh.seg, v);
-#pragma unroll
-      for (int k = 0; k < N1; k++) s0[k * 128 + threadIdx.x] = v[k];
-    }
-    float2 q[N1];
-    inv_column<N1> (src + N, sh.n2, twd + t2, sh.seg, q);
-    const uint64_t tb = (part0 + b) * sh.nkeep;
-#pragma unroll (N1 >= 32 ? 2 : N1)
-    for (int k = 0; k < N1; k++)
-    {
-      const uint64_t tl = uint64_t (k) * sh.seg + t2;
-      const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
-      const uint64_t t = tb + (tl - sh.nfilt_pos);
-      const float2 p = s0[k * 128 + threadIdx.x];
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        if (ok)
-        {
-          vv.out[(uint64_t (c) * 2) * vv.span + t] = p;
-          vv.out[(uint64_t (c) * 2 + 1) * vv.span + t] = q[k];
-        }
-      }
-      else
-        emit_fold<NOUT> (fv, c, 2, ok, t, p, q[k]);
-    }
-    return;
-  }
-  float2 w[N1];
-#pragma unroll
-  for (int k = 1; k < N1; k++)
-    w[k] = __ldg (twd + uint64_t (k) * sh.seg + t2);
-  float2 v[NPOL][N1];
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
-  {
-    const float2* src = scratch + ((uint64_t (b) * sh.nchan_in + cin) * NPOL + p) * N + i2;
-#pragma unroll
-    for (int k = 0; k < N1; k++)
-      v[p][k] = src[uint64_t (k) * sh.n2];
-#pragma unroll
-    for (int k = 1; k < N1; k++)
-      v[p][k] = cmulc (v[p][k], w[k]);
-    RegDFT<N1, +1>::run (v[p]);
-  }
-  const uint64_t tbase = (part0 + b) * sh.nkeep;
-#pragma unroll
-  for (int k = 0; k < N1; k++)
-  {
-    const uint64_t tl = uint64_t (k) * sh.seg + t2;
-    const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
-    const uint64_t t = tbase + (tl - sh.nfilt_pos);
-    if constexpr (MODE == OUT_VOLTAGE)
-    {
-      if (ok)
-      {
-#pragma unroll
-        for (int p = 0; p < NPOL; p++)
-          vv.out[(uint64_t (c) * NPOL + p) * vv.span + t] = v[p][k];
-      }
-    }
-    else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][k], v[NPOL - 1][k]);
-  }
-}
-
-// Column passes of N1 = 64 .. 512 points (big transforms of up to 2^22 =
-// 512 x 8192 points): a CTA of N1 threads takes COLW = 16 adjacent columns,
-// loads them row by row (16 consecutive samples per row) into shared memory,
-// one column per group of N1/16 threads, and runs the N1-point Stockham
-// transforms there (per-pass tables in shared memory).  Column stride
-// spad_size(N1) + 1 keeps the 16 columns of a row on different banks.
-constexpr int COLW = 16;
-
-// Buffer stride: with 16 columns per CTA (a half-warp touches one row) 1 mod
-// 16 float2 keeps the columns on distinct bank pairs; with 8 (a half-warp
-// touches two adjacent rows, k even and k + 1) 2 mod 16 does.
-template <int N1, int CW = COLW>
-B200_CE int colbig_stride () { return spad_size (N1) + (CW >= 16 ? 1 : 2); }
-
-template <int N1, int NPOL>
-constexpr size_t colbig_smem ()
-{
-  return size_t (NPOL * COLW * colbig_stride<N1> () + pass_tables_size (N1)) * sizeof (float2);
-}
-
-// columns per CTA of the inverse pass: 8 for 512-point columns, so that both
-// polarisations (72 KB) leave room for a second CTA on the SM
-template <int N1>
-B200_CE int inv_colw () { return N1 >= 512 ? 8 : COLW; }
-
-template <int N1, int NPOL>
-constexpr size_t colbig_inv_smem ()
-{
-  return size_t (NPOL * inv_colw<N1> () * colbig_stride<N1, inv_colw<N1> ()> ()
-                 + pass_tables_size (N1))
-         * sizeof (float2);
-}
-
-// the N1-point transform (direction D) of every column in col[]
-template <int N1, int D, int SP = colbig_stride<N1> ()>
-__device__ __forceinline__ void colbig_fft (float2* col, const float2* tab)
-{
-  constexpr int TS = stockham_threads (N1);
-  const int g = threadIdx.x / TS, lane = threadIdx.x % TS;
-  float2* base = col + g * SP;
-  float2 v[16];
-  gpass<N1, D, 0, true> (lane, base, base, v, tab);
-  gpass<N1, D, 1, true> (lane, base, base, v, tab);
-  gpass<N1, D, 2, true> (lane, base, base, v, tab);
-}
-
-// Forward: unpack (and window) on load, N1-point DFTs down the columns, the
-// four-step twiddle w_N^{k1 i2}, rows of the scratch out.
-template <int N1, int KIND>
-__global__ void __launch_bounds__ (N1, 1024 / N1)
-k_fwd_cols_big (const InputView in, const float* __restrict__ lut, const uint64_t step,
-                const uint64_t part0, const unsigned n2, const float2* __restrict__ tw4,
-                const float2* __restrict__ ptab_col, float2* __restrict__ scratch,
-                const float* __restrict__ apod)
-{
-  static_assert (stockham_npass (N1) <= 3, "column transforms of at most three passes");
-  constexpr int T = N1;
-  constexpr int SP = colbig_stride<N1> ();
-  constexpr int TAB = pass_tables_size (N1);
-  extern __shared__ __align__ (16) float2 s_cb[];
-  float2* col = s_cb;
-  float2* tab = s_cb + COLW * SP;
-  __shared__ float s_lut[256];
-  load_lut (in, lut, s_lut);
-  for (int i = threadIdx.x; i < TAB; i += T) tab[i] = __ldg (ptab_col + i);
-  const unsigned c0 = blockIdx.x * COLW;
-  const unsigned b = blockIdx.y;
-  const unsigned c = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * n2;
-  const uint64_t t0 = (part0 + b) * step + c0;
-  // thread (kk, j) takes rows k = kk + m KSTEP of column c0 + j
-  constexpr int KSTEP = T / COLW;
-  const int j = threadIdx.x % COLW, kk = threadIdx.x / COLW;
-  // The block's window t0 + k n2 + j lies in one segment of the input (the
-  // carried prefix or the main block) except in the parts that straddle the
-  // prefix's end; there each sample takes the general fetch.
-  const bool one_seg = t0 >= in.npre || t0 + uint64_t (N1 - 1) * n2 + (COLW - 1) < in.npre;
-  const bool in_pre = t0 < in.npre;
-  const uint64_t ts = in_pre ? t0 : t0 - in.npre;
-  const float* ap = apod ? apod + uint64_t (kk) * n2 + c0 + j : nullptr;
-  const uint64_t rstep = uint64_t (KSTEP) * n2;
-  for (unsigned p = 0; p < in.npol; p++)
-  {
-    __syncthreads ();
-    const auto put = [&] (int k, float2 x) {
-      if (ap)
-      {
-        const float w = __ldg (ap + uint64_t (k - kk) * n2);
-        x = make_float2 (__fmul_rn (x.x, w), __fmul_rn (x.y, w));
-      }
-      col[j * SP + spad (k)] = x;
-    };
-    if (one_seg && KIND == IN_FLOAT)
-    {
-      const float2* f = static_cast<const float2*> (in_pre ? in.pre : in.main)
-                        + (uint64_t (c) * in.npol + p) * (in_pre ? in.pre_span : in.main_span)
-                        + ts + uint64_t (kk) * n2 + j;
-      for (int k = kk; k < N1; k += KSTEP, f += rstep) put (k, __ldg (f));
-    }
-    else if (one_seg)
-    {
-      // one complex sample per (t, c, p): 2 bytes (int8) or 4 (int16)
-      const uint64_t cs = uint64_t (in.nchan) * in.npol;
-      const uint64_t i0 = (ts + uint64_t (kk) * n2 + j) * cs + c * in.npol + p;
-      const uint64_t istep = rstep * cs;
-      if constexpr (KIND == IN_INT8)
-      {
-        const unsigned short* q = static_cast<const unsigned short*> (in_pre ? in.pre : in.main) + i0;
-        for (int k = kk; k < N1; k += KSTEP, q += istep)
-        {
-          const unsigned short w = __ldg (q);
-          put (k, make_float2 (s_lut[w & 0xff], s_lut[w >> 8]));
-        }
-      }
-      else
-      {
-        const unsigned* q = static_cast<const unsigned*> (in_pre ? in.pre : in.main) + i0;
-        for (int k = kk; k < N1; k += KSTEP, q += istep)
-        {
-          const unsigned w = __ldg (q);
-          short re = short (w & 0xffff), im = short (w >> 16);
-          if (in.offset_binary)
-          {
-            re = short (re ^ 0x8000);
-            im = short (im ^ 0x8000);
-          }
-          // SixteenBitUnpacker.C:69: float(x) + 0.5
-          put (k, make_float2 (__fadd_rn (float (re), 0.5f), __fadd_rn (float (im), 0.5f)));
-        }
-      }
-    }
-    else
-      for (int k = kk; k < N1; k += KSTEP)
-        put (k, fetch<KIND> (in, s_lut, c, p, t0 + uint64_t (k) * n2 + j));
-    __syncthreads ();
-    colbig_fft<N1, -1> (col, tab);
-    __syncthreads ();                  // the output below reads across columns' groups
-    float2* dst = scratch + ((uint64_t (b) * in.nchan + c) * in.npol + p) * N + c0 + j
-                  + uint64_t (kk) * n2;
-    const float2* tw = tw4 + uint64_t (kk) * n2 + c0 + j;
-    for (int k1 = kk; k1 < N1; k1 += KSTEP, dst += rstep, tw += rstep)
-    {
-      float2 y = col[j * SP + spad (k1)];
-      if (k1) y = cmul (y, __ldg (tw));
-      *dst = y;
-    }
-  }
-}
-
-// Inverse columns of the During filterbank for N1 = 64 .. 512: the 16
-// columns of a CTA lie in one output channel's segment (seg >= 64); both
-// polarisations are loaded with the conjugate twiddle exp(+2 pi i k1 t2 /
-// freq_res), transformed, and read back in time order (16 consecutive
-// samples per row) for the discard and the voltages or detection + fold.
-template <int N1, int NPOL, int MODE, int NOUT>
-__global__ void __launch_bounds__ (inv_colw<N1> () * stockham_threads (N1), 1024 / N1)
-k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
-                       const uint64_t part0, const float2* __restrict__ twd,
-                       const float2* __restrict__ ptab_col, const FoldView fv, const VoltView vv)
-{
-  constexpr int CW = inv_colw<N1> ();
-  constexpr int T = CW * stockham_threads (N1);
-  constexpr int SP = colbig_stride<N1, CW> ();
-  constexpr int TAB = pass_tables_size (N1);
-  extern __shared__ __align__ (16) float2 s_cb[];
-  float2* tab = s_cb + NPOL * CW * SP;
-  for (int i = threadIdx.x; i < TAB; i += T) tab[i] = __ldg (ptab_col + i);
-  const unsigned c0 = blockIdx.x * CW;
-  const unsigned b = blockIdx.y;
-  const unsigned cin = blockIdx.z;
-  const uint64_t N = uint64_t (N1) * sh.n2;
-  const unsigned cs = c0 / sh.seg, t20 = c0 % sh.seg;
-  const unsigned c = cin * sh.nsub + cs;
-  // thread (kk, j) takes rows k1 = kk + m KSTEP of column c0 + j
-  constexpr int KSTEP = T / CW;
-  const int j = threadIdx.x % CW, kk = threadIdx.x / CW;
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
-  {
-    const float2* src = scratch + ((uint64_t (b) * sh.nchan_in + cin) * NPOL + p) * N + c0 + j
-                        + uint64_t (kk) * sh.n2;
-    const float2* tw = twd + uint64_t (kk) * sh.seg + t20 + j;
-    float2* col = s_cb + p * CW * SP + j * SP;
-    const uint64_t sstep = uint64_t (KSTEP) * sh.n2, tstep = uint64_t (KSTEP) * sh.seg;
-    for (int k1 = kk; k1 < N1; k1 += KSTEP, src += sstep, tw += tstep)
-    {
-      float2 x = *src;
-      if (k1) x = cmulc (x, __ldg (tw));
-      col[spad (k1)] = x;
-    }
-  }
-  __syncthreads ();
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
-    colbig_fft<N1, +1, SP> (s_cb + p * CW * SP, tab);
-  __syncthreads ();                    // the fold below reads across columns' groups
-  const uint64_t tbase = (part0 + b) * sh.nkeep;
-  const float2* c0p = s_cb;
-  const float2* c1p = s_cb + (NPOL - 1) * CW * SP;
-  for (int e = threadIdx.x; e < CW * N1; e += T)
-  {
-    const int j = e % CW, t1 = e / CW;
-    const uint64_t tl = uint64_t (t1) * sh.seg + t20 + j;
-    const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
-    const uint64_t t = tbase + (tl - sh.nfilt_pos);
-    const float2 pv = c0p[j * SP + spad (t1)];
-    const float2 qv = c1p[j * SP + spad (t1)];
-    if constexpr (MODE == OUT_VOLTAGE)
-    {
-      if (ok)
-      {
-        vv.out[(uint64_t (c) * NPOL) * vv.span + t] = pv;
-        if (NPOL == 2) vv.out[(uint64_t (c) * NPOL + 1) * vv.span + t] = qv;
-      }
-    }
-    else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, pv, qv);
-  }
-}
+namespace {
 
 // --------------------------------------------------------------------------
 // response construction
@@ -2434,34 +740,80 @@ __global__ void k_zeroed_fold (const float2* __restrict__ v, const uint64_t span
   warp_fold<NOUT> (ok, bin, d, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride, fv.hits);
 }
 
-// one thread per sample: the column warp_fold_bin would give it
-// A warp takes COLPLAN_GROUPS consecutive groups of 32 samples: one binary
-// search for the first sample, then each lane steps forward over the
-// segment boundaries from where the previous group's last lane ended.
-constexpr int COLPLAN_GROUPS = 32;
-
-__global__ void k_colplan (const FoldSegment* __restrict__ segs, const int nseg,
-                           const uint64_t ndat, const unsigned nbin, unsigned* __restrict__ cols)
+// Segment holding sample t, found by a whole warp: each round probes 32
+// evenly spaced starts at once (two dependent loads for up to 1024 segments,
+// where a binary search takes ten).
+__device__ __forceinline__ int warp_seg_search (const FoldSegment* __restrict__ segs, int nseg,
+                                                uint64_t t)
 {
   const int lane = threadIdx.x & 31;
-  const uint64_t w0 = (uint64_t (blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32) * 32
-                      * COLPLAN_GROUPS;
-  if (w0 >= ndat) return;             // whole warps
-  int s = 0;
-  if (lane == 0) s = seg_search (segs, nseg, w0);
-  s = __shfl_sync (FULL, s, 0);
-  for (int g = 0; g < COLPLAN_GROUPS; g++)
+  int lo = 0, len = nseg;
+  while (len > 1)
   {
-    const uint64_t t = w0 + uint64_t (g) * 32 + lane;
-    int sl = s;
-    while (sl + 1 < nseg && __ldg (&segs[sl + 1].start) <= t) sl++;
-    if (t < ndat)
+    const int step = (len + 31) / 32;
+    const int off = lane * step;
+    const bool le = off < len && (off == 0 || __ldg (&segs[lo + off].start) <= t);
+    const int j = 31 - __clz (__ballot_sync (FULL, le));
+    lo += j * step;
+    len = min (step, len - j * step);
+  }
+  return lo;
+}
+
+// The column warp_fold_bin would give each sample.  A warp takes
+// COLPLAN_SAMPLES consecutive samples, each lane four at a time (one 16-byte
+// store): one search for the first sample, then each lane steps forward over
+// the segment boundaries from where the previous group's last lane ended,
+// and a lane's samples advance m by dm within a segment.  Bound by latency
+// (the search, the segment loads and the double chain), so the serial chain
+// per warp is kept short: one sample per lane and 32 groups per warp took
+// 37.6 us for 10 M samples and 7.7 us for 60 k; this takes 24.2 and 3.9 us.
+// (Adding powers of two instead of the 64-bit conversions: 31.0 us.)
+constexpr int COLPLAN_SAMPLES = 512;
+
+__global__ void __launch_bounds__ (256)
+k_colplan (const FoldSegment* __restrict__ segs, const int nseg, const uint64_t ndat,
+           const unsigned nbin, unsigned* __restrict__ cols)
+{
+  const int lane = threadIdx.x & 31;
+  const uint64_t w0 = (uint64_t (blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32)
+                      * COLPLAN_SAMPLES;
+  if (w0 >= ndat) return;             // whole warps
+  int s = warp_seg_search (segs, nseg, w0);
+  const double fbin = double (nbin);
+#pragma unroll 1
+  for (int g = 0; g < COLPLAN_SAMPLES; g += 128)
+  {
+    const uint64_t t0 = w0 + unsigned (g) + 4 * lane;
+    unsigned c[4];
+    int64_t m = 0, dm = 0;
+    double gr = 0;
+    unsigned base = 0;
+    uint64_t next = 0;                // the segment's end; 0: none loaded yet
+#pragma unroll
+    for (int i = 0; i < 4; i++)
     {
-      const unsigned base = __ldg (&segs[sl].base);
-      const unsigned bin = seg_bin (segs, sl, t, nbin);
-      cols[t] = (base == FOLD_SKIP || bin >= nbin) ? NO_COLUMN : base + bin;
+      const uint64_t t = t0 + i;
+      if (t >= next)
+      {
+        if (next) s++;
+        while (s + 1 < nseg && __ldg (&segs[s + 1].start) <= t) s++;
+        next = s + 1 < nseg ? __ldg (&segs[s + 1].start) : ~uint64_t (0);
+        dm = __ldg (&segs[s].dm);
+        m = __ldg (&segs[s].m0) + int64_t (t - __ldg (&segs[s].start)) * dm;
+        gr = __ldg (&segs[s].g);
+        base = __ldg (&segs[s].base);
+      }
+      const unsigned bin = __double2uint_rz (__dmul_rn (__dmul_rn (double (m), gr), fbin));
+      c[i] = (base == FOLD_SKIP || bin >= nbin) ? NO_COLUMN : base + bin;
+      m += dm;
     }
-    s = __shfl_sync (FULL, sl, 31);
+    if (t0 + 4 <= ndat)
+      *reinterpret_cast<uint4*> (cols + t0) = make_uint4 (c[0], c[1], c[2], c[3]);
+    else
+      for (int i = 0; i < 4; i++)
+        if (t0 + i < ndat) cols[t0 + i] = c[i];
+    s = __shfl_sync (FULL, s, 31);
   }
 }
 
@@ -2473,224 +825,9 @@ __global__ void k_binplan (const FoldSegment* __restrict__ segs, const int nseg,
   out[t] = fold_bin (segs, nseg, t, nbin);
 }
 
-// --------------------------------------------------------------------------
-// launch helpers
-// --------------------------------------------------------------------------
-
-template <int N1, int NPOL, int MODE, int NOUT>
-void launch_inv (const ConvShape& sh, dim3 grid, float2* scratch, uint64_t part0,
-                 const ConvTables& tb, const FoldView& fv, const VoltView& vv, cudaStream_t st)
-{
-  if (N1 == 32) grid.x = sh.n2 / 64;        // two threads per column
-  k_inv_cols<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh.n2, sh.nchan, sh.nkeep,
-                                                          sh.nfilt_pos, part0, tb.tw4, fv, vv);
-}
-
-template <int N2>
-void launch_rows (unsigned nrows, float2* scratch, const ConvTables& tb, unsigned n1,
-                  const ConvShape& sh, cudaStream_t st)
-{
-  if (N2 == 8192 && tb.tc_splits)
-  {
-    launch_rows_mma (nrows, scratch, tb, n1, sh, st);
-    return;
-  }
-  // persistent: as many CTAs as are resident at once
-  const unsigned grid = std::min<unsigned> (nrows, rows_ctas_per_sm (N2) * unsigned (tb.nsm));
-  k_rows32<N2, true><<<grid, Row32<N2>::T, rows32_smem_bytes<N2> (), st>>> (
-      scratch, tb.H, n1, sh.nchan, sh.npol, nrows, nrows / (n1 * sh.nchan));
-}
-
-template <int N1>
-cudaError_t run_fourstep_n1 (const ConvShape& sh, const ConvTables& tb, const InputView& in,
-                             uint64_t part0, unsigned nbatch, float2* scratch, int mode,
-                             const FoldView& fv, const VoltView& vv, cudaStream_t st,
-                             const KernelClock* clk)
-{
-  const dim3 gcol (sh.n2 / 128, nbatch, sh.nchan);
-  const dim3 gfwd (sh.n2 / fwd_cols_per_block<N1> (), nbatch, sh.nchan);
-  if (in.fb_nsub)
-  {
-    // the 64-channel filterbank inside the column pass
-    if (N1 != 8 || in.fb_nsub != 64 || sh.nchan != 64 || in.nchan != 1 || in.npol != 2
-        || sh.npol != 2 || tb.apod || (in.kind != IN_INT8 && in.kind != IN_INT16))
-      return cudaErrorInvalidValue;
-    ClockScope cs (clk, KK_FWD_COLS, st);
-    const dim3 g (sh.n2 / FBC_COLS, nbatch);
-    if (in.kind == IN_INT8 && in.lut_scale != 0.f)
-      k_fwd_cols_fb64<IN_INT8, true><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep, part0,
-                                                                         sh.n2, tb.tw4, scratch);
-    else if (in.kind == IN_INT8)
-      k_fwd_cols_fb64<IN_INT8, false><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep, part0,
-                                                                          sh.n2, tb.tw4, scratch);
-    else
-      k_fwd_cols_fb64<IN_INT16, false><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep,
-                                                                           part0, sh.n2, tb.tw4,
-                                                                           scratch);
-  }
-  else
-  {
-  ClockScope cs (clk, KK_FWD_COLS, st);
-  if (in.kind == IN_INT8)
-    k_fwd_cols<N1, IN_INT8><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.nkeep, part0, sh.n2, tb.tw4,
-                                                   scratch, tb.apod);
-  else if (in.kind == IN_INT16)
-    k_fwd_cols<N1, IN_INT16><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.nkeep, part0, sh.n2, tb.tw4,
-                                                    scratch, tb.apod);
-  else
-    k_fwd_cols<N1, IN_FLOAT><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.nkeep, part0, sh.n2, tb.tw4,
-                                                    scratch, tb.apod);
-  }
-  const unsigned nrows = N1 * nbatch * sh.nchan * sh.npol;
-  {
-  ClockScope cs (clk, KK_ROWS, st);
-  if (sh.n2 == 8192)
-    launch_rows<8192> (nrows, scratch, tb, N1, sh, st);
-  else if (sh.n2 == 4096)
-    launch_rows<4096> (nrows, scratch, tb, N1, sh, st);
-  else
-    return cudaErrorInvalidValue;
-  }
-  ClockScope cs (clk, KK_INV_COLS, st);
-  if (sh.npol == 2)
-  {
-    if (mode == OUT_VOLTAGE)
-      launch_inv<N1, 2, OUT_VOLTAGE, 1> (sh, gcol, scratch, part0, tb, fv, vv, st);
-    else if (fv.nout == 1)
-      launch_inv<N1, 2, OUT_FOLD, 1> (sh, gcol, scratch, part0, tb, fv, vv, st);
-    else if (fv.nout == 2)
-      launch_inv<N1, 2, OUT_FOLD, 2> (sh, gcol, scratch, part0, tb, fv, vv, st);
-    else
-      launch_inv<N1, 2, OUT_FOLD, 4> (sh, gcol, scratch, part0, tb, fv, vv, st);
-  }
-  else
-  {
-    if (mode == OUT_VOLTAGE)
-      launch_inv<N1, 1, OUT_VOLTAGE, 1> (sh, gcol, scratch, part0, tb, fv, vv, st);
-    else
-      launch_inv<N1, 1, OUT_FOLD, 1> (sh, gcol, scratch, part0, tb, fv, vv, st);
-  }
-  return cudaGetLastError ();
-}
-
-// The fused kernel's shared-memory opt-in (sized for two polarisations), once
-// per device and instantiation; later calls only test a bit, so that calls
-// made inside a stream capture set nothing up.
-template <int N, int KIND, int MODE, int NOUT>
-cudaError_t fused_setup ()
-{
-  static std::atomic<unsigned> done {0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice (&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned bit = dev < 32 ? 1u << dev : 0u;    // devices past 32: set every time
-  if (bit && (done.load () & bit)) return cudaSuccess;
-  e = cudaFuncSetAttribute (k_fused<N, stockham_threads (N), KIND, MODE, NOUT>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            int (2 * spad_size (N) * sizeof (float2)));
-  if (e == cudaSuccess) done.fetch_or (bit);
-  return e;
-}
-
-template <int N, int KIND, int MODE, int NOUT>
-cudaError_t run_fused_t (const ConvShape& sh, const ConvTables& tb, const InputView& in,
-                         uint64_t part0, unsigned nbatch, const FoldView& fv,
-                         const VoltView& vv, cudaStream_t st, const KernelClock* clk)
-{
-  constexpr int T = stockham_threads (N);
-  const size_t smem = size_t (in.npol) * spad_size (N) * sizeof (float2);
-  auto kern = k_fused<N, T, KIND, MODE, NOUT>;
-  cudaError_t err = fused_setup<N, KIND, MODE, NOUT> ();
-  if (err != cudaSuccess) return err;
-  ClockScope cs (clk, KK_FUSED, st);
-  kern<<<dim3 (nbatch, sh.nchan), T, smem, st>>> (in, tb.lut, tb.tw2, tb.H, sh.nkeep,
-                                                  sh.nfilt_pos, part0, fv, vv, tb.apod);
-  return cudaGetLastError ();
-}
-
-template <int N, int KIND>
-cudaError_t run_fused_k (const ConvShape& sh, const ConvTables& tb, const InputView& in,
-                         uint64_t part0, unsigned nbatch, int mode, const FoldView& fv,
-                         const VoltView& vv, cudaStream_t st, const KernelClock* clk)
-{
-  if (mode == OUT_VOLTAGE)
-    return run_fused_t<N, KIND, OUT_VOLTAGE, 1> (sh, tb, in, part0, nbatch, fv, vv, st, clk);
-  if (fv.nout == 1)
-    return run_fused_t<N, KIND, OUT_FOLD, 1> (sh, tb, in, part0, nbatch, fv, vv, st, clk);
-  if (fv.nout == 2)
-    return run_fused_t<N, KIND, OUT_FOLD, 2> (sh, tb, in, part0, nbatch, fv, vv, st, clk);
-  return run_fused_t<N, KIND, OUT_FOLD, 4> (sh, tb, in, part0, nbatch, fv, vv, st, clk);
-}
-
-template <int N>
-cudaError_t run_fused (const ConvShape& sh, const ConvTables& tb, const InputView& in,
-                       uint64_t part0, unsigned nbatch, int mode, const FoldView& fv,
-                       const VoltView& vv, cudaStream_t st, const KernelClock* clk)
-{
-  if (in.kind == IN_INT8)
-    return run_fused_k<N, IN_INT8> (sh, tb, in, part0, nbatch, mode, fv, vv, st, clk);
-  if (in.kind == IN_INT16)
-    return run_fused_k<N, IN_INT16> (sh, tb, in, part0, nbatch, mode, fv, vv, st, clk);
-  return run_fused_k<N, IN_FLOAT> (sh, tb, in, part0, nbatch, mode, fv, vv, st, clk);
-}
-
-template <int LIN, int KIND>
-void launch_ifb_stitch (const IfbShape& sh, const IfbTables& tb, const InputView& in,
-                        uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
-{
-  constexpr int F = IFB_THREADS / stockham_threads (LIN);
-  const size_t smem = (size_t (F) * (spad_size (LIN) + 4) + pass_tables_size (LIN)) * sizeof (float2);
-  auto kern = k_ifb_stitch<LIN, KIND>;
-  cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-  const unsigned cg = F / sh.npol;
-  kern<<<dim3 ((sh.nin + cg - 1) / cg, nbatch), IFB_THREADS, smem, st>>> (in, sh, tb, part0,
-                                                                         scratch);
-}
-
-template <int LIN>
-void launch_ifb_stitch_k (const IfbShape& sh, const IfbTables& tb, const InputView& in,
-                          uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
-{
-  if (in.kind == IN_INT8)
-    launch_ifb_stitch<LIN, IN_INT8> (sh, tb, in, part0, nbatch, scratch, st);
-  else if (in.kind == IN_INT16)
-    launch_ifb_stitch<LIN, IN_INT16> (sh, tb, in, part0, nbatch, scratch, st);
-  else
-    launch_ifb_stitch<LIN, IN_FLOAT> (sh, tb, in, part0, nbatch, scratch, st);
-}
-
-template <int N1>
-void launch_ifb_cols (const IfbShape& sh, const IfbTables& tb, uint64_t part0, unsigned nbatch,
-                      const float2* scratch, const VoltView& vv, cudaStream_t st)
-{
-  k_ifb_cols<N1><<<dim3 (sh.n2 / 128, nbatch, sh.nout), 128, 0, st>>> (scratch, sh, tb.tw4, part0,
-                                                                       vv);
-}
-
-template <int N2>
-void launch_rows_inv (unsigned nrows, float2* scratch, const IfbTables& tb, unsigned n1,
-                      unsigned npol, cudaStream_t st)
-{
-  const unsigned grid = std::min<unsigned> (nrows, rows_ctas_per_sm (N2) * unsigned (tb.nsm));
-  k_rows32<N2, false><<<grid, Row32<N2>::T, rows32_smem_bytes<N2> (), st>>> (
-      scratch, nullptr, n1, 1, npol, nrows, nrows / n1);
-}
-
-template <int N2, bool CONV>
-cudaError_t set_rows_smem ()
-{
-  return cudaFuncSetAttribute (k_rows32<N2, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int (rows32_smem_bytes<N2> ()));
-}
-
 } // namespace
 
 uint64_t kernel_launches () { return g_launches.load (); }
-
-unsigned rows_ctas_per_sm (unsigned n2)
-{
-  return n2 == 8192 ? rows32_ctas_per_sm<8192> () : rows32_ctas_per_sm<4096> ();
-}
 
 unsigned pass_tables_count (unsigned n)
 {
@@ -2725,358 +862,6 @@ void make_pass_tables (unsigned n, float2* out, unsigned capacity)
         out[idx] = make_float2 (float (cos (ang)), float (sin (ang)));
       }
   }
-}
-
-// The four-step kernels' shared-memory opt-in, once per device (the current
-// one); later calls only test a bit.
-cudaError_t convolution_kernel_setup ()
-{
-  static std::atomic<unsigned> attr_done {0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice (&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned bit = dev < 32 ? 1u << dev : 0u;    // devices past 32: set every time
-  if (bit && (attr_done.load () & bit)) return cudaSuccess;
-  e = set_rows_smem<8192, true> ();
-  if (e == cudaSuccess) e = set_rows_smem<4096, true> ();
-  // the single-kernel transforms of the float voltage path (the no-alloc
-  // entry point's)
-  if (e == cudaSuccess) e = fused_setup<4096, IN_FLOAT, OUT_VOLTAGE, 1> ();
-  if (e == cudaSuccess) e = fused_setup<8192, IN_FLOAT, OUT_VOLTAGE, 1> ();
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT8, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT8, true>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT16, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
-  if (e == cudaSuccess) attr_done.fetch_or (bit);
-  return e;
-}
-
-cudaError_t launch_convolution (const ConvShape& sh, const ConvTables& tb, const InputView& in,
-                                uint64_t part0, unsigned nbatch, float2* scratch, int mode,
-                                const FoldView& fv, const VoltView& vv, cudaStream_t st,
-                                const KernelClock* clk)
-{
-  if (nbatch == 0) return cudaSuccess;
-  if (sh.n1 == 1)
-  {
-    switch (sh.nfft)
-    {
-      case 4096: return run_fused<4096> (sh, tb, in, part0, nbatch, mode, fv, vv, st, clk);
-      case 8192: return run_fused<8192> (sh, tb, in, part0, nbatch, mode, fv, vv, st, clk);
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  {
-    const cudaError_t e = convolution_kernel_setup ();
-    if (e != cudaSuccess) return e;
-  }
-  switch (sh.n1)
-  {
-    case 2: return run_fourstep_n1<2> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 4: return run_fourstep_n1<4> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 8: return run_fourstep_n1<8> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 16: return run_fourstep_n1<16> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 32: return run_fourstep_n1<32> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-namespace {
-
-template <int SEG>
-cudaError_t launch_rows_during (unsigned nrows, float2* scratch, const DuringShape& sh,
-                                const DuringTables& tb, cudaStream_t st)
-{
-  constexpr size_t smem = during_rows_smem<SEG> ();
-  static_assert (smem <= 227u * 1024u, "row kernel shared memory");
-  cudaError_t e = cudaFuncSetAttribute (k_rows_during<SEG>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-  if (e != cudaSuccess) return e;
-  // persistent: two CTAs per SM
-  const unsigned grid = std::min<unsigned> (nrows, 2 * unsigned (tb.nsm));
-  k_rows_during<SEG><<<grid, Row32<DUR_N2>::T, smem, st>>> (
-      scratch, tb.ptab_seg, tb.H, sh.n1, sh.nsub, sh.npol, sh.nchan_in, nrows,
-      nrows / (sh.n1 * sh.nchan_in));
-  return cudaSuccess;
-}
-
-template <int N1, int NPOL, int MODE, int NOUT>
-void launch_inv_during (const DuringShape& sh, dim3 grid, const float2* scratch, uint64_t part0,
-                        const DuringTables& tb, const FoldView& fv, const VoltView& vv,
-                        cudaStream_t st)
-{
-  k_inv_cols_during<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh, part0, tb.twd, fv,
-                                                                 vv);
-}
-
-template <int N1, int NPOL>
-void launch_inv_during_m (const DuringShape& sh, dim3 grid, const float2* scratch,
-                          uint64_t part0, const DuringTables& tb, int mode, const FoldView& fv,
-                          const VoltView& vv, cudaStream_t st)
-{
-  if (mode == OUT_VOLTAGE)
-    launch_inv_during<N1, NPOL, OUT_VOLTAGE, 1> (sh, grid, scratch, part0, tb, fv, vv, st);
-  else if (NPOL == 1 || fv.nout == 1)
-    launch_inv_during<N1, NPOL, OUT_FOLD, 1> (sh, grid, scratch, part0, tb, fv, vv, st);
-  else if (fv.nout == 2)
-    launch_inv_during<N1, NPOL, OUT_FOLD, 2> (sh, grid, scratch, part0, tb, fv, vv, st);
-  else
-    launch_inv_during<N1, NPOL, OUT_FOLD, 4> (sh, grid, scratch, part0, tb, fv, vv, st);
-}
-
-template <int N1>
-cudaError_t run_during_n1 (const DuringShape& sh, const DuringTables& tb, const InputView& in,
-                           uint64_t part0, unsigned nbatch, float2* scratch, int mode,
-                           const FoldView& fv, const VoltView& vv, cudaStream_t st,
-                           const KernelClock* clk)
-{
-  const dim3 gcol (sh.n2 / 128, nbatch, sh.nchan_in);
-  const dim3 gfwd (sh.n2 / fwd_cols_per_block<N1> (), nbatch, sh.nchan_in);
-  {
-    ClockScope cs (clk, KK_FWD_COLS, st);
-    if (in.kind == IN_INT8)
-      k_fwd_cols<N1, IN_INT8><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.in_step, part0, sh.n2, tb.tw4,
-                                                     scratch, tb.apod);
-    else if (in.kind == IN_INT16)
-      k_fwd_cols<N1, IN_INT16><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.in_step, part0, sh.n2,
-                                                      tb.tw4, scratch, tb.apod);
-    else
-      k_fwd_cols<N1, IN_FLOAT><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.in_step, part0, sh.n2,
-                                                      tb.tw4, scratch, tb.apod);
-  }
-  const unsigned nrows = N1 * nbatch * sh.nchan_in * sh.npol;
-  cudaError_t e = cudaSuccess;
-  {
-    ClockScope cs (clk, KK_ROWS, st);
-    switch (sh.seg)
-    {
-      case 64: e = launch_rows_during<64> (nrows, scratch, sh, tb, st); break;
-      case 128: e = launch_rows_during<128> (nrows, scratch, sh, tb, st); break;
-      case 256: e = launch_rows_during<256> (nrows, scratch, sh, tb, st); break;
-      case 512: e = launch_rows_during<512> (nrows, scratch, sh, tb, st); break;
-      case 1024: e = launch_rows_during<1024> (nrows, scratch, sh, tb, st); break;
-      case 2048: e = launch_rows_during<2048> (nrows, scratch, sh, tb, st); break;
-      case 4096: e = launch_rows_during<4096> (nrows, scratch, sh, tb, st); break;
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  if (e != cudaSuccess) return e;
-  ClockScope cs (clk, KK_INV_COLS, st);
-  if (sh.npol == 2)
-    launch_inv_during_m<N1, 2> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  else
-    launch_inv_during_m<N1, 1> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  return cudaGetLastError ();
-}
-
-template <int N1, int NPOL>
-void launch_inv_during_big (const DuringShape& sh, dim3 grid, const float2* scratch,
-                            uint64_t part0, const DuringTables& tb, int mode, const FoldView& fv,
-                            const VoltView& vv, cudaStream_t st)
-{
-  constexpr size_t smem = colbig_inv_smem<N1, NPOL> ();
-  constexpr int T = inv_colw<N1> () * stockham_threads (N1);
-  grid.x = sh.n2 / inv_colw<N1> ();
-  if (mode == OUT_VOLTAGE)
-  {
-    auto k = k_inv_cols_during_big<N1, NPOL, OUT_VOLTAGE, 1>;
-    cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-    k<<<grid, T, smem, st>>> (scratch, sh, part0, tb.twd, tb.ptab_col, fv, vv);
-    return;
-  }
-  auto k = NPOL == 1 || fv.nout == 1 ? k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 1>
-         : fv.nout == 2 ? k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 2>
-                        : k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 4>;
-  cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-  k<<<grid, T, smem, st>>> (scratch, sh, part0, tb.twd, tb.ptab_col, fv, vv);
-}
-
-template <int N1>
-cudaError_t run_during_big (const DuringShape& sh, const DuringTables& tb, const InputView& in,
-                            uint64_t part0, unsigned nbatch, float2* scratch, int mode,
-                            const FoldView& fv, const VoltView& vv, cudaStream_t st,
-                            const KernelClock* clk)
-{
-  static_assert (colbig_inv_smem<N1, 2> () <= 227u * 1024u, "column kernel shared memory");
-  const dim3 gcol (sh.n2 / COLW, nbatch, sh.nchan_in);
-  {
-    ClockScope cs (clk, KK_FWD_COLS, st);
-    constexpr size_t smem = colbig_smem<N1, 1> ();
-    if (in.kind == IN_INT8)
-    {
-      cudaFuncSetAttribute (k_fwd_cols_big<N1, IN_INT8>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-      k_fwd_cols_big<N1, IN_INT8><<<gcol, N1, smem, st>>> (in, tb.lut, sh.in_step, part0, sh.n2,
-                                                          tb.tw4, tb.ptab_col, scratch, tb.apod);
-    }
-    else if (in.kind == IN_INT16)
-    {
-      cudaFuncSetAttribute (k_fwd_cols_big<N1, IN_INT16>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-      k_fwd_cols_big<N1, IN_INT16><<<gcol, N1, smem, st>>> (in, tb.lut, sh.in_step, part0, sh.n2,
-                                                           tb.tw4, tb.ptab_col, scratch, tb.apod);
-    }
-    else
-    {
-      cudaFuncSetAttribute (k_fwd_cols_big<N1, IN_FLOAT>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-      k_fwd_cols_big<N1, IN_FLOAT><<<gcol, N1, smem, st>>> (in, tb.lut, sh.in_step, part0, sh.n2,
-                                                           tb.tw4, tb.ptab_col, scratch, tb.apod);
-    }
-  }
-  const unsigned nrows = N1 * nbatch * sh.nchan_in * sh.npol;
-  cudaError_t e = cudaSuccess;
-  {
-    ClockScope cs (clk, KK_ROWS, st);
-    switch (sh.seg)
-    {
-      case 64: e = launch_rows_during<64> (nrows, scratch, sh, tb, st); break;
-      case 128: e = launch_rows_during<128> (nrows, scratch, sh, tb, st); break;
-      case 256: e = launch_rows_during<256> (nrows, scratch, sh, tb, st); break;
-      case 512: e = launch_rows_during<512> (nrows, scratch, sh, tb, st); break;
-      case 1024: e = launch_rows_during<1024> (nrows, scratch, sh, tb, st); break;
-      case 2048: e = launch_rows_during<2048> (nrows, scratch, sh, tb, st); break;
-      case 4096: e = launch_rows_during<4096> (nrows, scratch, sh, tb, st); break;
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  if (e != cudaSuccess) return e;
-  ClockScope cs (clk, KK_INV_COLS, st);
-  if (sh.npol == 2)
-    launch_inv_during_big<N1, 2> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  else
-    launch_inv_during_big<N1, 1> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  return cudaGetLastError ();
-}
-
-} // namespace
-
-namespace {
-__global__ void k_window_response (float2* __restrict__ out, const float2* __restrict__ in,
-                                   const float* __restrict__ w, const uint64_t n,
-                                   const unsigned n1, const unsigned seg)
-{
-  const uint64_t idx = uint64_t (blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= n) return;
-  const uint64_t fr = uint64_t (n1) * seg;
-  const unsigned r = unsigned (idx % fr);
-  const unsigned f = r / seg + n1 * (r % seg);
-  const float2 h = in[idx];
-  const float x = __ldg (w + f);
-  out[idx] = make_float2 (__fmul_rn (h.x, x), __fmul_rn (h.y, x));
-}
-} // namespace
-
-cudaError_t launch_window_response (float2* out, const float2* in, const float* window,
-                                    unsigned nchan, unsigned n1, unsigned seg, cudaStream_t st)
-{
-  const uint64_t n = uint64_t (nchan) * n1 * seg;
-  g_launches++;
-  k_window_response<<<unsigned ((n + 255) / 256), 256, 0, st>>> (out, in, window, n, n1, seg);
-  return cudaGetLastError ();
-}
-
-bool during_supported (unsigned nsub, unsigned freq_res)
-{
-  if (nsub < 2 || nsub > 128 || (nsub & (nsub - 1))) return false;
-  const uint64_t n = uint64_t (nsub) * freq_res;
-  return freq_res && (freq_res & (freq_res - 1)) == 0 && n >= 2 * DUR_N2 && n <= 512 * DUR_N2;
-}
-
-cudaError_t launch_filterbank_during (const DuringShape& sh, const DuringTables& tb,
-                                      const InputView& in, uint64_t part0, unsigned nbatch,
-                                      float2* scratch, int mode, const FoldView& fv,
-                                      const VoltView& vv, cudaStream_t st,
-                                      const KernelClock* clk)
-{
-  if (nbatch == 0) return cudaSuccess;
-  if (!during_supported (sh.nsub, sh.freq_res) || sh.n2 != unsigned (DUR_N2)
-      || uint64_t (sh.n1) * sh.n2 != uint64_t (sh.nsub) * sh.freq_res || sh.seg * sh.nsub != sh.n2
-      || sh.npol < 1 || sh.npol > 2 || in.fb_nsub)
-    return cudaErrorInvalidValue;
-  switch (sh.n1)
-  {
-    case 2: return run_during_n1<2> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 4: return run_during_n1<4> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 8: return run_during_n1<8> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 16: return run_during_n1<16> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 32: return run_during_n1<32> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 64: return run_during_big<64> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 128:
-      return run_during_big<128> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 256:
-      return run_during_big<256> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    case 512:
-      return run_during_big<512> (sh, tb, in, part0, nbatch, scratch, mode, fv, vv, st, clk);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-bool ifb_supported_lin (unsigned lin)
-{
-  return lin == 64 || lin == 128 || lin == 256 || lin == 512 || lin == 1024 || lin == 2048 ||
-         lin == 4096;
-}
-
-cudaError_t launch_inverse_filterbank (const IfbShape& sh, const IfbTables& tb,
-                                       const InputView& in, uint64_t part0, unsigned nbatch,
-                                       float2* scratch, const VoltView& vv, cudaStream_t st,
-                                       const KernelClock* clk)
-{
-  if (nbatch == 0) return cudaSuccess;
-  if (sh.n2 != 8192 && sh.n2 != 4096) return cudaErrorInvalidValue;
-  static unsigned attr_done = 0;
-  int dev = 0;
-  cudaGetDevice (&dev);
-  if (dev < 32 && !(attr_done & (1u << dev)))
-  {
-    cudaError_t e = set_rows_smem<8192, false> ();
-    if (e == cudaSuccess) e = set_rows_smem<4096, false> ();
-    if (e != cudaSuccess) return e;
-    attr_done |= 1u << dev;
-  }
-  {
-    ClockScope cs (clk, KK_FWD_COLS, st);
-    switch (sh.lin)
-    {
-      case 64: launch_ifb_stitch_k<64> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 128: launch_ifb_stitch_k<128> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 256: launch_ifb_stitch_k<256> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 512: launch_ifb_stitch_k<512> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 1024: launch_ifb_stitch_k<1024> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 2048: launch_ifb_stitch_k<2048> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 4096: launch_ifb_stitch_k<4096> (sh, tb, in, part0, nbatch, scratch, st); break;
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  const unsigned nrows = sh.n1 * nbatch * sh.nout * sh.npol;
-  {
-    ClockScope cs (clk, KK_ROWS, st);
-    if (sh.n2 == 8192)
-      launch_rows_inv<8192> (nrows, scratch, tb, sh.n1, sh.npol, st);
-    else
-      launch_rows_inv<4096> (nrows, scratch, tb, sh.n1, sh.npol, st);
-  }
-  ClockScope cs (clk, KK_INV_COLS, st);
-  switch (sh.n1)
-  {
-    case 2: launch_ifb_cols<2> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 3: launch_ifb_cols<3> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 4: launch_ifb_cols<4> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 6: launch_ifb_cols<6> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 8: launch_ifb_cols<8> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 12: launch_ifb_cols<12> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 16: launch_ifb_cols<16> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 24: launch_ifb_cols<24> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    case 32: launch_ifb_cols<32> (sh, tb, part0, nbatch, scratch, vv, st); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError ();
 }
 
 cudaError_t launch_build_chirp (float2* H, const double* d_chan_freq, const double* d_coeff,
@@ -3272,7 +1057,7 @@ cudaError_t launch_colplan (const FoldSegment* segs, int nseg, uint64_t ndat, un
 {
   if (ndat == 0) return cudaSuccess;
   g_launches++;
-  const uint64_t per_block = uint64_t (256) * COLPLAN_GROUPS;
+  const uint64_t per_block = uint64_t (256 / 32) * COLPLAN_SAMPLES;
   k_colplan<<<unsigned ((ndat + per_block - 1) / per_block), 256, 0, st>>> (segs, nseg, ndat,
                                                                            nbin, cols);
   return cudaGetLastError ();
