@@ -1081,7 +1081,7 @@ int pipeline_block (dspsr_b200_pipeline* pl, const void* d_in, uint64_t ndat_new
   in.npol = cfg.npol;
   in.offset_binary = cfg.offset_binary;
   in.fb_nsub = fbraw ? pl->fb_nsub : 0;
-  in.lut_scale = fbraw ? pl->lut_scale : 0.f;
+  in.lut_scale = in.kind == IN_INT8 ? pl->lut_scale : 0.f;
 
   uint64_t npart = 0;
   if (ndat >= sh.nfft) npart = (ndat - nfilt) / sh.nkeep;   // Convolution.C:486-487
@@ -1874,6 +1874,7 @@ int dspsr_b200_filterbank_during_perform (dspsr_b200_filterbank_during* f, int i
   in.nchan = s.nchan_in;
   in.npol = s.npol;
   in.offset_binary = offset_binary;
+  if (input_kind == DSPSR_B200_INT8_TFPD) in.lut_scale = affine_lut_scale (lut256);
   VoltView vv {reinterpret_cast<float2*> (d_out), out_span};
   FoldView fv {};
   const DuringTables tb = f->tables ();
@@ -1927,6 +1928,7 @@ int dspsr_b200_filterbank_during_perform_fold (dspsr_b200_filterbank_during* f, 
   in.nchan = s.nchan_in;
   in.npol = s.npol;
   in.offset_binary = offset_binary;
+  if (input_kind == DSPSR_B200_INT8_TFPD) in.lut_scale = affine_lut_scale (lut256);
   VoltView vv {nullptr, 0};
   const FoldView fv = fold->view (state, nout, fold->nchan);
   const DuringTables tb = f->tables ();

@@ -21,6 +21,7 @@
 // does (Convolution.C:401-414).
 
 #include "fwd_cols.cuh"
+#include "fwd_cols_pair.cuh"
 #include "inv_cols.cuh"
 #include "rows32.cuh"
 
@@ -527,6 +528,12 @@ cudaError_t run_fourstep_n1 (const ConvShape& sh, const ConvTables& tb, const In
       k_fwd_cols_fb64<IN_INT16, false><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep,
                                                                            part0, sh.n2, tb.tw4,
                                                                            scratch);
+  }
+  else if (in.npol == 2 && fwd_pair_aligned (in))
+  {
+    ClockScope cs (clk, KK_FWD_COLS, st);
+    launch_fwd_pair<N1> (in, tb.lut, sh.nkeep, part0, nbatch, sh.n2, tb.tw4, scratch, tb.apod,
+                         tb.nsm, st);
   }
   else
   {

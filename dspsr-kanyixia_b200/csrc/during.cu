@@ -1,6 +1,7 @@
 // during.cu -- the filterbank with a response (FilterbankEngineCPU.C:379-535)
 
 #include "fwd_cols.cuh"
+#include "fwd_cols_pair.cuh"
 #include "inv_cols.cuh"
 #include "rows32.cuh"
 
@@ -532,7 +533,13 @@ cudaError_t run_during_n1 (const DuringShape& sh, const DuringTables& tb, const 
   const dim3 gfwd (sh.n2 / fwd_cols_per_block<N1> (), nbatch, sh.nchan_in);
   {
     ClockScope cs (clk, KK_FWD_COLS, st);
-    if (in.kind == IN_INT8)
+    if (N1 > 1 && in.npol == 2 && fwd_pair_aligned (in))
+    {
+      if constexpr (N1 > 1)
+        launch_fwd_pair<N1> (in, tb.lut, sh.in_step, part0, nbatch, sh.n2, tb.tw4, scratch, tb.apod,
+                             tb.nsm, st);
+    }
+    else if (in.kind == IN_INT8)
       k_fwd_cols<N1, IN_INT8><<<gfwd, 128, 0, st>>> (in, tb.lut, sh.in_step, part0, sh.n2, tb.tw4,
                                                      scratch, tb.apod);
     else if (in.kind == IN_INT16)
