@@ -409,15 +409,18 @@ struct dspsr_b200_fold
   // another stream has already given the copy engine.
   cudaStream_t up = nullptr;
   cudaEvent_t plan_ev = nullptr;
-  int set_plan (std::vector<FoldSegment>& segs, uint64_t n)
+  int set_plan (std::vector<FoldSegment>& segs, uint64_t n, double turns)
   {
+    pps = turns;
     plan.swap (segs);
     return upload_plan (n);
   }
+  double pps = 0;                     // turns per sample of the current plan
   // builds the exact plan on the host and uploads it on the context's stream
-  int set_bins (double phi, double pps, uint64_t n, double* x_end = nullptr)
+  int set_bins (double phi, double turns, uint64_t n, double* x_end = nullptr)
   {
-    build_fold_plan (phi, pps, n, &plan, x_end);
+    pps = turns;
+    build_fold_plan (phi, turns, n, &plan, x_end);
     return upload_plan (n);
   }
   int upload_plan (uint64_t n)
@@ -492,6 +495,7 @@ struct dspsr_b200_fold
     v.cols = use_cols && ndat && nseg ? d_cols[cur].ptr : nullptr;
     v.state = state;
     v.nout = nout;
+    v.long_bins = pps * nbin * 64 <= 1.0;
     return v;
   }
   void release ()
@@ -755,7 +759,7 @@ int pipeline_subint_plan (dspsr_b200_pipeline* pl, uint64_t out_base, uint64_t t
     cursor = a.idat_start + a.ndat;
   }
   if (cursor < nout || plan.empty ()) skip (cursor);
-  return pl->fold.set_plan (plan, nout);
+  return pl->fold.set_plan (plan, nout, pps);
 }
 
 // hands closed sub-integration slot k to the caller's buffers (or to the

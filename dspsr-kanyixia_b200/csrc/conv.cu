@@ -22,7 +22,7 @@
 
 #include "fwd_cols.cuh"
 #include "fwd_cols_pair.cuh"
-#include "inv_cols.cuh"
+#include "inv_cols_split.cuh"
 #include "rows32.cuh"
 
 namespace b200 {
@@ -271,6 +271,8 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
   const unsigned c = blockIdx.z;
   const uint64_t N = uint64_t (N1) * n2;
   const uint64_t tbase0 = (part0 + b) * nkeep;
+  float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
+  unsigned* hits = c == 0 ? fv.hits : nullptr;
   if constexpr (N1 == 32)
   {
     // Two threads per column (16 columns per warp): thread h = lane & 1 of a
@@ -329,48 +331,27 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
         }
       }
       else
-        emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][j], v[NPOL - 1][j]);
+        detect_fold<NOUT> (fv, NPOL, fold_column (fv, ok, t), v[0][j], v[NPOL - 1][j], prof, hits);
     }
     return;
   }
   const unsigned i2 = blockIdx.x * blockDim.x + threadIdx.x;
-  if constexpr (stage_first_pol<N1, NPOL> ())
-
-  {
-    __shared__ float2 s0[N1 * 128];
-    const float2* src = scratch + (uint64_t (b) * nchan + c) * 2 * N + i2;
-    {
-      float2 v[N1];
-      inv_column<N1> (src, n2, tw4 + i2, n2, v);
-#pragma unroll
-      for (int k = 0; k < N1; k++) s0[k * 128 + threadIdx.x] = v[k];
-    }
-    float2 q[N1];
-    inv_column<N1> (src + N, n2, tw4 + i2, n2, q);
-#pragma unroll (N1 >= 32 ? 2 : N1)
-    for (int k = 0; k < N1; k++)
-    {
-      const uint64_t tl = uint64_t (k) * n2 + i2;
-      const bool ok = tl >= nfilt_pos && tl < nfilt_pos + nkeep;
-      const uint64_t t = tbase0 + (tl - nfilt_pos);
-      const float2 p = s0[k * 128 + threadIdx.x];
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        if (ok)
-        {
-          vv.out[(uint64_t (c) * 2) * vv.span + t] = p;
-          vv.out[(uint64_t (c) * 2 + 1) * vv.span + t] = q[k];
-        }
-      }
-      else
-        emit_fold<NOUT> (fv, c, 2, ok, t, p, q[k]);
-    }
-    return;
-  }
   float2 w[N1];
 #pragma unroll
   for (int k = 1; k < N1; k++)
     w[k] = __ldg (tw4 + uint64_t (k) * n2 + i2);
+  // the profile columns, asked for with the values
+  unsigned fcol[MODE == OUT_FOLD ? N1 : 1];
+  if constexpr (MODE == OUT_FOLD)
+  {
+#pragma unroll
+    for (int k = 0; k < N1; k++)
+    {
+      const uint64_t tl = uint64_t (k) * n2 + i2;
+      const bool ok = tl >= nfilt_pos && tl < nfilt_pos + nkeep;
+      fcol[k] = fold_column (fv, ok, tbase0 + (tl - nfilt_pos));
+    }
+  }
   float2 v[NPOL][N1];
 #pragma unroll
   for (int p = 0; p < NPOL; p++)
@@ -379,6 +360,10 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
 #pragma unroll
     for (int k = 0; k < N1; k++)
       v[p][k] = src[uint64_t (k) * n2];
+  }
+#pragma unroll
+  for (int p = 0; p < NPOL; p++)
+  {
     // conjugate four-step twiddle, then the inverse n1-point DFT
 #pragma unroll
     for (int k = 1; k < N1; k++)
@@ -402,7 +387,7 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
       }
     }
     else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][k], v[NPOL - 1][k]);
+      detect_fold<NOUT> (fv, NPOL, fcol[k], v[0][k], v[NPOL - 1][k], prof, hits);
   }
 }
 
@@ -453,6 +438,8 @@ k_fused (const InputView in, const float* __restrict__ lut, const float2* __rest
     smem_fft<N, T, +1> (sp, tw);
   }
   const uint64_t tbase = part * nkeep;
+  float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
+  unsigned* hits = c == 0 ? fv.hits : nullptr;
   const unsigned rounds = unsigned ((nkeep + T - 1) / T);
   for (unsigned r = 0; r < rounds; r++)
   {
@@ -470,7 +457,7 @@ k_fused (const InputView in, const float* __restrict__ lut, const float2* __rest
       }
     }
     else
-      emit_fold<NOUT> (fv, c, npol, ok, tbase + j, pv, qv);
+      detect_fold<NOUT> (fv, npol, fold_column (fv, ok, tbase + j), pv, qv, prof, hits);
   }
 }
 
@@ -482,9 +469,18 @@ template <int N1, int NPOL, int MODE, int NOUT>
 void launch_inv (const ConvShape& sh, dim3 grid, float2* scratch, uint64_t part0,
                  const ConvTables& tb, const FoldView& fv, const VoltView& vv, cudaStream_t st)
 {
+  if constexpr (N1 >= 8 && NPOL == 2)
+  {
+    launch_inv_split<N1, MODE, NOUT> (scratch, {sh.n2, sh.n2, sh.nchan, sh.nkeep, sh.nfilt_pos},
+                                      part0, grid.y, tb.tw4, tb.nsm, fv, vv, st);
+    return;
+  }
+  else
+  {
   if (N1 == 32) grid.x = sh.n2 / 64;        // two threads per column
   k_inv_cols<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh.n2, sh.nchan, sh.nkeep,
                                                           sh.nfilt_pos, part0, tb.tw4, fv, vv);
+  }
 }
 
 template <int N2>

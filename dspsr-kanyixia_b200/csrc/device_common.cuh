@@ -186,78 +186,182 @@ __device__ __forceinline__ unsigned warp_fold_bin (const FoldSegment* __restrict
   return (base == FOLD_SKIP || bin >= nbin) ? NO_COLUMN : base + bin;
 }
 
-// All 32 lanes call this together.  Lanes holding consecutive time samples
-// with equal bins form runs; each run is summed by a segmented shuffle
-// reduction and added to the profile by its first lane with one atomic.
-template <int NOUT, bool HITS>
-__device__ __forceinline__ void warp_fold_t (bool ok, unsigned bin, const float* v,
-                                             float* prof, unsigned nbin, unsigned* hits)
+// Sums of the runs of equal columns in a row (one sample per lane), hm the
+// ballot of the lanes that begin a run: a segmented shuffle reduction (a lane
+// takes from the lane off further on while that one is in its run, which hm
+// tells without asking the other lane), then one atomic per run from its first
+// lane, the runs of a row in one instruction.  v is ignored where col is
+// NO_COLUMN.
+template <int NOUT>
+__device__ __forceinline__ void fold_runs (unsigned hm, unsigned col, const float* v, float* prof,
+                                           unsigned stride, unsigned* hits)
 {
   const int lane = threadIdx.x & 31;
-  const unsigned key = ok ? bin : 0xffffffffu;
-  const unsigned prev = __shfl_up_sync (FULL, key, 1);
-  const bool head = (lane == 0) || (prev != key);
-  const unsigned hm = __ballot_sync (FULL, head);
-  const int rid = __popc (hm & (FULL >> (31 - lane)));
+  const unsigned later = (hm >> lane) >> 1;              // heads after this lane
+  const int rest = later ? __ffs (later) - 1 : 31 - lane;  // lanes of the run after this one
   float acc[NOUT];
 #pragma unroll
-  for (int k = 0; k < NOUT; k++) acc[k] = ok ? v[k] : 0.0f;
-  int cnt = ok ? 1 : 0;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1)
+  for (int k = 0; k < NOUT; k++) acc[k] = v[k];
+  if (hm != FULL)                      // some run is longer than one
   {
-    const int orid = __shfl_down_sync (FULL, rid, off);
-    const bool take = (lane + off < 32) && (orid == rid);
 #pragma unroll
-    for (int k = 0; k < NOUT; k++)
+    for (int off = 1; off < 32; off <<= 1)
     {
-      const float o = __shfl_down_sync (FULL, acc[k], off);
-      if (take) acc[k] += o;
-    }
-    if constexpr (HITS)
-    {
-      const int oc = __shfl_down_sync (FULL, cnt, off);
-      if (take) cnt += oc;
+      const bool take = off <= rest;
+#pragma unroll
+      for (int k = 0; k < NOUT; k++)
+      {
+        const float o = __shfl_down_sync (FULL, acc[k], off);
+        if (take) acc[k] += o;
+      }
     }
   }
-  if (head && ok)
+  if ((hm >> lane & 1) && col != NO_COLUMN)
   {
 #pragma unroll
-    for (int k = 0; k < NOUT; k++)
-      atomicAdd (prof + uint64_t (k) * nbin + bin, acc[k]);
-    if constexpr (HITS) atomicAdd (hits + bin, unsigned (cnt));
+    for (int k = 0; k < NOUT; k++) atomicAdd (prof + uint64_t (k) * stride + col, acc[k]);
+    if (hits) atomicAdd (hits + col, unsigned (rest + 1));
   }
 }
 
-// Only the warps that count hits (one channel's) reduce the counts; hits is
-// the same pointer in every lane, so the choice is warp-uniform.
-template <int NOUT>
-__device__ __forceinline__ void warp_fold (bool ok, unsigned bin, const float* v,
-                                           float* prof, unsigned nbin, unsigned* hits)
+// Fold of a warp's detected samples where a bin is long (FoldView::long_bins),
+// K rows of 32 lanes at a time (a row: the samples the lanes hold for one value
+// of a kernel's sample loop).  put() leaves a row in the warp's shared buffer;
+// flush() finds the rows that have one column -- most of them -- and has 1 to
+// 8 lanes sum each (row, product), 32 values in eight 16-byte loads, one atomic
+// each; the others go to fold_runs in one rolled loop.  Against fold_runs for
+// every row (5 x NOUT shuffles) C1's inverse columns went from 239 to 162 us
+// with the rest of the pass; with 11 samples a bin (C2) the detour through
+// shared memory is slower, 803 against 664 us at n1 = 8.  Rows of 36 words: the
+// row-wise accesses and the 16-byte loads of 8 lanes fall in distinct banks.
+template <int NOUT, int K>
+struct RowFold
 {
-  if (hits)
-    warp_fold_t<NOUT, true> (ok, bin, v, prof, nbin, hits);
-  else
-    warp_fold_t<NOUT, false> (ok, bin, v, prof, nbin, hits);
+  static_assert (NOUT * K <= 32, "a row and product per lane");
+  static constexpr int ROWS = K;
+  static constexpr int LD = 36;
+  static constexpr int WORDS = (NOUT + 1) * K * LD;      // per warp
+  float* vals;                                           // [row * NOUT + product][LD]
+  unsigned* cols;                                        // [row][LD]
+  float* prof;
+  unsigned stride;
+  unsigned* hits;
+  int n = 0;                                             // rows held (warp-uniform)
+
+  __device__ __forceinline__ RowFold (float* warp_buffer, float* p, unsigned st, unsigned* h)
+    : vals (warp_buffer), cols (reinterpret_cast<unsigned*> (warp_buffer + NOUT * K * LD)),
+      prof (p), stride (st), hits (h)
+  {}
+
+  // all 32 lanes, with room for a row (n < K); v is ignored where col is NO_COLUMN
+  __device__ __forceinline__ void put (unsigned col, const float* v)
+  {
+    const int lane = threadIdx.x & 31;
+    cols[n * LD + lane] = col;
+#pragma unroll
+    for (int o = 0; o < NOUT; o++) vals[(n * NOUT + o) * LD + lane] = v[o];
+    n++;
+  }
+
+  __device__ __forceinline__ void flush ()
+  {
+    if (n == 0) return;
+    const int lane = threadIdx.x & 31;
+    unsigned whole = 0;                // rows with one column
+#pragma unroll 1
+    for (int r = 0; r < n; r++)
+    {
+      // each lane reads back what it stored
+      const unsigned col = cols[r * LD + lane];
+      const unsigned prev = __shfl_up_sync (FULL, col, 1);
+      const unsigned hm = __ballot_sync (FULL, lane == 0 || prev != col);
+      if (hm == 1)
+      {
+        if (col != NO_COLUMN) whole |= 1u << r;
+        continue;
+      }
+      float v[NOUT];
+#pragma unroll
+      for (int o = 0; o < NOUT; o++) v[o] = vals[(r * NOUT + o) * LD + lane];
+      fold_runs<NOUT> (hm, col, v, prof, stride, hits);
+    }
+    if (whole)
+    {
+      __syncwarp ();
+      const int rows = n * NOUT;
+      const int lg = rows > 16 ? 0 : rows > 8 ? 1 : rows > 4 ? 2 : 3;
+      const int sub = lane & ((1 << lg) - 1), len = 32 >> lg;
+      const int row = min (lane >> lg, rows - 1);
+      const float4* vp = reinterpret_cast<const float4*> (vals + row * LD + sub * len);
+      float4 acc = vp[0];
+      for (int i = 1; i < len / 4; i++)
+      {
+        const float4 x = vp[i];
+        acc.x += x.x;
+        acc.y += x.y;
+        acc.z += x.z;
+        acc.w += x.w;
+      }
+      float a = (acc.x + acc.y) + (acc.z + acc.w);
+      for (int off = 1; off < (1 << lg); off <<= 1) a += __shfl_xor_sync (FULL, a, off);
+      const int k = row / NOUT, o = row % NOUT;
+      if (sub == 0 && (lane >> lg) < rows && (whole >> k & 1))
+      {
+        const unsigned col = cols[k * LD];
+        atomicAdd (prof + uint64_t (o) * stride + col, a);
+        if (hits && o == 0) atomicAdd (hits + col, 32u);
+      }
+      __syncwarp ();
+    }
+    n = 0;
+  }
+};
+
+// The profile column of sample t of every lane (NO_COLUMN where !ok).
+__device__ __forceinline__ unsigned fold_column (const FoldView& fv, bool ok, uint64_t t)
+{
+  const unsigned col = fv.cols ? (ok ? __ldg (fv.cols + t) : NO_COLUMN)
+                               : warp_fold_bin (fv.segs, fv.nseg, ok, t, fv.nbin);
+  return col < fv.stride ? col : NO_COLUMN;
 }
 
+// One row folded at once.
 template <int NOUT>
-__device__ __forceinline__ void emit_fold (const FoldView& fv, unsigned c, unsigned npol, bool ok,
-                                           uint64_t t, float2 p, float2 q)
+__device__ __forceinline__ void fold_row (unsigned col, const float* v, float* prof,
+                                          unsigned stride, unsigned* hits)
 {
-  // a warp whose samples all fall in the overlap discard has nothing to add
-  // (all 32 lanes are here, so the vote and the return are warp-uniform)
-  if (!__any_sync (FULL, ok)) return;
+  const unsigned prev = __shfl_up_sync (FULL, col, 1);
+  const unsigned hm = __ballot_sync (FULL, (threadIdx.x & 31) == 0 || prev != col);
+  fold_runs<NOUT> (hm, col, v, prof, stride, hits);
+}
+
+// Detects a row and folds it: LONG rows wait in rf (the caller flushes after
+// every RowFold::ROWS calls), others are folded at once.  A row with no column
+// to go to -- all in the overlap discard -- has nothing to add (the vote is
+// warp-uniform).  Callers ask for the columns (fold_column) with the values
+// they belong to: loaded here, each row would wait for memory in turn.
+template <bool LONG, int NOUT, int K>
+__device__ __forceinline__ void detect_row (RowFold<NOUT, K>& rf, int state, unsigned npol,
+                                            unsigned col, float2 p, float2 q)
+{
+  if (!__any_sync (FULL, col != NO_COLUMN)) return;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
-  unsigned bin = fv.cols ? (ok ? __ldg (fv.cols + t) : NO_COLUMN)
-                         : warp_fold_bin (fv.segs, fv.nseg, ok, t, fv.nbin);
-  if (ok)
-  {
-    detect_values (fv.state, npol, p, q, v);
-    ok = bin < fv.stride;
-  }
-  warp_fold<NOUT> (ok, bin, v, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride,
-                   c == 0 ? fv.hits : nullptr);
+  detect_values (state, npol, p, q, v);
+  if constexpr (LONG)
+    rf.put (col, v);
+  else
+    fold_row<NOUT> (col, v, rf.prof, rf.stride, rf.hits);
+}
+
+// The same without a RowFold.
+template <int NOUT>
+__device__ __forceinline__ void detect_fold (const FoldView& fv, unsigned npol, unsigned col,
+                                             float2 p, float2 q, float* prof, unsigned* hits)
+{
+  if (!__any_sync (FULL, col != NO_COLUMN)) return;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  detect_values (fv.state, npol, p, q, v);
+  fold_row<NOUT> (col, v, prof, fv.stride, hits);
 }
 
 } // namespace

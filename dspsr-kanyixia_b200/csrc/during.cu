@@ -2,7 +2,7 @@
 
 #include "fwd_cols.cuh"
 #include "fwd_cols_pair.cuh"
-#include "inv_cols.cuh"
+#include "inv_cols_split.cuh"
 #include "rows32.cuh"
 
 namespace b200 {
@@ -187,39 +187,8 @@ k_inv_cols_during (const float2* __restrict__ scratch, const DuringShape sh, con
   const uint64_t N = uint64_t (N1) * sh.n2;
   const unsigned cs = i2 / sh.seg, t2 = i2 % sh.seg;
   const unsigned c = cin * sh.nsub + cs;
-  if constexpr (stage_first_pol<N1, NPOL> ())
-  {
-    __shared__ float2 s0[N1 * 128];
-    const float2* src = scratch + (uint64_t (b) * sh.nchan_in + cin) * 2 * N + i2;
-    {
-      float2 v[N1];
-      inv_column<N1> (src, sh.n2, twd + t2, sh.seg, v);
-#pragma unroll
-      for (int k = 0; k < N1; k++) s0[k * 128 + threadIdx.x] = v[k];
-    }
-    float2 q[N1];
-    inv_column<N1> (src + N, sh.n2, twd + t2, sh.seg, q);
-    const uint64_t tb = (part0 + b) * sh.nkeep;
-#pragma unroll (N1 >= 32 ? 2 : N1)
-    for (int k = 0; k < N1; k++)
-    {
-      const uint64_t tl = uint64_t (k) * sh.seg + t2;
-      const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
-      const uint64_t t = tb + (tl - sh.nfilt_pos);
-      const float2 p = s0[k * 128 + threadIdx.x];
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        if (ok)
-        {
-          vv.out[(uint64_t (c) * 2) * vv.span + t] = p;
-          vv.out[(uint64_t (c) * 2 + 1) * vv.span + t] = q[k];
-        }
-      }
-      else
-        emit_fold<NOUT> (fv, c, 2, ok, t, p, q[k]);
-    }
-    return;
-  }
+  float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
+  unsigned* hits = c == 0 ? fv.hits : nullptr;
   float2 w[N1];
 #pragma unroll
   for (int k = 1; k < N1; k++)
@@ -254,7 +223,7 @@ k_inv_cols_during (const float2* __restrict__ scratch, const DuringShape sh, con
       }
     }
     else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, v[0][k], v[NPOL - 1][k]);
+      detect_fold<NOUT> (fv, NPOL, fold_column (fv, ok, t), v[0][k], v[NPOL - 1][k], prof, hits);
   }
 }
 
@@ -457,6 +426,8 @@ k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
   const uint64_t tbase = (part0 + b) * sh.nkeep;
   const float2* c0p = s_cb;
   const float2* c1p = s_cb + (NPOL - 1) * CW * SP;
+  float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
+  unsigned* hits = c == 0 ? fv.hits : nullptr;
   for (int e = threadIdx.x; e < CW * N1; e += T)
   {
     const int j = e % CW, t1 = e / CW;
@@ -474,7 +445,7 @@ k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
       }
     }
     else
-      emit_fold<NOUT> (fv, c, NPOL, ok, t, pv, qv);
+      detect_fold<NOUT> (fv, NPOL, fold_column (fv, ok, t), pv, qv, prof, hits);
   }
 }
 
@@ -504,8 +475,12 @@ void launch_inv_during (const DuringShape& sh, dim3 grid, const float2* scratch,
                         const DuringTables& tb, const FoldView& fv, const VoltView& vv,
                         cudaStream_t st)
 {
-  k_inv_cols_during<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh, part0, tb.twd, fv,
-                                                                 vv);
+  if constexpr (N1 >= 8 && N1 <= 32 && NPOL == 2)
+    launch_inv_split<N1, MODE, NOUT> (scratch, {sh.n2, sh.seg, sh.nchan_in, sh.nkeep, sh.nfilt_pos},
+                                      part0, grid.y, tb.twd, tb.nsm, fv, vv, st);
+  else
+    k_inv_cols_during<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh, part0, tb.twd, fv,
+                                                                   vv);
 }
 
 template <int N1, int NPOL>

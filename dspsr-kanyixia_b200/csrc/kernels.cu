@@ -450,21 +450,47 @@ __global__ void k_detect (const float2* __restrict__ in, const uint64_t in_span,
     out[(uint64_t (c) * nout + k) * out_span + t] = v[k];
 }
 
-// Fold::Engine::fold on detected FPT floats (ndim 1): one warp covers 32
-// consecutive samples of one (chan, pol).
-__global__ void k_fold (const float* __restrict__ in, const uint64_t in_span,
-                        const uint64_t ndat, const unsigned npol, const FoldView fv)
+// Fold::Engine::fold on detected FPT floats (ndim 1): a warp takes
+// 32 * FOLD_K consecutive samples of NP products of one channel (all of them
+// when there are 1, 2 or 4; otherwise one per blockIdx.z), so that
+// RowFold sums whole sets of rows.  Bound by issue and by the
+// latency of its loads.
+constexpr int FOLD_K = 8;
+
+template <int NP, bool LONG>
+__global__ void __launch_bounds__ (128)
+k_fold (const float* __restrict__ in, const uint64_t in_span, const uint64_t ndat,
+        const unsigned npol, const FoldView fv)
 {
-  const uint64_t t = uint64_t (blockIdx.x) * blockDim.x + threadIdx.x;
+  using RF = RowFold<NP, FOLD_K>;
+  __shared__ __align__ (16) float s_fold[LONG ? 4 * RF::WORDS : 4];
+  const unsigned lane = threadIdx.x & 31;
+  const uint64_t t0 = (uint64_t (blockIdx.x) * 4 + (threadIdx.x >> 5)) * (32 * FOLD_K) + lane;
   const unsigned c = blockIdx.y;
-  bool ok = t < ndat;
-  const unsigned bin = warp_fold_bin (fv.segs, fv.nseg, ok, t, fv.nbin);
-  ok = ok && bin < fv.stride;
-  for (unsigned p = 0; p < npol; p++)
+  for (unsigned z = blockIdx.z; z < npol / NP; z += gridDim.z)
   {
-    float v = ok ? in[(uint64_t (c) * npol + p) * in_span + t] : 0.f;
-    warp_fold<1> (ok, bin, &v, fv.profiles + (uint64_t (c) * npol + p) * fv.stride, fv.stride,
-                  (c == 0 && p == 0) ? fv.hits : nullptr);
+    const uint64_t row0 = uint64_t (c) * npol + z * NP;
+    RF rf (s_fold + (LONG ? (threadIdx.x >> 5) * RF::WORDS : 0), fv.profiles + row0 * fv.stride, fv.stride,
+           row0 == 0 ? fv.hits : nullptr);
+    float v[FOLD_K][NP];
+  #pragma unroll
+    for (int k = 0; k < FOLD_K; k++)
+  #pragma unroll
+      for (int p = 0; p < NP; p++)
+        v[k][p] = t0 + 32 * k < ndat ? __ldg (in + (row0 + p) * in_span + t0 + 32 * k) : 0.f;
+      unsigned col[FOLD_K];
+#pragma unroll
+    for (int k = 0; k < FOLD_K; k++) col[k] = fold_column (fv, t0 + 32 * k < ndat, t0 + 32 * k);
+#pragma unroll
+    for (int k = 0; k < FOLD_K; k++)
+    {
+      if (!__any_sync (FULL, col[k] != NO_COLUMN)) continue;
+      if constexpr (LONG)
+        rf.put (col[k], v[k]);
+      else
+        fold_row<NP> (col[k], v[k], rf.prof, rf.stride, rf.hits);
+    }
+    if constexpr (LONG) rf.flush ();
   }
 }
 
@@ -486,7 +512,12 @@ __global__ void k_delay_fold (const float2* __restrict__ v, const uint64_t span,
     p = v[(uint64_t (c) * npol) * span + i];
     if (npol == 2) q = v[(uint64_t (c) * npol + 1) * span + i];
   }
-  emit_fold<NOUT> (fv, c, npol, ok, t, p, q);
+  if (!__any_sync (FULL, ok)) return;
+  const unsigned col = fold_column (fv, ok, t);
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  detect_values (fv.state, npol, p, q, d);
+  fold_row<NOUT> (col, d, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride,
+                  c == 0 ? fv.hits : nullptr);
 }
 
 // SpectralKurtosis::detect_skfb (SpectralKurtosis.C:1105-1222) from sums
@@ -720,7 +751,7 @@ __global__ void k_zeroed_fold (const float2* __restrict__ v, const uint64_t span
 {
   const uint64_t t = uint64_t (blockIdx.x) * blockDim.x + threadIdx.x;
   const unsigned c = blockIdx.y;
-  bool ok = t < ndat;
+  const bool ok = t < ndat;
   if (!__any_sync (FULL, ok)) return;
   float2 p = make_float2 (0.f, 0.f), q = make_float2 (0.f, 0.f);
   if (ok)
@@ -728,16 +759,12 @@ __global__ void k_zeroed_fold (const float2* __restrict__ v, const uint64_t span
     p = v[(uint64_t (c) * npol) * span + t];
     if (npol == 2) q = v[(uint64_t (c) * npol + 1) * span + t];
   }
+  unsigned col = fold_column (fv, ok, t);
   float d[4] = {0.f, 0.f, 0.f, 0.f};
-  const unsigned bin = fv.cols ? (ok ? __ldg (fv.cols + t) : NO_COLUMN)
-                               : warp_fold_bin (fv.segs, fv.nseg, ok, t, fv.nbin);
-  if (ok)
-  {
-    detect_values (fv.state, npol, p, q, d);
-    // a zeroed sample adds nothing to the profile and counts no hit
-    ok = bin < fv.stride && d[0] != 0.f;
-  }
-  warp_fold<NOUT> (ok, bin, d, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride, fv.hits);
+  detect_values (fv.state, npol, p, q, d);
+  // a zeroed sample adds nothing to the profile and counts no hit
+  if (d[0] == 0.f) col = NO_COLUMN;
+  fold_row<NOUT> (col, d, fv.profiles + uint64_t (c) * NOUT * fv.stride, fv.stride, fv.hits);
 }
 
 // Segment holding sample t, found by a whole warp: each round probes 32
@@ -1047,8 +1074,16 @@ cudaError_t launch_fold (const float* in, uint64_t in_span, uint64_t ndat, unsig
 {
   if (ndat == 0) return cudaSuccess;
   g_launches++;
-  k_fold<<<dim3 (unsigned ((ndat + 255) / 256), nchan), 256, 0, st>>> (in, in_span, ndat, npol,
-                                                                        fv);
+  const unsigned gx = unsigned ((ndat + 128 * FOLD_K - 1) / (128 * FOLD_K));
+  const auto run = [&] (auto kern, unsigned gz) {
+    kern<<<dim3 (gx, nchan, gz), 128, 0, st>>> (in, in_span, ndat, npol, fv);
+  };
+  if (npol == 4)
+    run (fv.long_bins ? k_fold<4, true> : k_fold<4, false>, 1);
+  else if (npol == 2)
+    run (fv.long_bins ? k_fold<2, true> : k_fold<2, false>, 1);
+  else
+    run (fv.long_bins ? k_fold<1, true> : k_fold<1, false>, std::min (npol, 65535u));
   return cudaGetLastError ();
 }
 

@@ -52,6 +52,9 @@ struct FoldView
   const unsigned* cols = nullptr;
   int state;
   int nout;
+  // 64 samples and more per bin: at least half the rows of 32 consecutive
+  // samples lie in one bin, and the column passes sum whole rows (RowFold)
+  bool long_bins = false;
 };
 
 // Voltage epilogue (Convolution::Engine::perform output)
