@@ -126,6 +126,16 @@ std::vector<float2> make_tw4 (unsigned n1, unsigned n2)
 // convolution engine
 // ---------------------------------------------------------------------------
 
+namespace {
+
+// The four-step row length when the caller names none: 4096-point rows
+// (k_rows64) for transforms of 16384 to 65536 points, whose 4- to 16-point
+// columns fit one thread for both polarisations; 8192-point rows above, and
+// the single-kernel transforms below.
+unsigned default_row_length (unsigned nfft) { return nfft >= 16384 && nfft <= 65536 ? 4096 : 8192; }
+
+} // namespace
+
 struct dspsr_b200_convolution
 {
   dspsr_b200_context* ctx = nullptr;
@@ -142,10 +152,17 @@ struct dspsr_b200_convolution
 
   int set_fft_precision (int mode);
 
-  // row_len: the four-step row length, 8192 (0 = default) or 4096 (nfft
-  // from 8192 to 131072: then n1 = nfft / 4096 columns)
+  uint64_t budget = 0;        // scratch bytes (parts in flight)
+  bool row_fixed = false;     // the caller named the row length
+
+  // row_len: the four-step row length, 4096 (nfft from 8192 to 131072: then
+  // n1 = nfft / 4096 columns), 8192, or 0 for default_row_length
   int init (dspsr_b200_context* c, unsigned nchan, unsigned npol, unsigned nfft,
             unsigned pos, unsigned neg, uint64_t scratch_bytes, unsigned row_len = 0);
+  // n1, n2, their tables, the batch and its scratch
+  int split (unsigned row_len);
+  // changes the row length of an engine in use (its response follows)
+  int resplit (unsigned row_len);
   ConvTables tables () const
   {
     ConvTables t;
@@ -208,11 +225,23 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
   if (row_len != 0 && row_len != 4096 && row_len != 8192)
     return fail (ctx, DSPSR_B200_EINVAL, "convolution: row length %u is not 4096 or 8192",
                  row_len);
+  if (row_len == 4096 && nfft > 131072)
+    return fail (ctx, DSPSR_B200_EINVAL,
+                 "convolution: 4096-point rows need nfft <= 131072 (nfft=%u)", nfft);
+  row_fixed = row_len != 0;
+  budget = scratch_bytes ? scratch_bytes : (uint64_t (512) << 20);
+  const int rc = split (row_len ? row_len : default_row_length (nfft));
+  if (rc) return rc;
+  B200_CHECK (ctx, H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
+  B200_CHECK (ctx, lut.reserve (256), "cudaMalloc lut");
+  return DSPSR_B200_OK;
+}
+
+int dspsr_b200_convolution::split (unsigned row_len)
+{
+  const unsigned nfft = shape.nfft, nchan = shape.nchan, npol = shape.npol;
   if (row_len == 4096 && nfft >= 8192)
   {
-    if (nfft > 131072)
-      return fail (ctx, DSPSR_B200_EINVAL,
-                   "convolution: 4096-point rows need nfft <= 131072 (nfft=%u)", nfft);
     shape.n2 = 4096;
     shape.n1 = nfft / 4096;
   }
@@ -246,7 +275,6 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
     // otherwise, and the batch is chosen so that its rows spread evenly over
     // the persistent row kernel's CTAs.
     const uint64_t per_part = uint64_t (nchan) * npol * nfft * sizeof (float2);
-    const uint64_t budget = scratch_bytes ? scratch_bytes : (uint64_t (512) << 20);
     const uint64_t bmax = std::max<uint64_t> (1, std::min<uint64_t> (65535, budget / per_part));
     const uint64_t rows_per_part = uint64_t (shape.n1) * nchan * npol;
     // (a multiple of the SM count, so also even for the tensor-core rows'
@@ -264,8 +292,25 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
   }
   else
     max_batch = 65535;
-  B200_CHECK (ctx, H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
-  B200_CHECK (ctx, lut.reserve (256), "cudaMalloc lut");
+  return DSPSR_B200_OK;
+}
+
+int dspsr_b200_convolution::resplit (unsigned row_len)
+{
+  if (shape.n1 < 2 || shape.n2 == row_len) return DSPSR_B200_OK;
+  const uint64_t n = uint64_t (shape.nchan) * shape.nfft;
+  if (have_response)
+  {
+    B200_CHECK (ctx, tmp.reserve (n), "cudaMalloc response staging");
+    B200_CHECK (ctx, launch_unpermute_response (tmp.ptr, H.ptr, shape.nchan, shape.n1, shape.n2,
+                                                ctx->stream), "unpermute response");
+  }
+  B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "sync before the new split");
+  const int rc = split (row_len);
+  if (rc) return rc;
+  if (have_response)
+    B200_CHECK (ctx, launch_permute_response (H.ptr, tmp.ptr, shape.nchan, shape.n1, shape.n2,
+                                              ctx->stream), "permute response");
   return DSPSR_B200_OK;
 }
 
@@ -610,6 +655,7 @@ struct dspsr_b200_pipeline
   DevBuf<uint32_t> sk_counts;
   DevBuf<uint8_t> sk_pmask;
   DevBuf<float2> fbbuf;             // filterbank output, FPT
+  DevBuf<uint8_t> aligned_in;       // a misaligned block of the fused filterbank, copied
   float2* fb_tab = nullptr;         // pass tables of the filterbank FFT (fb_nsub >= 128)
   size_t fb_tab_cap = 0;
   // run_host folds a block in pieces: the first piece that folds starts the
@@ -1205,7 +1251,20 @@ int pipeline_input (dspsr_b200_pipeline* pl, const void* d_in, uint64_t ndat, ui
     return fail (ctx, DSPSR_B200_EINVAL, "pipeline: block of %llu samples is not a multiple of "
                  "the %u filterbank channels", (unsigned long long) ndat, pl->fb_nsub);
   if (pl->fb_fused)
+  {
+    // its loads take both polarisations of a sample in one word: a block that
+    // starts between words is copied to an aligned one first
+    const unsigned word = cfg.input_kind == DSPSR_B200_INT8_TFPD ? 4 : 8;
+    if (reinterpret_cast<uintptr_t> (d_in) % word)
+    {
+      const uint64_t bytes = ndat * pl->bytes_per_sample;
+      B200_CHECK (ctx, pl->aligned_in.reserve (bytes), "cudaMalloc aligned input");
+      B200_CHECK (ctx, cudaMemcpyAsync (pl->aligned_in.ptr, d_in, bytes, cudaMemcpyDeviceToDevice,
+                                        ctx->stream), "align input");
+      d_in = pl->aligned_in.ptr;
+    }
     return pipeline_block (pl, d_in, ndat / pl->fb_nsub, 0, ndat_folded);
+  }
   const uint64_t nb = ndat / pl->fb_nsub;
   const uint64_t rows = uint64_t (pl->conv.shape.nchan) * cfg.npol;
   B200_CHECK (ctx, pl->fbbuf.reserve (std::max<uint64_t> (rows * nb, 1)), "cudaMalloc filterbank");
@@ -2562,7 +2621,12 @@ int dspsr_b200_convolution::set_fft_precision (int mode)
   if (mode == DSPSR_B200_FFT_FP32)
   {
     tc_splits = 0;
-    return DSPSR_B200_OK;
+    return row_fixed ? DSPSR_B200_OK : resplit (default_row_length (shape.nfft));
+  }
+  if (!row_fixed && shape.nfft >= 16384)      // the tensor-core rows are 8192 points long
+  {
+    const int rc = resplit (8192);
+    if (rc) return rc;
   }
   if (shape.n1 < 2 || shape.n2 != 8192)
     return fail (ctx, DSPSR_B200_EINVAL,
@@ -2919,10 +2983,11 @@ int dspsr_b200_pipeline_create (dspsr_b200_context* ctx, const dspsr_b200_pipeli
                                pl->sub_on ? unsigned (pl->sub_slots.size ()) : 1);
   pl->fold.use_cols = true;
   // C2's shape -- a 64-channel filterbank of one dual-polarisation int8 or
-  // int16 channel with four-step parts of 8 x n2 -- runs the filterbank
+  // int16 channel with four-step parts of 8 x n2 or 16 x n2 -- runs the filterbank
   // inside the forward column pass: its output never goes through memory
   pl->fb_fused = !rc && fb == 64 && cfg->nchan == 1 && cfg->npol == 2
-                 && cfg->input_kind != DSPSR_B200_FLOAT_FPT && pl->conv.shape.n1 == 8
+                 && cfg->input_kind != DSPSR_B200_FLOAT_FPT
+                 && (pl->conv.shape.n1 == 8 || pl->conv.shape.n1 == 16)
                  && cfg->fused_filterbank >= 0 && cfg->sk_M == 0;
   // SpectralKurtosis between the convolution and detection: its zero-DM
   // input needs the filterbank's channels in memory
@@ -3001,6 +3066,7 @@ int dspsr_b200_pipeline_destroy (dspsr_b200_pipeline* pl)
     if (u.ev) cudaEventDestroy (u.ev);
   }
   pl->fbbuf.release ();
+  pl->aligned_in.release ();
   pl->sd_applied.release ();
   pl->sd_buf[0].release ();
   pl->sd_buf[1].release ();

@@ -21,9 +21,11 @@
 // does (Convolution.C:401-414).
 
 #include "fwd_cols.cuh"
+#include "fb64_cols.cuh"
 #include "fwd_cols_pair.cuh"
 #include "inv_cols_split.cuh"
 #include "rows32.cuh"
+#include "rows64.cuh"
 
 namespace b200 {
 
@@ -55,206 +57,6 @@ __device__ __forceinline__ void smem_fft (float2* s, const float2* tw)
 {
   float2 v[N / T];
   smem_pass<N, T, D, 0> (s, v, tw);
-}
-
-// --------------------------------------------------------------------------
-// K1 with the filterbank in front (Filterbank with freq_res 1 and 64 channels,
-// FilterbankEngineCPU.C:379-535, then the first four-step pass of each
-// channel's convolution), for raw TFPD input of one channel and two
-// polarisations and n1 = 8.  The filterbank's own output never reaches
-// memory: a warp takes one column i2 of one part and computes, for the eight
-// filterbank samples t0 + j*n2 of that column, all 64 channels of both
-// polarisations, then each channel's 8-point column DFT.
-//
-// Lane (j, q), j = lane/4, q = lane%4, reads raw samples s = q + 4m (m < 16)
-// of filterbank sample j: a 16-point DFT over m and the twiddle w64^(q ka)
-// give Y[q][ka] (ka < 16).  One transpose through the warp's shared buffer
-// hands lane 2 ka + pol the 32 values Y[q][ka] of every (q, j): 4-point DFTs
-// over q give channels c = ka + 16 kb (kb < 4) of each filterbank sample,
-// and 8-point DFTs over j the four channels' column DFTs, all in registers
-// (64-point DFT as 16 x 4, X[ka + 16 kb] = sum_q w4^(q kb) w64^(q ka)
-// Y[q][ka]).  The block's four warps (four consecutive
-// columns) stage their outputs in shared memory and write each scratch row
-// in runs of one 32-byte sector (blocks of two or eight warps measured
-// slower).  The transpose's rows are 34 float2 apart, so its stores (one row,
-// 32 lanes) and 16-byte loads (32 rows) are free of bank conflicts.  The staging is column-major with the even and odd rows in two
-// halves (row -> row/2 + (row odd) FBC_SODD, column stride FBC_SP = 2 mod 16):
-// the 16 rows a half-warp stores (two apart) and the 4 x 4 (row, column)
-// pairs it loads for the write-out then fall in 16 distinct bank pairs.
-// --------------------------------------------------------------------------
-
-constexpr int FBC_THREADS = 128;
-constexpr int FBC_COLS = FBC_THREADS / 32;      // columns per block, one per warp
-constexpr int FBC_XROW = 34;                    // exchange row stride (float2; 16-byte reads)
-constexpr int FBC_XSTRIDE = 32 * FBC_XROW;      // float2 per warp exchange buffer
-constexpr int FBC_SODD = 520;                   // staging offset of the odd rows (8 mod 16)
-constexpr int FBC_SP = 1042;                    // staging column stride (2 mod 16)
-constexpr size_t FBC_SMEM =
-    (size_t (FBC_SP) * FBC_COLS > size_t (FBC_COLS) * FBC_XSTRIDE ? size_t (FBC_SP) * FBC_COLS
-                                                                  : size_t (FBC_COLS) * FBC_XSTRIDE)
-    * sizeof (float2);
-
-__host__ __device__ constexpr int fbc_stage (int row, int col)
-{
-  return col * FBC_SP + (row >> 1) + (row & 1) * FBC_SODD;
-}
-
-// (float(x) + 0.5f) * scale for the two's-complement byte x, bit for bit:
-// 2^22 + (x + 128) has its last mantissa bit worth 0.5, so subtracting
-// 2^22 + 127.5 leaves x + 0.5 exactly; no int -> float conversion
-__device__ __forceinline__ float unpack_affine (unsigned byte, float scale)
-{
-  const float big = __int_as_float (0x4a800000u | (((byte & 0xffu) ^ 0x80u) << 1));
-  return __fmul_rn (__fsub_rn (big, 4194431.5f), scale);
-}
-
-// The 8-bit table of the fused filterbank pass is one 1 KB copy in shared
-// memory.  Eight interleaved copies (lane l reading copy l % 8, so a warp's
-// random lookups spread over all banks) measured 10 % slower on the C2 pass:
-// the 8 KB table costs more in occupancy than the bank conflicts it removes.
-
-template <int KIND, bool AFFINE>
-__device__ __forceinline__ void fetch_raw2 (const InputView& in, const float* s_lut, uint64_t r,
-                                            float2& p0, float2& p1)
-{
-  const void* base = in.main;
-  const uint64_t npre = in.npre * 64;
-  if (r < npre)
-    base = in.pre;
-  else
-    r -= npre;
-  if constexpr (KIND == IN_INT8)
-  {
-    const unsigned w = __ldg (static_cast<const unsigned*> (base) + r);
-    if constexpr (AFFINE)
-    {
-      const float sc = in.lut_scale;
-      p0 = make_float2 (unpack_affine (w, sc), unpack_affine (w >> 8, sc));
-      p1 = make_float2 (unpack_affine (w >> 16, sc), unpack_affine (w >> 24, sc));
-    }
-    else
-    {
-      p0 = make_float2 (s_lut[w & 0xff], s_lut[(w >> 8) & 0xff]);
-      p1 = make_float2 (s_lut[(w >> 16) & 0xff], s_lut[w >> 24]);
-    }
-  }
-  else
-  {
-    const uint2 w = __ldg (static_cast<const uint2*> (base) + r);
-    short a = short (w.x & 0xffff), b = short (w.x >> 16);
-    short c = short (w.y & 0xffff), d = short (w.y >> 16);
-    if (in.offset_binary)
-    {
-      a = short (a ^ 0x8000);
-      b = short (b ^ 0x8000);
-      c = short (c ^ 0x8000);
-      d = short (d ^ 0x8000);
-    }
-    p0 = make_float2 (__fadd_rn (float (a), 0.5f), __fadd_rn (float (b), 0.5f));
-    p1 = make_float2 (__fadd_rn (float (c), 0.5f), __fadd_rn (float (d), 0.5f));
-  }
-}
-
-template <int KIND, bool AFFINE>
-__global__ void __launch_bounds__ (FBC_THREADS, 768 / FBC_THREADS)
-k_fwd_cols_fb64 (const InputView in, const float* __restrict__ lut, const uint64_t nkeep,
-                 const uint64_t part0, const unsigned n2, const float2* __restrict__ tw4,
-                 float2* __restrict__ scratch)
-{
-  extern __shared__ __align__ (16) float2 s_fbc[];
-  __shared__ float s_lut[AFFINE ? 1 : 256];
-  __shared__ float2 s_tw64[64];
-  if (!AFFINE && in.kind == IN_INT8)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-      s_lut[i] = lut[i];
-  if (threadIdx.x < 64)
-    s_tw64[threadIdx.x] = make_float2 (cos64 (int (threadIdx.x)), -sin64 (int (threadIdx.x)));
-  __syncthreads ();
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned j = lane >> 2, q = lane & 3;
-  const unsigned i0 = blockIdx.x * FBC_COLS;
-  const unsigned i2 = i0 + warp;
-  const unsigned b = blockIdx.y;
-  const uint64_t N = 8ull * n2;
-  float2* xb = s_fbc + warp * FBC_XSTRIDE;
-
-  // raw samples q + 4m of filterbank sample t, both polarisations
-  const uint64_t t = (part0 + b) * nkeep + i2 + uint64_t (j) * n2;
-  float2 x0[16], x1[16];
-#pragma unroll
-  for (int m = 0; m < 16; m++)
-    fetch_raw2<KIND, AFFINE> (in, s_lut, t * 64 + q + 4 * m, x0[m], x1[m]);
-  RegDFT<16, -1>::run (x0);
-  RegDFT<16, -1>::run (x1);
-  // twiddle w64^(q ka); lane (j, q) then hands Y[q][ka] of both
-  // polarisations to lane 2 ka + pol through the warp's buffer (row 2 ka + pol,
-  // column 4 j + q, rows FBC_XROW float2 apart)
-#pragma unroll
-  for (int ka = 0; ka < 16; ka++)
-  {
-    const float2 w = s_tw64[(q * ka) & 63];
-    xb[(2 * ka) * FBC_XROW + lane] = cmul (x0[ka], w);
-    xb[(2 * ka + 1) * FBC_XROW + lane] = cmul (x1[ka], w);
-  }
-  __syncwarp ();
-  // lane 2 ka + pol reads its row in 16-byte pairs: z[jj][qq] = Y[qq][ka] of
-  // filterbank sample jj
-  float2 z[8][4];
-#pragma unroll
-  for (int jj = 0; jj < 8; jj++)
-#pragma unroll
-    for (int qq = 0; qq < 4; qq += 2)
-    {
-      const float4 t = *reinterpret_cast<const float4*> (xb + lane * FBC_XROW + 4 * jj + qq);
-      z[jj][qq] = make_float2 (t.x, t.y);
-      z[jj][qq + 1] = make_float2 (t.z, t.w);
-    }
-  // 4-point DFTs over q: z[jj][kb] = channel ka + 16 kb of filterbank sample jj
-#pragma unroll
-  for (int jj = 0; jj < 8; jj++) RegDFT<4, -1>::run (z[jj]);
-  // the column DFTs over the eight filterbank samples, per channel
-  float2 col[4][8];
-#pragma unroll
-  for (int kb = 0; kb < 4; kb++)
-  {
-#pragma unroll
-    for (int jj = 0; jj < 8; jj++) col[kb][jj] = z[jj][kb];
-    RegDFT<8, -1>::run (col[kb]);
-  }
-  // four-step twiddle w_N^(k1 n2) of column i2, and the filterbank
-  // normaliser 1/sqrt(64) (exact)
-  float2 tw[8];
-  tw[0] = make_float2 (1.f, 0.f);
-#pragma unroll
-  for (int k1 = 1; k1 < 8; k1++) tw[k1] = __ldg (tw4 + uint64_t (k1) * n2 + i2);
-  __syncthreads ();                    // every warp is done with its exchange buffer
-  // channel c = ka + 16 kb, pol of lane 2 ka + pol; staging row
-  // k1*128 + c*2 + pol, column = warp
-  {
-    const unsigned ka = lane >> 1, pol = lane & 1;
-#pragma unroll
-    for (int kb = 0; kb < 4; kb++)
-    {
-      const unsigned c = ka + 16 * kb;
-#pragma unroll
-      for (int k1 = 0; k1 < 8; k1++)
-      {
-        float2 o = k1 ? cmul (col[kb][k1], tw[k1]) : col[kb][k1];
-        o = make_float2 (__fmul_rn (o.x, 0.125f), __fmul_rn (o.y, 0.125f));
-        s_fbc[fbc_stage (k1 * 128 + c * 2 + pol, warp)] = o;
-      }
-    }
-  }
-  __syncthreads ();
-  // scratch row ((b*64 + c)*2 + pol)*N + k1*n2, columns i0 .. i0+FBC_COLS-1
-#pragma unroll 4
-  for (unsigned idx = threadIdx.x; idx < 1024 * FBC_COLS; idx += FBC_THREADS)
-  {
-    const unsigned row = idx / FBC_COLS, w = idx % FBC_COLS;
-    const unsigned k1 = row >> 7, c = (row & 127) >> 1, pol = row & 1;
-    scratch[((uint64_t (b) * 64 + c) * 2 + pol) * N + uint64_t (k1) * n2 + i0 + w] =
-        s_fbc[fbc_stage (row, w)];
-  }
 }
 
 // --------------------------------------------------------------------------
@@ -483,18 +285,24 @@ void launch_inv (const ConvShape& sh, dim3 grid, float2* scratch, uint64_t part0
   }
 }
 
-template <int N2>
+// 4096-point rows: k_rows64.  8192-point rows: k_rows32, or k_rows_mma when
+// the tensor-core arithmetic is asked for.
 void launch_rows (unsigned nrows, float2* scratch, const ConvTables& tb, unsigned n1,
                   const ConvShape& sh, cudaStream_t st)
 {
-  if (N2 == 8192 && tb.tc_splits)
+  if (sh.n2 == 4096)
+  {
+    launch_rows64 (nrows, scratch, tb.H, n1, sh.nchan, sh.npol, tb.nsm, tb.err, st);
+    return;
+  }
+  if (tb.tc_splits)
   {
     launch_rows_mma (nrows, scratch, tb, n1, sh, st);
     return;
   }
   // persistent: as many CTAs as are resident at once
-  const unsigned grid = std::min<unsigned> (nrows, rows_ctas_per_sm (N2) * unsigned (tb.nsm));
-  k_rows32<N2, true><<<grid, Row32<N2>::T, rows32_smem_bytes<N2> (), st>>> (
+  const unsigned grid = std::min<unsigned> (nrows, rows32_ctas_per_sm<8192> () * unsigned (tb.nsm));
+  k_rows32<8192, true><<<grid, Row32<8192>::T, rows32_smem_bytes<8192> (), st>>> (
       scratch, tb.H, n1, sh.nchan, sh.npol, nrows, nrows / (n1 * sh.nchan));
 }
 
@@ -509,21 +317,12 @@ cudaError_t run_fourstep_n1 (const ConvShape& sh, const ConvTables& tb, const In
   if (in.fb_nsub)
   {
     // the 64-channel filterbank inside the column pass
-    if (N1 != 8 || in.fb_nsub != 64 || sh.nchan != 64 || in.nchan != 1 || in.npol != 2
-        || sh.npol != 2 || tb.apod || (in.kind != IN_INT8 && in.kind != IN_INT16))
+    if ((N1 != 8 && N1 != 16) || in.fb_nsub != 64 || sh.nchan != 64 || in.nchan != 1
+        || in.npol != 2 || sh.npol != 2 || tb.apod || (in.kind != IN_INT8 && in.kind != IN_INT16))
       return cudaErrorInvalidValue;
     ClockScope cs (clk, KK_FWD_COLS, st);
-    const dim3 g (sh.n2 / FBC_COLS, nbatch);
-    if (in.kind == IN_INT8 && in.lut_scale != 0.f)
-      k_fwd_cols_fb64<IN_INT8, true><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep, part0,
-                                                                         sh.n2, tb.tw4, scratch);
-    else if (in.kind == IN_INT8)
-      k_fwd_cols_fb64<IN_INT8, false><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep, part0,
-                                                                          sh.n2, tb.tw4, scratch);
-    else
-      k_fwd_cols_fb64<IN_INT16, false><<<g, FBC_THREADS, FBC_SMEM, st>>> (in, tb.lut, sh.nkeep,
-                                                                           part0, sh.n2, tb.tw4,
-                                                                           scratch);
+    if constexpr (N1 == 8 || N1 == 16)
+      launch_fb64<N1> (in, tb.lut, sh.nkeep, part0, nbatch, sh.n2, tb.tw4, scratch, st);
   }
   else if (in.npol == 2 && fwd_pair_aligned (in))
   {
@@ -547,12 +346,8 @@ cudaError_t run_fourstep_n1 (const ConvShape& sh, const ConvTables& tb, const In
   const unsigned nrows = N1 * nbatch * sh.nchan * sh.npol;
   {
   ClockScope cs (clk, KK_ROWS, st);
-  if (sh.n2 == 8192)
-    launch_rows<8192> (nrows, scratch, tb, N1, sh, st);
-  else if (sh.n2 == 4096)
-    launch_rows<4096> (nrows, scratch, tb, N1, sh, st);
-  else
-    return cudaErrorInvalidValue;
+  if (sh.n2 != 8192 && sh.n2 != 4096) return cudaErrorInvalidValue;
+  launch_rows (nrows, scratch, tb, N1, sh, st);
   }
   ClockScope cs (clk, KK_INV_COLS, st);
   if (sh.npol == 2)
@@ -641,7 +436,7 @@ cudaError_t run_fused (const ConvShape& sh, const ConvTables& tb, const InputVie
 
 unsigned rows_ctas_per_sm (unsigned n2)
 {
-  return n2 == 8192 ? rows32_ctas_per_sm<8192> () : rows32_ctas_per_sm<4096> ();
+  return n2 == 8192 ? rows32_ctas_per_sm<8192> () : unsigned (R64_GROUPS);
 }
 
 // The four-step kernels' shared-memory opt-in, once per device (the current
@@ -655,20 +450,14 @@ cudaError_t convolution_kernel_setup ()
   const unsigned bit = dev < 32 ? 1u << dev : 0u;    // devices past 32: set every time
   if (bit && (attr_done.load () & bit)) return cudaSuccess;
   e = set_rows_smem<8192, true> ();
-  if (e == cudaSuccess) e = set_rows_smem<4096, true> ();
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute (k_rows64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int (R64_SMEM));
   // the single-kernel transforms of the float voltage path (the no-alloc
   // entry point's)
   if (e == cudaSuccess) e = fused_setup<4096, IN_FLOAT, OUT_VOLTAGE, 1> ();
   if (e == cudaSuccess) e = fused_setup<8192, IN_FLOAT, OUT_VOLTAGE, 1> ();
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT8, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT8, true>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_fwd_cols_fb64<IN_INT16, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (FBC_SMEM));
+  if (e == cudaSuccess) e = fb64_setup ();
   if (e == cudaSuccess) attr_done.fetch_or (bit);
   return e;
 }

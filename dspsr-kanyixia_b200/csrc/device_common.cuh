@@ -83,6 +83,16 @@ __device__ __forceinline__ void load_lut (const InputView& in, const float* lut,
       s_lut[i] = lut[i];
 }
 
+// read-only load kept in L1 ahead of other lines (reused by later rows)
+__device__ __forceinline__ float2 ldg_evict_last (const float2* p)
+{
+  float2 v;
+  asm volatile ("ld.global.nc.L1::evict_last.v2.f32 {%0, %1}, [%2];"
+                : "=f"(v.x), "=f"(v.y)
+                : "l"(p));
+  return v;
+}
+
 // --------------------------------------------------------------------------
 // detection (Detection.C:253-301 Intensity/PPQQ order, cross_detect.ic:38-41,
 // stokes_detect.ic:40-43); explicit _rn arithmetic so that no product is

@@ -256,7 +256,7 @@ template <int N2>
 void launch_rows_inv (unsigned nrows, float2* scratch, const IfbTables& tb, unsigned n1,
                       unsigned npol, cudaStream_t st)
 {
-  const unsigned grid = std::min<unsigned> (nrows, rows_ctas_per_sm (N2) * unsigned (tb.nsm));
+  const unsigned grid = std::min<unsigned> (nrows, rows32_ctas_per_sm<N2> () * unsigned (tb.nsm));
   k_rows32<N2, false><<<grid, Row32<N2>::T, rows32_smem_bytes<N2> (), st>>> (
       scratch, nullptr, n1, 1, npol, nrows, nrows / n1);
 }

@@ -118,8 +118,9 @@ struct KernelClock
 // Number of kernels this library has launched since it was loaded.
 uint64_t kernel_launches ();
 
-// CTAs of the FP32 convolution row kernel resident per SM for n2-point rows
-// (the persistent grid is this times the SM count)
+// Rows in flight per SM in the FP32 convolution row kernel for n2-point rows
+// (CTAs of k_rows32, row groups of k_rows64): batches are multiples of this
+// times the SM count
 unsigned rows_ctas_per_sm (unsigned n2);
 
 // SpectralKurtosis engine steps on their own: the test of sums already formed

@@ -29,16 +29,6 @@ __device__ __forceinline__ void tpass (const float2* src, float2* dst, float2* v
   }
 }
 
-// read-only load kept in L1 ahead of other lines (reused by later rows)
-__device__ __forceinline__ float2 ldg_evict_last (const float2* p)
-{
-  float2 v;
-  asm volatile ("ld.global.nc.L1::evict_last.v2.f32 {%0, %1}, [%2];"
-                : "=f"(v.x), "=f"(v.y)
-                : "l"(p));
-  return v;
-}
-
 // L2 prefetch of a global range (16-byte aligned, multiple of 16 bytes)
 __device__ __forceinline__ void prefetch_l2 (const void* p, unsigned bytes)
 {
