@@ -1299,7 +1299,7 @@ struct dspsr_b200_inverse_filterbank
   IfbShape shape {};
   unsigned in_discard_pos = 0, in_discard_neg = 0;
   DevBuf<int4> map;
-  DevBuf<float2> tw_lin, tw4, response, scratch;
+  DevBuf<float2> tw_lin, tw1024, tw4, response, scratch;
   DevBuf<float> temporal, spectral;
   DevBuf<int> err;
   bool have_response = false, have_temporal = false, have_spectral = false;
@@ -1312,6 +1312,7 @@ struct dspsr_b200_inverse_filterbank
     IfbTables t;
     t.map = map.ptr;
     t.ptab_lin = tw_lin.ptr;
+    t.tw1024 = tw1024.ptr;
     t.tw4 = tw4.ptr;
     t.response = have_response ? response.ptr : nullptr;
     t.temporal = have_temporal ? temporal.ptr : nullptr;
@@ -1325,6 +1326,7 @@ struct dspsr_b200_inverse_filterbank
   {
     map.release ();
     tw_lin.release ();
+    tw1024.release ();
     tw4.release ();
     response.release ();
     scratch.release ();
@@ -1491,6 +1493,10 @@ int dspsr_b200_inverse_filterbank::init (dspsr_b200_context* c, const dspsr_b200
   make_pass_tables (lin, t.data (), ntab_lin);
   B200_CHECK (ctx, tw_lin.reserve (t.size ()), "cudaMalloc twiddles");
   B200_CHECK (ctx, cudaMemcpy (tw_lin.ptr, t.data (), t.size () * sizeof (float2),
+                               cudaMemcpyHostToDevice), "copy twiddles");
+  t = make_tw2 (1024);
+  B200_CHECK (ctx, tw1024.reserve (1024), "cudaMalloc twiddles");
+  B200_CHECK (ctx, cudaMemcpy (tw1024.ptr, t.data (), 1024 * sizeof (float2),
                                cudaMemcpyHostToDevice), "copy twiddles");
   t = make_tw4 (n1, n2);
   B200_CHECK (ctx, tw4.reserve (lout), "cudaMalloc four-step twiddles");

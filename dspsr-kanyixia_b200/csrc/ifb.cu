@@ -1,5 +1,6 @@
 // ifb.cu -- inverse filterbank kernels (InverseFilterbankEngineCPU.C)
 
+#include "fb_warp.cuh"
 #include "group_fft.cuh"
 #include "rows32.cuh"
 
@@ -10,6 +11,80 @@ namespace {
 // --------------------------------------------------------------------------
 // inverse filterbank (InverseFilterbankEngineCPU.C:309-779 restructured)
 // --------------------------------------------------------------------------
+
+// The kept bins of one (channel, pol) spectrum (s, padded layout) to the
+// output channels' spectra, by the TF threads of the transform (tid).
+template <int LIN, int TF>
+__device__ __forceinline__ void stitch_out (const float2* s, const IfbShape& sh,
+                                            const IfbTables& tb, float2* __restrict__ scratch,
+                                            unsigned b, unsigned c, unsigned p, unsigned tid)
+{
+  const int4 m = __ldg (tb.map + c);
+  const unsigned keep2 = sh.keep / 2;
+  const unsigned skip2 = (LIN - sh.keep) / 2;
+  const unsigned src_neg = sh.dual_sideband ? LIN - keep2 : skip2;
+  const unsigned src_pos = sh.dual_sideband ? 0 : skip2 + keep2;
+  if (keep2 % sh.n1 == 0)
+  {
+    // n1 divides keep/2, so every half starts on a multiple of n1 and its
+    // bins fill per_row consecutive columns of each four-step row: threads
+    // walk them row by row, consecutive threads writing consecutive columns.
+    const unsigned per_row = keep2 / sh.n1;
+    const bool pow2 = (per_row & (per_row - 1)) == 0;
+    const unsigned lg = __ffs (per_row) - 1;
+    for (int h = 0; h < 2; h++)
+    {
+      const int o = h ? m.z : m.x;
+      const int offz = h ? m.w : m.y;
+      const unsigned off = unsigned (offz & (IFB_ZERO - 1));
+      const unsigned src0 = h ? src_pos : src_neg;
+      float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout + off / sh.n1;
+      for (unsigned r = tid; r < keep2; r += TF)
+      {
+        const unsigned a = pow2 ? r >> lg : r / per_row;
+        const unsigned q = r - a * per_row;
+        const unsigned j = q * sh.n1 + a;
+        float2 y = (offz & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad (src0 + j)];
+        if (tb.response)
+        {
+          const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + off + j);
+          y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
+                           __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
+        }
+        if (tb.spectral)
+        {
+          const float w = __ldg (tb.spectral + off + j);
+          y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
+        }
+        dst[uint64_t (a) * sh.n2 + q] = y;
+      }
+    }
+    return;
+  }
+  for (unsigned i = tid; i < sh.keep; i += TF)
+  {
+    const bool neg = i < keep2;
+    const unsigned j = neg ? i : i - keep2;
+    const int o = neg ? m.x : m.z;
+    const int off = neg ? m.y : m.w;
+    const unsigned k = unsigned (off & (IFB_ZERO - 1)) + j;
+    float2 y = (off & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad ((neg ? src_neg : src_pos) + j)];
+    if (tb.response)
+    {
+      // Response::operate: (f_r d_r - f_i d_i, f_i d_r + f_r d_i)
+      const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + k);
+      y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
+                       __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
+    }
+    if (tb.spectral)
+    {
+      const float w = __ldg (tb.spectral + k);
+      y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
+    }
+    float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout;
+    dst[uint64_t (k % sh.n1) * sh.n2 + k / sh.n1] = y;
+  }
+}
 
 // A CTA of IFB_THREADS threads transforms F = 8192/LIN (channel, pol) slots of
 // one part: CG = F/npol consecutive fine channels, both pols.  The input tile
@@ -118,72 +193,133 @@ k_ifb_stitch (const InputView in, const IfbShape sh, const IfbTables tb, const u
     group_fft_pass<LIN, TF, -1, 0> (s, v, s_tab, tid);
   }
   const unsigned c = c0 + group / npol, p = group % npol;
-  if (c >= sh.nin) return;
-  const int4 m = __ldg (tb.map + c);
-  const unsigned keep2 = sh.keep / 2;
-  const unsigned skip2 = (LIN - sh.keep) / 2;
-  const unsigned src_neg = sh.dual_sideband ? LIN - keep2 : skip2;
-  const unsigned src_pos = sh.dual_sideband ? 0 : skip2 + keep2;
-  if (keep2 % sh.n1 == 0)
+  if (c < sh.nin) stitch_out<LIN, TF> (s, sh, tb, scratch, b, c, p, tid);
+}
+
+// The same for LIN = 128 .. 1024 with 32 points per thread (FbWarp's split
+// LIN = 32 x M: one exchange, warp barriers only).  A block takes
+// 8 * (32 / M) slots; TFPD samples are loaded in address order (all slots of a
+// time sample together) and handed over as raw words in the slots' own
+// regions, whose stride of 4 mod 32 words keeps both sides free of bank
+// conflicts; FPT samples are loaded by the slot's own lanes.  16 points per
+// thread in three block-wide passes moved 80 bytes per point through shared
+// memory, this 48: 790 us before, 760 us now with 256 channels of
+// 1024 points.
+template <int LIN, int KIND>
+__global__ void __launch_bounds__ (FBW_WARPS * 32, 2)
+k_ifb_stitch_warp (const InputView in, const IfbShape sh, const IfbTables tb, const uint64_t part0,
+                   float2* __restrict__ scratch)
+{
+  using FW = FbWarp<LIN>;
+  constexpr int M = FW::M;
+  constexpr int T = FBW_WARPS * 32;
+  constexpr unsigned F = FW::NB;                   // slots per block
+  static_assert (spad_size (LIN) <= FW::RS, "the spectrum fits its region");
+  extern __shared__ __align__ (16) float2 s_ifw[];
+  float2* tw = s_ifw + F * FW::RS;                 // w_LIN^(q t) at [q * M + t]
+  __shared__ float s_lut[KIND == IN_INT8 ? 256 : 1];
+  const unsigned npol = sh.npol;
+  const unsigned c0 = blockIdx.x * (F / npol);
+  const unsigned b = blockIdx.y;
+  if constexpr (KIND == IN_INT8) load_lut (in, tb.lut, s_lut);
+  for (int i = threadIdx.x; i < LIN; i += T)
   {
-    // n1 divides keep/2, so every half starts on a multiple of n1 and its
-    // bins fill per_row consecutive columns of each four-step row: threads
-    // walk them row by row, consecutive threads writing consecutive columns.
-    const unsigned per_row = keep2 / sh.n1;
-    const bool pow2 = (per_row & (per_row - 1)) == 0;
-    const unsigned lg = __ffs (per_row) - 1;
-    for (int h = 0; h < 2; h++)
+    // w_LIN^m is w_1024^(m 1024 / LIN)
+    const int m = (i / M) * (i % M) % LIN;
+    tw[i] = __ldg (tb.tw1024 + m * (1024 / LIN));
+  }
+  const uint64_t t0 = (part0 + b) * sh.in_step;
+  const unsigned nslot = min (F, (sh.nin - c0) * npol);                // live slots
+  const int t = threadIdx.x % M;
+  const unsigned slot = threadIdx.x / M;
+  float2* s = s_ifw + slot * FW::RS;
+  CP v[32];
+  if constexpr (KIND == IN_FLOAT)
+  {
+#pragma unroll
+    for (int r = 0; r < 32; r++)
+      v[r].z = slot < nslot ? __ldg (static_cast<const float2*> (in.main)
+                                     + (uint64_t (c0) * npol + slot) * in.main_span + t0 + t + M * r)
+                            : make_float2 (0.f, 0.f);
+    __syncthreads ();                  // the twiddles are there
+  }
+  else
+  {
+    const uint64_t row = uint64_t (sh.nin) * npol;                     // TFPD values per sample
+    uint32_t word[32];
+#pragma unroll
+    for (int k = 0; k < 32; k++)
     {
-      const int o = h ? m.z : m.x;
-      const int offz = h ? m.w : m.y;
-      const unsigned off = unsigned (offz & (IFB_ZERO - 1));
-      const unsigned src0 = h ? src_pos : src_neg;
-      float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout + off / sh.n1;
-      for (unsigned r = tid; r < keep2; r += TF)
+      const unsigned e = threadIdx.x + k * T, sl = e % F, tt = e / F;
+      const uint64_t idx = (t0 + tt) * row + uint64_t (c0) * npol + sl;
+      if constexpr (KIND == IN_INT16)
+        word[k] = sl < nslot ? __ldg (static_cast<const uint32_t*> (in.main) + idx) : 0u;
+      else
+        word[k] = sl < nslot ? __ldg (static_cast<const unsigned short*> (in.main) + idx) : 0u;
+    }
+    uint32_t* raw = reinterpret_cast<uint32_t*> (s_ifw);
+#pragma unroll
+    for (int k = 0; k < 32; k++)
+    {
+      const unsigned e = threadIdx.x + k * T;
+      raw[(e % F) * (2 * FW::RS) + e / F] = word[k];
+    }
+    __syncthreads ();
+#pragma unroll
+    for (int r = 0; r < 32; r++)
+    {
+      const uint32_t w = raw[slot * (2 * FW::RS) + t + M * r];
+      float2 x;
+      if constexpr (KIND == IN_INT16)
       {
-        const unsigned a = pow2 ? r >> lg : r / per_row;
-        const unsigned q = r - a * per_row;
-        const unsigned j = q * sh.n1 + a;
-        float2 y = (offz & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad (src0 + j)];
-        if (tb.response)
+        short re = short (w & 0xffff), im = short (w >> 16);
+        if (in.offset_binary)
         {
-          const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + off + j);
-          y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
-                           __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
+          re = short (re ^ 0x8000);
+          im = short (im ^ 0x8000);
         }
-        if (tb.spectral)
-        {
-          const float w = __ldg (tb.spectral + off + j);
-          y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
-        }
-        dst[uint64_t (a) * sh.n2 + q] = y;
+        // SixteenBitUnpacker.C:69: float(x) + 0.5
+        x = make_float2 (__fadd_rn (float (re), 0.5f), __fadd_rn (float (im), 0.5f));
       }
+      else
+        x = make_float2 (s_lut[w & 0xff], s_lut[w >> 8]);
+      v[r].z = slot < nslot ? x : make_float2 (0.f, 0.f);
     }
-    return;
   }
-  for (unsigned i = tid; i < sh.keep; i += TF)
+  if (tb.temporal)
   {
-    const bool neg = i < keep2;
-    const unsigned j = neg ? i : i - keep2;
-    const int o = neg ? m.x : m.z;
-    const int off = neg ? m.y : m.w;
-    const unsigned k = unsigned (off & (IFB_ZERO - 1)) + j;
-    float2 y = (off & IFB_ZERO) ? make_float2 (0.f, 0.f) : s[spad ((neg ? src_neg : src_pos) + j)];
-    if (tb.response)
+#pragma unroll
+    for (int r = 0; r < 32; r++)
     {
-      // Response::operate: (f_r d_r - f_i d_i, f_i d_r + f_r d_i)
-      const float2 f = __ldg (tb.response + uint64_t (o) * sh.lout + k);
-      y = make_float2 (__fsub_rn (__fmul_rn (f.x, y.x), __fmul_rn (f.y, y.y)),
-                       __fadd_rn (__fmul_rn (f.y, y.x), __fmul_rn (f.x, y.y)));
+      const float w = __ldg (tb.temporal + t + M * r);
+      v[r].z = make_float2 (__fmul_rn (v[r].z.x, w), __fmul_rn (v[r].z.y, w));
     }
-    if (tb.spectral)
-    {
-      const float w = __ldg (tb.spectral + k);
-      y = make_float2 (__fmul_rn (y.x, w), __fmul_rn (y.y, w));
-    }
-    float2* dst = scratch + ((uint64_t (b) * sh.nout + o) * sh.npol + p) * sh.lout;
-    dst[uint64_t (k % sh.n1) * sh.n2 + k / sh.n1] = y;
   }
+  dft::run<32, -1> (v);
+  __syncwarp ();                       // the raw words of the warp's slots have been read
+#pragma unroll
+  for (int q = 0; q < 32; q++) s[q * FW::LD + t] = q ? cmul (v[q].z, tw[q * M + t]) : v[q].z;
+  __syncwarp ();
+#pragma unroll
+  for (int i = 0; i < FW::G; i++)
+#pragma unroll
+    for (int j = 0; j < M / 2; j++)
+    {
+      const float4 x = *reinterpret_cast<const float4*> (s + (t + M * i) * FW::LD + 2 * j);
+      v[i * M + 2 * j].z = make_float2 (x.x, x.y);
+      v[i * M + 2 * j + 1].z = make_float2 (x.z, x.w);
+    }
+  __syncwarp ();
+#pragma unroll
+  for (int i = 0; i < FW::G; i++)
+  {
+    dft::run<M, -1> (v + i * M);
+#pragma unroll
+    for (int p = 0; p < M; p++) s[spad (t + M * i + 32 * p)] = v[i * M + p].z;
+  }
+  __syncwarp ();
+  if (slot < nslot)
+    stitch_out<LIN, M> (s, sh, tb, scratch, b, c0 + slot / npol, slot % npol, t);
 }
 
 // Inverse column DFTs of the lout-point transforms (after the row kernel):
@@ -230,6 +366,31 @@ void launch_ifb_stitch (const IfbShape& sh, const IfbTables& tb, const InputView
   const unsigned cg = F / sh.npol;
   kern<<<dim3 ((sh.nin + cg - 1) / cg, nbatch), IFB_THREADS, smem, st>>> (in, sh, tb, part0,
                                                                          scratch);
+}
+
+template <int LIN, int KIND>
+void launch_ifb_stitch_warp (const IfbShape& sh, const IfbTables& tb, const InputView& in,
+                             uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
+{
+  using FW = FbWarp<LIN>;
+  auto kern = k_ifb_stitch_warp<LIN, KIND>;
+  cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int (FW::SMEM));
+  const unsigned cg = FW::NB / sh.npol;
+  kern<<<dim3 ((sh.nin + cg - 1) / cg, nbatch), FBW_WARPS * 32, FW::SMEM, st>>> (in, sh, tb, part0,
+                                                                                scratch);
+}
+
+// 128- to 1024-point transforms fit a warp with 32 points per thread
+template <int LIN>
+void launch_ifb_stitch_w (const IfbShape& sh, const IfbTables& tb, const InputView& in,
+                          uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
+{
+  if (in.kind == IN_INT8)
+    launch_ifb_stitch_warp<LIN, IN_INT8> (sh, tb, in, part0, nbatch, scratch, st);
+  else if (in.kind == IN_INT16)
+    launch_ifb_stitch_warp<LIN, IN_INT16> (sh, tb, in, part0, nbatch, scratch, st);
+  else
+    launch_ifb_stitch_warp<LIN, IN_FLOAT> (sh, tb, in, part0, nbatch, scratch, st);
 }
 
 template <int LIN>
@@ -291,10 +452,10 @@ cudaError_t launch_inverse_filterbank (const IfbShape& sh, const IfbTables& tb,
     switch (sh.lin)
     {
       case 64: launch_ifb_stitch_k<64> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 128: launch_ifb_stitch_k<128> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 256: launch_ifb_stitch_k<256> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 512: launch_ifb_stitch_k<512> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 1024: launch_ifb_stitch_k<1024> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 128: launch_ifb_stitch_w<128> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 256: launch_ifb_stitch_w<256> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 512: launch_ifb_stitch_w<512> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 1024: launch_ifb_stitch_w<1024> (sh, tb, in, part0, nbatch, scratch, st); break;
       case 2048: launch_ifb_stitch_k<2048> (sh, tb, in, part0, nbatch, scratch, st); break;
       case 4096: launch_ifb_stitch_k<4096> (sh, tb, in, part0, nbatch, scratch, st); break;
       default: return cudaErrorInvalidValue;

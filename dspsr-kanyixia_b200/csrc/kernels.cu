@@ -2,6 +2,7 @@
 // SpectralKurtosis, unpackers, detection, fold (sm_100a)
 
 #include "device_common.cuh"
+#include "fb_warp.cuh"
 #include "group_fft.cuh"
 
 namespace b200 {
@@ -110,7 +111,7 @@ k_filterbank (const InputView in, const float* __restrict__ lut, const uint64_t 
                                                          __fmul_rn (scale, v[k].y));
 }
 
-// The same filterbank for NSUB = 128 .. 4096 with the transforms in shared
+// The same filterbank for NSUB = 2048 and 4096 with the transforms in shared
 // memory: a CTA of FB_THREADS threads takes F = 8192/NSUB (block, pol) slots of
 // one input channel, reads their samples in address order (coalesced), runs
 // one NSUB-point FFT per group of NSUB/16 threads (per-pass twiddle tables in
@@ -937,6 +938,55 @@ cudaError_t run_filterbank (const InputView& in, const float* d_lut, uint64_t nb
     k_filterbank<NSUB, IN_FLOAT><<<grid, 128, 0, st>>> (in, d_lut, nblk, scale, out, out_span);
   return cudaGetLastError ();
 }
+// multiprocessors of the current device, asked for once per device
+cudaError_t sm_count (int* n)
+{
+  static std::atomic<int> known[32] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice (&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 32 && known[dev].load ())
+  {
+    *n = known[dev].load ();
+    return cudaSuccess;
+  }
+  e = cudaDeviceGetAttribute (n, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess && dev < 32) known[dev].store (*n);
+  return e;
+}
+
+template <int NSUB, int KIND>
+cudaError_t run_filterbank_warp_t (const InputView& in, const float* d_lut, uint64_t nblk,
+                                   float scale, float2* out, uint64_t out_span, cudaStream_t st)
+{
+  using F = FbWarp<NSUB>;
+  int nsm = 0;
+  cudaError_t e = sm_count (&nsm);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute (k_filterbank_warp<NSUB, KIND>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (F::SMEM));
+  if (e != cudaSuccess) return e;
+  const uint64_t per_row = (nblk + F::NB - 1) / F::NB;
+  const uint64_t ntile = per_row * in.nchan * in.npol;
+  const unsigned grid = unsigned (std::min<uint64_t> (ntile, 2 * uint64_t (nsm)));
+  k_filterbank_warp<NSUB, KIND><<<grid, FBW_WARPS * 32, F::SMEM, st>>> (
+      in, d_lut, nblk, scale, out, out_span, per_row, ntile);
+  return cudaGetLastError ();
+}
+
+template <int NSUB>
+cudaError_t run_filterbank_warp (const InputView& in, const float* d_lut, uint64_t nblk, float scale,
+                                 float2* out, uint64_t out_span, cudaStream_t st,
+                                 const KernelClock* clk)
+{
+  ClockScope cs (clk, KK_FILTERBANK, st);
+  if (in.kind == IN_INT8)
+    return run_filterbank_warp_t<NSUB, IN_INT8> (in, d_lut, nblk, scale, out, out_span, st);
+  if (in.kind == IN_INT16)
+    return run_filterbank_warp_t<NSUB, IN_INT16> (in, d_lut, nblk, scale, out, out_span, st);
+  return run_filterbank_warp_t<NSUB, IN_FLOAT> (in, d_lut, nblk, scale, out, out_span, st);
+}
+
 template <int NSUB>
 cudaError_t run_filterbank_smem (const InputView& in, const float* d_lut, const float2* ptab,
                                  uint64_t nblk, float scale, float2* out, uint64_t out_span,
@@ -983,16 +1033,17 @@ cudaError_t launch_filterbank (const InputView& in, const float* d_lut, unsigned
                                cudaStream_t st, const KernelClock* clk, const float2* ptab)
 {
   if (nblk == 0) return cudaSuccess;
-  // up to 64 channels the one-thread-per-block register transform is faster
+  // up to 64 channels the one-thread-per-block register transform is faster;
+  // 128 to 1024 fit a warp with 32 points per thread, more need the block
   if (nsub >= 128)
   {
     if (!ptab) return cudaErrorInvalidValue;
     switch (nsub)
     {
-      case 128: return run_filterbank_smem<128> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
-      case 256: return run_filterbank_smem<256> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
-      case 512: return run_filterbank_smem<512> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
-      case 1024: return run_filterbank_smem<1024> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
+      case 128: return run_filterbank_warp<128> (in, d_lut, nblk, scale, out, out_span, st, clk);
+      case 256: return run_filterbank_warp<256> (in, d_lut, nblk, scale, out, out_span, st, clk);
+      case 512: return run_filterbank_warp<512> (in, d_lut, nblk, scale, out, out_span, st, clk);
+      case 1024: return run_filterbank_warp<1024> (in, d_lut, nblk, scale, out, out_span, st, clk);
       case 2048: return run_filterbank_smem<2048> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
       case 4096: return run_filterbank_smem<4096> (in, d_lut, ptab, nblk, scale, out, out_span, st, clk);
       default: return cudaErrorInvalidValue;

@@ -221,6 +221,7 @@ struct IfbTables
   // bin marks a half that is zeroed instead
   const int4* map;
   const float2* ptab_lin;    // per-pass Stockham tables of the lin-point transform
+  const float2* tw1024;      // w_1024^m, m < 1024
   const float2* tw4;         // [n1][n2] four-step table of the lout-point transform
   const float2* response;    // [nout][lout] or null
   const float* temporal;     // [lin] or null
