@@ -1658,7 +1658,7 @@ struct dspsr_b200_filterbank_during
 {
   dspsr_b200_context* ctx = nullptr;
   DuringShape shape {};
-  DevBuf<float2> tw4, ptab_seg, ptab_col, twd, H, Hw, tmp, scratch;
+  DevBuf<float2> tw4, ptab_seg, ptab_col, tw1024, twd, H, Hw, tmp, scratch;
   DevBuf<double> chan_par;
   DevBuf<float> temporal, spectral;
   bool have_response = false, have_temporal = false, have_spectral = false;
@@ -1672,6 +1672,7 @@ struct dspsr_b200_filterbank_during
     t.ptab_seg = ptab_seg.ptr;
     t.twd = twd.ptr;
     t.ptab_col = ptab_col.ptr;
+    t.tw1024 = tw1024.ptr;
     t.H = have_spectral ? Hw.ptr : H.ptr;
     t.lut = ctx->d_lut;
     t.nsm = nsm;
@@ -1690,6 +1691,7 @@ struct dspsr_b200_filterbank_during
     tw4.release ();
     ptab_seg.release ();
     ptab_col.release ();
+    tw1024.release ();
     twd.release ();
     H.release ();
     Hw.release ();
@@ -1750,6 +1752,13 @@ int dspsr_b200_filterbank_during::init (dspsr_b200_context* c, const dspsr_b200_
     B200_CHECK (ctx, dst.reserve (pt.size ()), "cudaMalloc pass tables");
     B200_CHECK (ctx, cudaMemcpy (dst.ptr, pt.data (), pt.size () * sizeof (float2),
                                  cudaMemcpyHostToDevice), "copy pass tables");
+  }
+  if (s.n1 >= 64)
+  {
+    const std::vector<float2> t = make_tw2 (1024);
+    B200_CHECK (ctx, tw1024.reserve (1024), "cudaMalloc twiddles");
+    B200_CHECK (ctx, cudaMemcpy (tw1024.ptr, t.data (), 1024 * sizeof (float2),
+                                 cudaMemcpyHostToDevice), "copy twiddles");
   }
   int dev = 0;
   B200_CHECK (ctx, cudaGetDevice (&dev), "cudaGetDevice");

@@ -1,5 +1,6 @@
 // during.cu -- the filterbank with a response (FilterbankEngineCPU.C:379-535)
 
+#include "big_cols.cuh"
 #include "fwd_cols.cuh"
 #include "fwd_cols_pair.cuh"
 #include "inv_cols_split.cuh"
@@ -549,26 +550,32 @@ cudaError_t run_during_n1 (const DuringShape& sh, const DuringTables& tb, const 
   return cudaGetLastError ();
 }
 
-template <int N1, int NPOL>
-void launch_inv_during_big (const DuringShape& sh, dim3 grid, const float2* scratch,
-                            uint64_t part0, const DuringTables& tb, int mode, const FoldView& fv,
-                            const VoltView& vv, cudaStream_t st)
+// two polarisations: k_inv_cols_big_pair; one: k_inv_cols_during_big
+template <int N1>
+cudaError_t launch_inv_during_big (const DuringShape& sh, dim3 grid, const float2* scratch,
+                                   uint64_t part0, const DuringTables& tb, int mode,
+                                   const FoldView& fv, const VoltView& vv, cudaStream_t st)
 {
-  constexpr size_t smem = colbig_inv_smem<N1, NPOL> ();
+  if (sh.npol == 2)
+  {
+    if (mode == OUT_VOLTAGE)
+      return launch_inv_big_pair<N1, OUT_VOLTAGE, 1> (sh, tb, part0, grid.y, scratch, fv, vv, st);
+    if (fv.nout == 1)
+      return launch_inv_big_pair<N1, OUT_FOLD, 1> (sh, tb, part0, grid.y, scratch, fv, vv, st);
+    if (fv.nout == 2)
+      return launch_inv_big_pair<N1, OUT_FOLD, 2> (sh, tb, part0, grid.y, scratch, fv, vv, st);
+    return launch_inv_big_pair<N1, OUT_FOLD, 4> (sh, tb, part0, grid.y, scratch, fv, vv, st);
+  }
+  constexpr size_t smem = colbig_inv_smem<N1, 1> ();
   constexpr int T = inv_colw<N1> () * stockham_threads (N1);
   grid.x = sh.n2 / inv_colw<N1> ();
-  if (mode == OUT_VOLTAGE)
-  {
-    auto k = k_inv_cols_during_big<N1, NPOL, OUT_VOLTAGE, 1>;
-    cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
-    k<<<grid, T, smem, st>>> (scratch, sh, part0, tb.twd, tb.ptab_col, fv, vv);
-    return;
-  }
-  auto k = NPOL == 1 || fv.nout == 1 ? k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 1>
-         : fv.nout == 2 ? k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 2>
-                        : k_inv_cols_during_big<N1, NPOL, OUT_FOLD, 4>;
-  cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
+  auto k = mode == OUT_VOLTAGE ? k_inv_cols_during_big<N1, 1, OUT_VOLTAGE, 1>
+                               : k_inv_cols_during_big<N1, 1, OUT_FOLD, 1>;
+  const cudaError_t e = cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int (smem));
+  if (e != cudaSuccess) return e;
   k<<<grid, T, smem, st>>> (scratch, sh, part0, tb.twd, tb.ptab_col, fv, vv);
+  return cudaGetLastError ();
 }
 
 template <int N1>
@@ -577,12 +584,17 @@ cudaError_t run_during_big (const DuringShape& sh, const DuringTables& tb, const
                             const FoldView& fv, const VoltView& vv, cudaStream_t st,
                             const KernelClock* clk)
 {
-  static_assert (colbig_inv_smem<N1, 2> () <= 227u * 1024u, "column kernel shared memory");
+  static_assert (colbig_inv_smem<N1, 1> () <= 227u * 1024u, "column kernel shared memory");
   const dim3 gcol (sh.n2 / COLW, nbatch, sh.nchan_in);
   {
     ClockScope cs (clk, KK_FWD_COLS, st);
     constexpr size_t smem = colbig_smem<N1, 1> ();
-    if (in.kind == IN_INT8)
+    if (in.npol == 2 && fwd_pair_aligned (in))
+    {
+      const cudaError_t e = launch_fwd_big_pair<N1> (sh, tb, in, part0, nbatch, scratch, st);
+      if (e != cudaSuccess) return e;
+    }
+    else if (in.kind == IN_INT8)
     {
       cudaFuncSetAttribute (k_fwd_cols_big<N1, IN_INT8>,
                             cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
@@ -622,11 +634,7 @@ cudaError_t run_during_big (const DuringShape& sh, const DuringTables& tb, const
   }
   if (e != cudaSuccess) return e;
   ClockScope cs (clk, KK_INV_COLS, st);
-  if (sh.npol == 2)
-    launch_inv_during_big<N1, 2> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  else
-    launch_inv_during_big<N1, 1> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
-  return cudaGetLastError ();
+  return launch_inv_during_big<N1> (sh, gcol, scratch, part0, tb, mode, fv, vv, st);
 }
 
 } // namespace

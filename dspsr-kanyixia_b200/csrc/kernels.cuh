@@ -264,6 +264,7 @@ struct DuringTables
   const float2* ptab_seg;  // per-pass tables of the seg-point FFT
   const float2* twd;       // [n1][seg] exp(-2 pi i k1 t2 / freq_res)
   const float2* ptab_col;  // per-pass tables of the n1-point FFT (n1 >= 64)
+  const float2* tw1024;    // w_1024^m, m < 1024 (n1 >= 64)
   const float2* H;         // [nchan_in*nsub][n1][seg]: bin k1 + n1*f2 of each channel
   const float* lut;        // 8-bit table for int8 input
   int nsm;
