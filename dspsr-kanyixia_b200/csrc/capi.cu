@@ -129,10 +129,12 @@ std::vector<float2> make_tw4 (unsigned n1, unsigned n2)
 namespace {
 
 // The four-step row length when the caller names none: 4096-point rows
-// (k_rows64) for transforms of 16384 to 65536 points, whose 4- to 16-point
-// columns fit one thread for both polarisations; 8192-point rows above, and
-// the single-kernel transforms below.
-unsigned default_row_length (unsigned nfft) { return nfft >= 16384 && nfft <= 65536 ? 4096 : 8192; }
+// (k_rows64) where they leave columns of at most 32 points, whose passes run a
+// thread or two per column; 8192-point rows above, and the single-kernel
+// transforms below.  Blocks with either: 2^14 x 32 channels 0.357 against
+// 0.420 ms, 2^15 x 1024 (C5) 4.83 against 5.22, 2^16 x 64 (C2) 3.07 against
+// 3.27, 2^17 (C1) 0.620 against 0.655.
+unsigned default_row_length (unsigned nfft) { return nfft >= 16384 && nfft <= 131072 ? 4096 : 8192; }
 
 } // namespace
 

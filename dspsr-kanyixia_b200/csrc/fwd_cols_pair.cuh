@@ -75,6 +75,8 @@ __device__ __forceinline__ typename RawPair<KIND>::T load_pair (const void* base
 // buffer (words): a warp stores 4 columns x 8 channels and loads 32 columns
 // of one channel, both in distinct banks
 constexpr int FWP_CH = 8, FWP_LD = 36;
+// the same for tiles of 16 columns (a half-warp loads one channel's)
+constexpr int FWP32_LD = 20;
 
 template <int N1, int KIND, bool TILE>
 constexpr size_t fwp_smem ()
@@ -194,46 +196,77 @@ k_fwd_cols_pair (const InputView in, const float* __restrict__ lut, const uint64
   }
 }
 
+// Threads per block of the n1 = 32 pass: 64 columns of one channel, or with
+// TILE 16 columns of 8 channels, two threads per column.
+template <bool TILE> B200_CE int fwp32_threads () { return TILE ? 256 : 128; }
+template <int KIND, bool TILE>
+constexpr size_t fwp32_smem ()
+{
+  return size_t (16) * fwp32_threads<TILE> () * sizeof (float4)
+         + (TILE ? 32 * FWP_CH * FWP32_LD * sizeof (typename RawPair<KIND>::T) : 0);
+}
+
 // The same for n1 = 32: two threads per column, thread h with rows 2m + h (16
 // points of both polarisations in registers; 32 spill).  They exchange
 // through shared memory -- E, and w32^j O already turned -- and each forms
 // X[j] = E[j] + w32^j O[j] and X[j + 16] = E[j] - w32^j O[j] for half the j.
-// 64 columns per block.
-template <int KIND, bool AFFINE>
-__global__ void __launch_bounds__ (128, 4)
+template <int KIND, bool AFFINE, bool TILE>
+__global__ void __launch_bounds__ (fwp32_threads<TILE> (), TILE ? 2 : 4)
 k_fwd_cols_pair32 (const InputView in, const float* __restrict__ lut, const uint64_t nkeep,
                    const uint64_t part0, const unsigned nbatch, const unsigned n2,
                    const float2* __restrict__ tw4, float2* __restrict__ scratch,
                    const float* __restrict__ apod)
 {
   using Raw = typename RawPair<KIND>::T;
+  constexpr int T = fwp32_threads<TILE> (), P = T / 2;     // (column, channel) pairs of the block
+  constexpr int COLS = TILE ? 16 : 64;
   __shared__ float s_lut[KIND == IN_INT8 && !AFFINE ? 256 : 1];
-  __shared__ float4 s_x[2 * 16 * 64];              // [half][j][column]
+  extern __shared__ __align__ (16) unsigned char s_fwp[];
+  float4* s_x = reinterpret_cast<float4*> (s_fwp);         // [half][j][pair]
+  Raw* tile = reinterpret_cast<Raw*> (s_fwp + size_t (16) * T * sizeof (float4));
   if (KIND == IN_INT8 && !AFFINE)
   {
     load_lut (in, lut, s_lut);
     __syncthreads ();
   }
   const UnpackPair u {s_lut, in.lut_scale, in.offset_binary ? 0u : 0x80008000u};
-  const unsigned c = blockIdx.z;
-  const unsigned col = threadIdx.x % 64, h = threadIdx.x / 64;
-  const unsigned i2 = blockIdx.x * 64 + col;
+  const unsigned pr = threadIdx.x % P, h = threadIdx.x / P;
+  const unsigned c0 = TILE ? blockIdx.z * FWP_CH : blockIdx.z, c = c0 + pr / COLS;
+  const unsigned i0 = blockIdx.x * COLS, i2 = i0 + pr % COLS;
   const uint64_t N = 32ull * n2;
   const uint64_t step = KIND == IN_FLOAT ? 1 : in.nchan;
   for (unsigned b = blockIdx.y; b < nbatch; b += gridDim.y)
   {
-    const uint64_t ta = (part0 + b) * nkeep + i2;
+    const uint64_t ta = (part0 + b) * nkeep + i0;
+    const auto at = [&] (uint64_t t, unsigned ch) -> Raw {
+      t += ta;
+      const bool pre = t < in.npre;
+      const uint64_t sp = pre ? in.pre_span : in.main_span, tt = pre ? t : t - in.npre;
+      return load_pair<KIND> (pre ? in.pre : in.main,
+                              KIND == IN_FLOAT ? uint64_t (ch) * 2 * sp + tt : tt * step + ch, sp);
+    };
     C2 v[16];
     {
       Raw raw[16];
-#pragma unroll
-      for (int m = 0; m < 16; m++)
+      if constexpr (TILE)
       {
-        const uint64_t t = ta + uint64_t (2 * m + h) * n2;
-        const bool pre = t < in.npre;
-        const uint64_t sp = pre ? in.pre_span : in.main_span, tt = pre ? t : t - in.npre;
-        raw[m] = load_pair<KIND> (pre ? in.pre : in.main,
-                                  KIND == IN_FLOAT ? uint64_t (c) * 2 * sp + tt : tt * step + c, sp);
+        // 16 columns x 8 channels of every row, in address order
+        const unsigned ch = threadIdx.x % FWP_CH, col = threadIdx.x / FWP_CH % COLS;
+        const unsigned odd = threadIdx.x / (FWP_CH * COLS);
+#pragma unroll
+        for (int m = 0; m < 16; m++) raw[m] = at (uint64_t (2 * m + odd) * n2 + col, c0 + ch);
+#pragma unroll
+        for (int m = 0; m < 16; m++)
+          tile[((2 * m + odd) * FWP_CH + ch) * FWP32_LD + col] = raw[m];
+        __syncthreads ();
+#pragma unroll
+        for (int m = 0; m < 16; m++)
+          raw[m] = tile[((2 * m + h) * FWP_CH + pr / COLS) * FWP32_LD + pr % COLS];
+      }
+      else
+      {
+#pragma unroll
+        for (int m = 0; m < 16; m++) raw[m] = at (uint64_t (2 * m + h) * n2 + pr, c);
       }
 #pragma unroll
       for (int m = 0; m < 16; m++) v[m] = unpack_pair<KIND, AFFINE> (raw[m], u);
@@ -258,14 +291,14 @@ k_fwd_cols_pair32 (const InputView in, const float* __restrict__ lut, const uint
     __syncthreads ();                  // the last part's reads are done
 #pragma unroll
     for (int j = 0; j < 16; j++)
-      s_x[(h * 16 + j) * 64 + col] = make_float4 (v[j].re.x, v[j].re.y, v[j].im.x, v[j].im.y);
+      s_x[(h * 16 + j) * P + pr] = make_float4 (v[j].re.x, v[j].re.y, v[j].im.x, v[j].im.y);
     __syncthreads ();
     float2* d0 = scratch + (uint64_t (b) * in.nchan + c) * 2 * N + i2;
 #pragma unroll
     for (int m = 0; m < 8; m++)
     {
       const unsigned j = 8 * h + m;
-      const float4 a = s_x[j * 64 + col], o = s_x[(16 + j) * 64 + col];
+      const float4 a = s_x[j * P + pr], o = s_x[(16 + j) * P + pr];
       const C2 e = {make_float2 (a.x, a.y), make_float2 (a.z, a.w)};
       const C2 f = {make_float2 (o.x, o.y), make_float2 (o.z, o.w)};
       const C2 x[2] = {dft::add (e, f), dft::sub (e, f)};
@@ -289,9 +322,13 @@ void launch_fwd_pair_t (const InputView& in, const float* lut, uint64_t nkeep, u
 {
   if constexpr (N1 == 32)
   {
-    const unsigned gx = n2 / 64;
-    const unsigned want = std::max (1u, 32 * unsigned (nsm) / std::max (1u, gx * in.nchan));
-    k_fwd_cols_pair32<KIND, AFFINE><<<dim3 (gx, std::min (nbatch, want), in.nchan), 128, 0, st>>> (
+    const unsigned gx = n2 / (TILE ? 16 : 64), gz = TILE ? in.nchan / FWP_CH : in.nchan;
+    const unsigned want = std::max (1u, (TILE ? 16 : 32) * unsigned (nsm) / std::max (1u, gx * gz));
+    auto kern = k_fwd_cols_pair32<KIND, AFFINE, TILE>;
+    constexpr size_t smem = fwp32_smem<KIND, TILE> ();
+    if (TILE)
+      cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int (smem));
+    kern<<<dim3 (gx, std::min (nbatch, want), gz), fwp32_threads<TILE> (), smem, st>>> (
         in, lut, nkeep, part0, nbatch, n2, tw4, scratch, apod);
     return;
   }
@@ -325,15 +362,15 @@ void launch_fwd_pair (const InputView& in, const float* lut, uint64_t nkeep, uin
                       unsigned nbatch, unsigned n2, const float2* tw4, float2* scratch,
                       const float* apod, int nsm, cudaStream_t st)
 {
-  const bool tile = N1 <= 16 && in.nchan % FWP_CH == 0;
+  const bool tile = in.nchan % FWP_CH == 0;
   if (in.kind == IN_INT8 && in.lut_scale != 0.f)
-    (tile ? launch_fwd_pair_t<N1, IN_INT8, true, N1 <= 16> : launch_fwd_pair_t<N1, IN_INT8, true, false>) (
+    (tile ? launch_fwd_pair_t<N1, IN_INT8, true, true> : launch_fwd_pair_t<N1, IN_INT8, true, false>) (
         in, lut, nkeep, part0, nbatch, n2, tw4, scratch, apod, nsm, st);
   else if (in.kind == IN_INT8)
-    (tile ? launch_fwd_pair_t<N1, IN_INT8, false, N1 <= 16> : launch_fwd_pair_t<N1, IN_INT8, false, false>) (
+    (tile ? launch_fwd_pair_t<N1, IN_INT8, false, true> : launch_fwd_pair_t<N1, IN_INT8, false, false>) (
         in, lut, nkeep, part0, nbatch, n2, tw4, scratch, apod, nsm, st);
   else if (in.kind == IN_INT16)
-    (tile ? launch_fwd_pair_t<N1, IN_INT16, false, N1 <= 16> : launch_fwd_pair_t<N1, IN_INT16, false, false>) (
+    (tile ? launch_fwd_pair_t<N1, IN_INT16, false, true> : launch_fwd_pair_t<N1, IN_INT16, false, false>) (
         in, lut, nkeep, part0, nbatch, n2, tw4, scratch, apod, nsm, st);
   else
     launch_fwd_pair_t<N1, IN_FLOAT, false, false> (in, lut, nkeep, part0, nbatch, n2, tw4, scratch,
