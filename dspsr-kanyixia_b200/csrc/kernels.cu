@@ -790,13 +790,14 @@ __device__ __forceinline__ int warp_seg_search (const FoldSegment* __restrict__ 
 
 // The column warp_fold_bin would give each sample.  A warp takes
 // COLPLAN_SAMPLES consecutive samples, each lane four at a time (one 16-byte
-// store): one search for the first sample, then each lane steps forward over
-// the segment boundaries from where the previous group's last lane ended,
-// and a lane's samples advance m by dm within a segment.  Bound by latency
-// (the search, the segment loads and the double chain), so the serial chain
-// per warp is kept short: one sample per lane and 32 groups per warp took
-// 37.6 us for 10 M samples and 7.7 us for 60 k; this takes 24.2 and 3.9 us.
+// store): one search for the first sample, further ones in groups that cross
+// a segment boundary, and a lane's samples advance m by dm within a segment.
+// Bound by latency (the search, the segment loads and the double chain), so
+// the serial chain per warp is kept short: one sample per lane and 32 groups
+// per warp took 37.6 us for 10 M samples and 7.7 us for 60 k; this takes 24.2 and 3.9 us.
 // (Adding powers of two instead of the 64-bit conversions: 31.0 us.)
+// Stepping lane by lane through runs of one-sample segments took 33 us for
+// 860 segments in 6 M samples, the search per lane 16 us.
 constexpr int COLPLAN_SAMPLES = 512;
 
 __global__ void __launch_bounds__ (256)
@@ -813,6 +814,14 @@ k_colplan (const FoldSegment* __restrict__ segs, const int nseg, const uint64_t 
   for (int g = 0; g < COLPLAN_SAMPLES; g += 128)
   {
     const uint64_t t0 = w0 + unsigned (g) + 4 * lane;
+    // where the group crosses segments (hundreds of one-sample ones can follow
+    // one another) each lane searches for its own
+    const uint64_t last = w0 + unsigned (g) + 127;
+    if (s + 1 < nseg && __ldg (&segs[s + 1].start) <= last)
+    {
+      const int e = s + warp_seg_search (segs + s, nseg - s, last);
+      s += seg_search (segs + s, e - s + 1, t0);
+    }
     unsigned c[4];
     int64_t m = 0, dm = 0;
     double gr = 0;
