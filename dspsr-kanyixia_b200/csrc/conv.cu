@@ -42,16 +42,17 @@ __device__ __forceinline__ void smem_pass (float2* s, float2* v, const float2* t
   {
     constexpr int R = stockham_radix (N, P);
     constexpr int Ns = stockham_ns (N, P);
-    StockhamPass<N, R, T, D>::load (threadIdx.x, s, v);
+    StockhamPass<N, R, T, D>::load (threadIdx.x % T, s, v);
     __syncthreads ();
-    StockhamPass<N, R, T, D>::compute_store (threadIdx.x, Ns, v, s, tw);
+    StockhamPass<N, R, T, D>::compute_store (threadIdx.x % T, Ns, v, s, tw);
     __syncthreads ();
     smem_pass<N, T, D, P + 1> (s, v, tw);
   }
 }
 
-// N-point FFT of s[spad(0..N-1)] in place; the caller has synchronised after
-// writing s.  Returns synchronised.
+// N-point FFT of s[spad(0..N-1)] in place by T threads; the caller has
+// synchronised after writing s.  Returns synchronised.  Groups of T threads may
+// transform their own arrays side by side (the barriers are the block's).
 template <int N, int T, int D>
 __device__ __forceinline__ void smem_fft (float2* s, const float2* tw)
 {
@@ -197,8 +198,14 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
 // single-kernel path (n1 == 1): everything in shared memory
 // --------------------------------------------------------------------------
 
+// Groups of T threads take one polarisation each, side by side where 512
+// threads hold them (a call of one or two parts waits for one block's chain of
+// passes: 31 us one after the other, 24 us side by side at 4096 points), one
+// after the other at 8192 points.
+template <int T> B200_CE int fused_groups (unsigned npol) { return 2 * T <= 512 ? npol : 1; }
+
 template <int N, int T, int KIND, int MODE, int NOUT>
-__global__ void __launch_bounds__ (T, 512 / T)
+__global__ void __launch_bounds__ (512, 1)
 k_fused (const InputView in, const float* __restrict__ lut, const float2* __restrict__ tw,
          const float2* __restrict__ H, const uint64_t nkeep, const unsigned nfilt_pos,
          const uint64_t part0, const FoldView fv, const VoltView vv,
@@ -211,10 +218,15 @@ k_fused (const InputView in, const float* __restrict__ lut, const float2* __rest
   const unsigned c = blockIdx.y;
   const uint64_t part = part0 + b;
   const unsigned npol = in.npol;
+  const unsigned groups = blockDim.x / T, group = threadIdx.x / T, tid = threadIdx.x % T;
   load_lut (in, lut, s_lut);
   __syncthreads ();
-  for (unsigned p = 0; p < npol; p++)
-    for (int i = threadIdx.x; i < N; i += T)
+  const float2* h = H + uint64_t (c) * N;
+  for (unsigned p = group; p < npol; p += groups)
+  {
+    float2* sp = s + p * SP;
+#pragma unroll 4
+    for (int i = tid; i < N; i += T)
     {
       float2 x = fetch<KIND> (in, s_lut, c, p, part * nkeep + i);
       if (apod)
@@ -222,15 +234,12 @@ k_fused (const InputView in, const float* __restrict__ lut, const float2* __rest
         const float w = __ldg (apod + i);
         x = make_float2 (__fmul_rn (x.x, w), __fmul_rn (x.y, w));
       }
-      s[p * SP + spad (i)] = x;
+      sp[spad (i)] = x;
     }
-  __syncthreads ();
-  const float2* h = H + uint64_t (c) * N;
-  for (unsigned p = 0; p < npol; p++)
-  {
-    float2* sp = s + p * SP;
+    __syncthreads ();
     smem_fft<N, T, -1> (sp, tw);
-    for (int i = threadIdx.x; i < N; i += T)
+#pragma unroll 4
+    for (int i = tid; i < N; i += T)
     {
       const float2 d = sp[spad (i)];
       const float2 f = __ldg (h + i);
@@ -242,10 +251,10 @@ k_fused (const InputView in, const float* __restrict__ lut, const float2* __rest
   const uint64_t tbase = part * nkeep;
   float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
   unsigned* hits = c == 0 ? fv.hits : nullptr;
-  const unsigned rounds = unsigned ((nkeep + T - 1) / T);
+  const unsigned rounds = unsigned ((nkeep + blockDim.x - 1) / blockDim.x);
   for (unsigned r = 0; r < rounds; r++)
   {
-    const uint64_t j = uint64_t (r) * T + threadIdx.x;
+    const uint64_t j = uint64_t (r) * blockDim.x + threadIdx.x;
     const bool ok = j < nkeep;
     const int tl = ok ? int (nfilt_pos + j) : 0;
     const float2 pv = s[spad (tl)];
@@ -401,8 +410,8 @@ cudaError_t run_fused_t (const ConvShape& sh, const ConvTables& tb, const InputV
   cudaError_t err = fused_setup<N, KIND, MODE, NOUT> ();
   if (err != cudaSuccess) return err;
   ClockScope cs (clk, KK_FUSED, st);
-  kern<<<dim3 (nbatch, sh.nchan), T, smem, st>>> (in, tb.lut, tb.tw2, tb.H, sh.nkeep,
-                                                  sh.nfilt_pos, part0, fv, vv, tb.apod);
+  kern<<<dim3 (nbatch, sh.nchan), T * fused_groups<T> (in.npol), smem, st>>> (
+      in, tb.lut, tb.tw2, tb.H, sh.nkeep, sh.nfilt_pos, part0, fv, vv, tb.apod);
   return cudaGetLastError ();
 }
 
