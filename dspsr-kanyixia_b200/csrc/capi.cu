@@ -2479,7 +2479,8 @@ int dspsr_b200_unpack8 (dspsr_b200_context* ctx, const void* d_in, uint64_t ndat
   B200_CHECK (ctx, cudaMemcpyAsync (ctx->d_lut, lut256, 256 * sizeof (float),
                                     cudaMemcpyHostToDevice, ctx->stream), "upload lut");
   B200_CHECK (ctx, launch_unpack8 (static_cast<const uint8_t*> (d_in), ndat, nchan, npol, ndim,
-                                   ctx->d_lut, d_out, out_span, ctx->stream), "unpack8");
+                                   ctx->d_lut, affine_lut_scale (lut256), d_out, out_span,
+                                   ctx->stream), "unpack8");
   // the LUT buffer is reused by the next call: keep this call's upload ordered
   return DSPSR_B200_OK;
 }

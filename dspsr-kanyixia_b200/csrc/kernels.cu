@@ -3,6 +3,7 @@
 
 #include "device_common.cuh"
 #include "fb_warp.cuh"
+#include "fwd_cols_pair.cuh"
 #include "group_fft.cuh"
 
 namespace b200 {
@@ -432,6 +433,43 @@ __global__ void k_unpack16 (const int16_t* __restrict__ in, const uint64_t ndat,
       short v = src[p * ndim + d];
       if (offset_binary) v = short (v ^ 0x8000);
       out[(uint64_t (c) * npol + p) * span + t * ndim + d] = __fadd_rn (float (v), 0.5f);
+    }
+}
+
+// The unpackers for dual-polarisation complex samples: one word per sample,
+// both polarisations unpacked together, an affine 8-bit table computed instead
+// of looked up (a warp's lookups fall in few banks at a time).  UNPACK_T
+// samples per thread keep that many loads in flight.  Bound by HBM: 17.0 us
+// before, 7.9 us now for 2^21 samples (42 MB).
+constexpr int UNPACK_T = 4;
+
+template <int KIND, bool AFFINE>
+__global__ void __launch_bounds__ (256)
+k_unpack_pair (const typename RawPair<KIND>::T* __restrict__ in, const uint64_t ndat,
+               const unsigned nchan, const float* __restrict__ lut, const float scale,
+               const int offset_binary, float2* __restrict__ out, const uint64_t span)
+{
+  __shared__ float s_lut[KIND == IN_INT8 && !AFFINE ? 256 : 1];
+  if constexpr (KIND == IN_INT8 && !AFFINE)
+  {
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = lut[i];
+    __syncthreads ();
+  }
+  const UnpackPair u {s_lut, scale, offset_binary ? 0u : 0x80008000u};
+  const uint64_t t0 = uint64_t (blockIdx.x) * (256 * UNPACK_T) + threadIdx.x;
+  const unsigned c = blockIdx.y;
+  typename RawPair<KIND>::T w[UNPACK_T];
+#pragma unroll
+  for (int k = 0; k < UNPACK_T; k++)
+    if (t0 + 256 * k < ndat) w[k] = __ldg (in + (t0 + 256 * k) * nchan + c);
+#pragma unroll
+  for (int k = 0; k < UNPACK_T; k++)
+    if (t0 + 256 * k < ndat)
+    {
+      const C2 x = unpack_pair<KIND, AFFINE> (w[k], u);
+      float2* o = out + uint64_t (c) * 2 * span + t0 + 256 * k;
+      o[0] = make_float2 (x.re.x, x.im.x);
+      o[span] = make_float2 (x.re.y, x.im.y);
     }
 }
 
@@ -1097,12 +1135,32 @@ cudaError_t launch_sk (const float2* in, uint64_t in_span, float2* out, uint64_t
   return cudaGetLastError ();
 }
 
+namespace {
+
+// dual-polarisation complex samples whose words and output values are aligned
+bool unpack_as_pairs (const void* in, unsigned word, unsigned npol, unsigned ndim, const float* out,
+                      uint64_t span)
+{
+  return npol == 2 && ndim == 2 && reinterpret_cast<uintptr_t> (in) % word == 0
+         && reinterpret_cast<uintptr_t> (out) % 8 == 0 && span % 2 == 0;
+}
+
+} // namespace
+
 cudaError_t launch_unpack8 (const uint8_t* in, uint64_t ndat, unsigned nchan, unsigned npol,
-                            unsigned ndim, const float* d_lut, float* out, uint64_t span,
-                            cudaStream_t st)
+                            unsigned ndim, const float* d_lut, float lut_scale, float* out,
+                            uint64_t span, cudaStream_t st)
 {
   if (ndat == 0) return cudaSuccess;
   g_launches++;
+  if (unpack_as_pairs (in, 4, npol, ndim, out, span))
+  {
+    const dim3 grid (unsigned ((ndat + 256 * UNPACK_T - 1) / (256 * UNPACK_T)), nchan);
+    auto k = lut_scale != 0.f ? k_unpack_pair<IN_INT8, true> : k_unpack_pair<IN_INT8, false>;
+    k<<<grid, 256, 0, st>>> (reinterpret_cast<const unsigned*> (in), ndat, nchan, d_lut, lut_scale, 0,
+                             reinterpret_cast<float2*> (out), span / 2);
+    return cudaGetLastError ();
+  }
   k_unpack8<<<dim3 (unsigned ((ndat + 255) / 256), nchan), 256, 0, st>>> (
       in, ndat, nchan, npol, ndim, d_lut, out, span);
   return cudaGetLastError ();
@@ -1114,6 +1172,14 @@ cudaError_t launch_unpack16 (const int16_t* in, uint64_t ndat, unsigned nchan, u
 {
   if (ndat == 0) return cudaSuccess;
   g_launches++;
+  if (unpack_as_pairs (in, 8, npol, ndim, out, span))
+  {
+    const dim3 grid (unsigned ((ndat + 256 * UNPACK_T - 1) / (256 * UNPACK_T)), nchan);
+    k_unpack_pair<IN_INT16, false><<<grid, 256, 0, st>>> (
+        reinterpret_cast<const uint2*> (in), ndat, nchan, nullptr, 0.f, offset_binary,
+        reinterpret_cast<float2*> (out), span / 2);
+    return cudaGetLastError ();
+  }
   k_unpack16<<<dim3 (unsigned ((ndat + 255) / 256), nchan), 256, 0, st>>> (
       in, ndat, nchan, npol, ndim, offset_binary, out, span);
   return cudaGetLastError ();

@@ -302,8 +302,8 @@ cudaError_t launch_sk (const float2* in, uint64_t in_span, float2* out, uint64_t
                        cudaStream_t stream);
 
 cudaError_t launch_unpack8 (const uint8_t* in, uint64_t ndat, unsigned nchan, unsigned npol,
-                            unsigned ndim, const float* d_lut, float* out, uint64_t span,
-                            cudaStream_t stream);
+                            unsigned ndim, const float* d_lut, float lut_scale, float* out,
+                            uint64_t span, cudaStream_t stream);
 cudaError_t launch_unpack16 (const int16_t* in, uint64_t ndat, unsigned nchan, unsigned npol,
                              unsigned ndim, int offset_binary, float* out, uint64_t span,
                              cudaStream_t stream);
