@@ -248,12 +248,20 @@ k_filterbank_smem (const InputView in, const float* __restrict__ lut, const floa
 // shared atomic as they are met.  Shared memory holds U * npol columns of
 // Ms floats, Ms = M rounded up to a multiple of 4 plus 4 (so that the
 // columns read together fall on different banks).
-constexpr int SK_THREADS = 128;
+// Bound by HBM (16 B per sample) where M is short and by the chains of double
+// additions where it is long.  With a load behind each store, 128 threads and
+// two blocks per CTA 512 channels x 131072 samples took 459 us at M = 1024 and
+// 536 us at M = 256; now 376 and 329 us (6.5 TB/s).  More threads or blocks per
+// CTA (eight blocks, 512 threads) took 440 to 505 us at M = 1024, streaming
+// hints on the loads and stores 388.
+constexpr int SK_THREADS = 256;
+constexpr size_t SK_TILE = 40u << 10;           // five CTAs per SM
+constexpr int SK_BATCH = 4;
 
 __host__ __device__ inline unsigned sk_column (unsigned M) { return ((M + 3) & ~3u) + 4; }
 
 template <int U>
-__global__ void __launch_bounds__ (SK_THREADS, 12)
+__global__ void __launch_bounds__ (SK_THREADS, 5)
 k_sk (const float2* __restrict__ in, const uint64_t in_span, float2* out, const uint64_t out_span,
       const uint64_t npart, const unsigned nchan, const unsigned npol, const unsigned M,
       const int zero_is_valid, const unsigned Nd, const float lower,
@@ -281,30 +289,47 @@ k_sk (const float2* __restrict__ in, const uint64_t in_span, float2* out, const 
   float4* dst1 = dst0 + (two ? out_span / 2 : 0);
   __syncthreads ();
   const unsigned total = nu * n4;
-#pragma unroll 4
-  for (unsigned f = threadIdx.x; f < total; f += SK_THREADS)
+  // SK_BATCH loads per polarisation are issued before any is used: the stores
+  // may alias the loads, and the compiler would keep each load behind the
+  // store before it
+  for (unsigned f0 = threadIdx.x; f0 < total; f0 += SK_BATCH * SK_THREADS)
   {
-    const unsigned u = f / n4, i = f - u * n4;
-    const float4 a = __ldcs (src0 + f);
-    float4 b = a;
-    if (two) b = __ldcs (src1 + f);
-    if (through)
+    float4 a[SK_BATCH], b[SK_BATCH];
+#pragma unroll
+    for (int k = 0; k < SK_BATCH; k++)
     {
-      __stcs (dst0 + f, a);
-      if (two) __stcs (dst1 + f, b);
+      const unsigned f = f0 + k * SK_THREADS;
+      a[k] = b[k] = make_float4 (1.f, 1.f, 1.f, 1.f);
+      if (f < total)
+      {
+        a[k] = src0[f];
+        if (two) b[k] = src1[f];
+      }
     }
-    const float a0 = __fadd_rn (__fmul_rn (a.x, a.x), __fmul_rn (a.y, a.y));
-    const float a1 = __fadd_rn (__fmul_rn (a.z, a.z), __fmul_rn (a.w, a.w));
-    float2* q0 = reinterpret_cast<float2*> (s_sqld + (u * npol) * Ms);
-    q0[i] = make_float2 (a0, a1);
-    // Mprime counts pol 0, as detect_skfb reads it
-    if (!zero_is_valid && (a0 == 0.0f || a1 == 0.0f))
-      atomicAdd (&s_zero[u], unsigned (a0 == 0.0f) + unsigned (a1 == 0.0f));
-    if (two)
+#pragma unroll
+    for (int k = 0; k < SK_BATCH; k++)
     {
-      float2* q1 = reinterpret_cast<float2*> (s_sqld + (u * npol + 1) * Ms);
-      q1[i] = make_float2 (__fadd_rn (__fmul_rn (b.x, b.x), __fmul_rn (b.y, b.y)),
-                           __fadd_rn (__fmul_rn (b.z, b.z), __fmul_rn (b.w, b.w)));
+      const unsigned f = f0 + k * SK_THREADS;
+      if (f >= total) break;
+      if (through)
+      {
+        dst0[f] = a[k];
+        if (two) dst1[f] = b[k];
+      }
+      const unsigned u = U == 1 || f < n4 ? 0 : f / n4, i = f - u * n4;
+      const float a0 = __fadd_rn (__fmul_rn (a[k].x, a[k].x), __fmul_rn (a[k].y, a[k].y));
+      const float a1 = __fadd_rn (__fmul_rn (a[k].z, a[k].z), __fmul_rn (a[k].w, a[k].w));
+      float2* q0 = reinterpret_cast<float2*> (s_sqld + (u * npol) * Ms);
+      q0[i] = make_float2 (a0, a1);
+      // Mprime counts pol 0, as detect_skfb reads it
+      if (!zero_is_valid && (a0 == 0.0f || a1 == 0.0f))
+        atomicAdd (&s_zero[u], unsigned (a0 == 0.0f) + unsigned (a1 == 0.0f));
+      if (two)
+      {
+        float2* q1 = reinterpret_cast<float2*> (s_sqld + (u * npol + 1) * Ms);
+        q1[i] = make_float2 (__fadd_rn (__fmul_rn (b[k].x, b[k].x), __fmul_rn (b[k].y, b[k].y)),
+                             __fadd_rn (__fmul_rn (b[k].z, b[k].z), __fmul_rn (b[k].w, b[k].w)));
+      }
     }
   }
   __syncthreads ();
@@ -1118,13 +1143,15 @@ cudaError_t launch_sk (const float2* in, uint64_t in_span, float2* out, uint64_t
                        unsigned* counts, uint8_t* mask, unsigned long long* nzap, cudaStream_t st)
 {
   if (npart == 0) return cudaSuccess;
-  // two blocks per CTA while they fit in a modest footprint, else one
-  const unsigned units = sk_smem_bytes (npol, M, 2) <= (48u << 10) ? 2 : 1;
+  // as many blocks per CTA as SK_TILE holds: the sums of one occupy 4 lanes of
+  // a warp, and a tile is streamed in two rounds of loads
+  unsigned units = 8;
+  while (units > 1 && sk_smem_bytes (npol, M, units) > SK_TILE) units /= 2;
   const size_t smem = sk_smem_bytes (npol, M, units);
   if (smem > SK_SMEM_MAX) return cudaErrorInvalidValue;
   const uint64_t nblk = (npart + units - 1) / units;
   if (nblk > 0x7fffffffull || nchan > 65535) return cudaErrorInvalidValue;
-  auto kern = units == 2 ? k_sk<2> : k_sk<1>;
+  auto kern = units == 8 ? k_sk<8> : units == 4 ? k_sk<4> : units == 2 ? k_sk<2> : k_sk<1>;
   cudaError_t e = cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int (smem));
   if (e != cudaSuccess) return e;

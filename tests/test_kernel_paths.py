@@ -10,6 +10,7 @@ oracle chain's power (float sums of a few hundred samples per bin), voltages
 import numpy as np
 import pytest
 
+import test_sk as sk
 from test_gpu_pipeline import base_cfg, check, make_blocks, oracle_chain, run_pipeline
 
 torch = pytest.importorskip("torch")
@@ -233,3 +234,15 @@ def test_rows_change_with_the_arithmetic(ctx, b2, orc):
         c.status()
         assert rel_rms(out.cpu().numpy(), ref) < VOLTAGE_RTOL
     c.close()
+
+
+# spectral kurtosis: 8, 4, 2 and 1 blocks per thread block at the edges of the
+# shared tile, counts that leave the last one partly empty
+SK_EDGES = [(4, 2, 636, 9), (4, 2, 638, 9), (4, 2, 1276, 7), (4, 2, 1278, 7), (4, 2, 2556, 5),
+            (4, 2, 2558, 5), (4, 1, 1276, 17), (4, 1, 1278, 17), (4, 2, 30, 49)]
+
+
+@pytest.mark.parametrize("nchan,npol,M,npart", SK_EDGES)
+@pytest.mark.parametrize("inplace", [False, True])
+def test_sk_tiles_bit_exact(ctx, b2, orc, nchan, npol, M, npart, inplace):
+    sk.test_sk_kernel_bit_exact(ctx, b2, orc, nchan, npol, M, npart * M + 6, 0, False, 1, inplace)
