@@ -680,9 +680,9 @@ typedef struct
      on its own (fused_filterbank is ignored). */
   unsigned sk_M;
   float sk_std_devs;
-  /* tuning: the four-step split's row length, 8192 (0 = default) or 4096
-     (nfft from 8192 to 131072, n1 = nfft / 4096 columns; the tensor-core rows
-     need 8192) */
+  /* tuning: the four-step split's row length, 8192 or 4096 (nfft from 8192 to
+     131072, n1 = nfft / 4096 columns; the tensor-core rows need 8192); 0 =
+     4096 for FP32 rows and nfft from 16384 to 131072, else 8192 */
   unsigned row_length;
 } dspsr_b200_pipeline_config;
 
