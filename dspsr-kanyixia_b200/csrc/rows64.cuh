@@ -3,6 +3,7 @@
 
 #include "device_common.cuh"
 #include "dft_pair.cuh"
+#include "tcgen05.cuh"
 
 namespace b200 {
 
@@ -59,23 +60,6 @@ __device__ __forceinline__ bool r64_all (int g, bool ok)
                 : "r"(unsigned (ok)), "r"(g + 1)
                 : "memory");
   return r != 0;
-}
-
-// bounded wait for the bulk copy of a row: about 2^21 polls
-__device__ __forceinline__ bool r64_wait (uint64_t* bar, unsigned parity)
-{
-  for (int it = 0; it < (1 << 21); it++)
-  {
-    uint32_t ok;
-    asm volatile ("{\n\t.reg .pred p;\n\t"
-                  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                  "selp.u32 %0, 1, 0, p;\n\t}"
-                  : "=r"(ok)
-                  : "r"(r64_saddr (bar)), "r"(parity)
-                  : "memory");
-    if (ok) return true;
-  }
-  return false;
 }
 
 // one thread: copy a row (32 KB, both ends 16-byte aligned) into the group's
@@ -164,12 +148,12 @@ k_rows64 (float2* scratch, const float2* __restrict__ H, const unsigned n1, cons
         asm volatile ("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(next + o), "r"(16384u)
                       : "memory");
     }
-    if (!r64_all (g, r64_wait (bar, phase)))
+    if (!r64_all (g, tc::bar_wait (bar, phase)))
     {
       // the copy did not land in time: report, give it a last chance to
       // finish before the block's shared memory goes, and leave
       if (t == 0 && err) *err = 1;
-      r64_wait (bar, phase);
+      tc::bar_wait (bar, phase);
       return;
     }
     phase ^= 1;

@@ -71,11 +71,27 @@ __device__ __forceinline__ bool bar_try (uint64_t* bar, unsigned parity)
   return ok != 0;
 }
 
-// bounded: about 2^21 polls (a second or so)
+__device__ __forceinline__ uint64_t wall_ns ()
+{
+  uint64_t t;
+  asm volatile ("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Bounded: gives up after 2^21 polls, or after BAR_WAIT_NS.  A poll may be
+// suspended for as long as the hardware likes, so that a number of polls alone
+// is no bound in time; the time is looked at every 16 polls (and never before
+// 16, so that a block taken off the SM for long finds a copy that has landed).
+constexpr uint64_t BAR_WAIT_NS = 1000000000ull;
 __device__ __forceinline__ bool bar_wait (uint64_t* bar, unsigned parity)
 {
-  for (int it = 0; it < (1 << 21); it++)
+  if (bar_try (bar, parity)) return true;
+  const uint64_t t0 = wall_ns ();
+  for (int it = 1; it < (1 << 21); it++)
+  {
     if (bar_try (bar, parity)) return true;
+    if ((it & 15) == 0 && wall_ns () - t0 > BAR_WAIT_NS) return false;
+  }
   return false;
 }
 
