@@ -81,6 +81,18 @@ uint64_t ConvolutionEngine::perform (const TimeSeriesView& in, TimeSeriesView& o
   return npart;
 }
 
+void ConvolutionEngine::status ()
+{
+  ctx.check (dspsr_b200_convolution_status (conv), "ConvolutionEngine::status");
+}
+
+int* ConvolutionEngine::status_word ()
+{
+  int* word = nullptr;
+  ctx.check (dspsr_b200_convolution_status_word (conv, &word), "ConvolutionEngine::status_word");
+  return word;
+}
+
 // ---- filterbank ---------------------------------------------------------------
 
 uint64_t FilterbankEngine::perform (const TimeSeriesView& in, TimeSeriesView& out)

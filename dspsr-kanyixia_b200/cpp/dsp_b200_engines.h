@@ -81,8 +81,14 @@ public:
   // Dedispersion built on the device (FP64 phase); chirp_mode as in the C ABI
   void set_dedispersion (double centre_freq, double bandwidth, double dm, int input_nchan,
                          int dual_sideband, int chirp_mode = DSPSR_B200_CHIRP_REFERENCE);
-  // Engine::perform(input, output, npart); returns npart
+  // Engine::perform(input, output, npart); returns npart.  Queued, not waited
+  // for: a device-side wait that gives up is reported by the call that takes
+  // results or waits (FoldEngine::synch, Context::synchronize), or by status
   uint64_t perform (const TimeSeriesView& input, TimeSeriesView& output);
+  // waits for the queued work; throws if a device-side wait gave up
+  void status ();
+  // the status word (dspsr_b200_convolution_status_word)
+  int* status_word ();
 private:
   Context& ctx;
   dspsr_b200_convolution* conv = nullptr;

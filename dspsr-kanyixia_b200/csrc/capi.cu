@@ -52,6 +52,56 @@ int cuda_fail (dspsr_b200_context* ctx, cudaError_t err, const char* where)
 
 bool is_pow2 (uint64_t x) { return x && !(x & (x - 1)); }
 
+// Status word of a convolution: a kernel sets it when one of its bounded waits
+// gave up.  It lies in host memory that the device can write, so that whoever
+// hands out results reads it after the synchronisation that it makes anyway.
+struct WaitFlag
+{
+  std::shared_ptr<dspsr_b200_wait_words> owner;
+  int* host = nullptr;
+  int* dev = nullptr;
+  cudaError_t create (dspsr_b200_context* ctx)
+  {
+    const cudaError_t e = cudaHostAlloc (&host, sizeof (int), cudaHostAllocMapped);
+    if (e != cudaSuccess)
+    {
+      host = nullptr;
+      return e;
+    }
+    *host = 0;
+    owner = ctx->waits;
+    std::lock_guard<std::mutex> g (owner->lock);
+    owner->words.push_back (host);
+    return cudaHostGetDevicePointer (&dev, host, 0);
+  }
+  bool set () const { return host && *static_cast<const volatile int*> (host); }
+  void release ()
+  {
+    if (!host) return;
+    {
+      std::lock_guard<std::mutex> g (owner->lock);
+      owner->words.erase (std::find (owner->words.begin (), owner->words.end (), host));
+    }
+    cudaFreeHost (host);
+    host = dev = nullptr;
+  }
+};
+
+int wait_failed (dspsr_b200_context* ctx)
+{
+  return fail (ctx, DSPSR_B200_ESTATE, "a device-side wait timed out");
+}
+
+// ESTATE when a wait of any convolution of the context has given up; the
+// caller has synchronised with the work that it asks about
+int context_waits (dspsr_b200_context* ctx)
+{
+  std::lock_guard<std::mutex> g (ctx->waits->lock);
+  for (const volatile int* w : ctx->waits->words)
+    if (*w) return wait_failed (ctx);
+  return DSPSR_B200_OK;
+}
+
 // Per-pass Stockham tables of an n-point transform uploaded into a device
 // buffer (the shared-memory filterbank's twiddles).
 cudaError_t upload_pass_tables (unsigned n, float2** dst, size_t* cap)
@@ -145,7 +195,7 @@ struct dspsr_b200_convolution
   DevBuf<float2> tw2, tw4, H, tmp, scratch;
   DevBuf<double> chan_par;
   DevBuf<float> lut, apod;
-  DevBuf<int> err;
+  WaitFlag waits;
   DevBuf<uint8_t> tc_dft;
   int tc_splits = 0;
   int nsm = 148;
@@ -172,7 +222,7 @@ struct dspsr_b200_convolution
     t.tw4 = tw4.ptr;
     t.H = H.ptr;
     t.lut = lut.ptr;
-    t.err = err.ptr;
+    t.err = waits.dev;
     t.nsm = nsm;
     t.apod = have_apod ? apod.ptr : nullptr;
     t.tc_dft = tc_dft.ptr;
@@ -190,18 +240,13 @@ struct dspsr_b200_convolution
     scratch.release ();
     chan_par.release ();
     lut.release ();
-    err.release ();
+    waits.release ();
   }
   // ESTATE when a bounded device wait of the row kernel gave up
   int status ()
   {
-    if (!err.ptr) return DSPSR_B200_OK;
-    int h = 0;
-    B200_CHECK (ctx, cudaMemcpyAsync (&h, err.ptr, sizeof (int), cudaMemcpyDeviceToHost,
-                                      ctx->stream), "read device status");
     B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "device status sync");
-    if (h) return fail (ctx, DSPSR_B200_ESTATE, "a device-side wait timed out");
-    return DSPSR_B200_OK;
+    return waits.set () ? wait_failed (ctx) : DSPSR_B200_OK;
   }
 };
 
@@ -238,6 +283,7 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
   if (rc) return rc;
   B200_CHECK (ctx, H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
   B200_CHECK (ctx, lut.reserve (256), "cudaMalloc lut");
+  B200_CHECK (ctx, waits.create (ctx), "status word");
   return DSPSR_B200_OK;
 }
 
@@ -269,8 +315,6 @@ int dspsr_b200_convolution::split (unsigned row_len)
     std::vector<float2> t4 = make_tw4 (shape.n1, shape.n2);
     B200_CHECK (ctx, cudaMemcpy (tw4.ptr, t4.data (), t4.size () * sizeof (float2),
                                  cudaMemcpyHostToDevice), "copy tw4");
-    B200_CHECK (ctx, err.reserve (1), "cudaMalloc status flag");
-    B200_CHECK (ctx, cudaMemset (err.ptr, 0, sizeof (int)), "clear status flag");
     int dev = 0;
     B200_CHECK (ctx, cudaGetDevice (&dev), "cudaGetDevice");
     B200_CHECK (ctx, cudaDeviceGetAttribute (&nsm, cudaDevAttrMultiProcessorCount, dev),
@@ -699,7 +743,6 @@ struct dspsr_b200_pipeline
   uint64_t pinned_bytes = 0;
   cudaEvent_t host_free[2] = {nullptr, nullptr};   // uploads of pinned[b] done
   cudaEvent_t snap_ev = nullptr;    // the last asynchronous profile snapshot landed
-  int* snap_err = nullptr;          // pinned copy of the row kernel's wait flag at the snapshot
   bool host_free_pending[2] = {false, false};
 };
 
@@ -825,7 +868,7 @@ int subint_take (dspsr_b200_pipeline* pl, int k, dspsr_b200_subint* info, float*
   rc = pl->fold.reset_slot (unsigned (k));
   if (rc) return rc;
   pl->sub_slots[k].used = false;
-  return DSPSR_B200_OK;
+  return pl->conv.waits.set () ? wait_failed (ctx) : DSPSR_B200_OK;
 }
 
 // PhaseSeriesUnloader::unload for every closed sub-integration, in order.
@@ -877,6 +920,17 @@ int subint_drain (dspsr_b200_pipeline* pl, bool wait)
       const cudaError_t e = cudaEventQuery (u.ev);
       if (e == cudaErrorNotReady) break;
       B200_CHECK (ctx, e, "unload copy");
+    }
+    if (pl->conv.waits.set ())
+    {
+      // what has been folded is not valid: none of it goes to the callback
+      for (auto& v : pl->sub_pending)
+      {
+        B200_CHECK (ctx, cudaEventSynchronize (v.ev), "wait unload");
+        pl->sub_spare.push_back (v);
+      }
+      pl->sub_pending.clear ();
+      return wait_failed (ctx);
     }
     pl->unload_fn (pl->unload_user, &u.info, u.prof, u.hits);
     pl->sub_spare.push_back (u);
@@ -2097,7 +2151,7 @@ int dspsr_b200_synchronize (dspsr_b200_context* ctx)
 {
   if (!ctx) return DSPSR_B200_EINVAL;
   B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "cudaStreamSynchronize");
-  return DSPSR_B200_OK;
+  return context_waits (ctx);
 }
 
 unsigned dspsr_b200_smearing_samples (double cf, double bw, double dm, unsigned nchan, int half)
@@ -2534,6 +2588,13 @@ int dspsr_b200_convolution_status (dspsr_b200_convolution* c)
   return c->status ();
 }
 
+int dspsr_b200_convolution_status_word (dspsr_b200_convolution* c, int** word)
+{
+  if (!c || !word) return DSPSR_B200_EINVAL;
+  *word = c->waits.host;
+  return DSPSR_B200_OK;
+}
+
 int dspsr_b200_convolution_copy_response (dspsr_b200_convolution* c, const float* response)
 {
   if (!c) return DSPSR_B200_EINVAL;
@@ -2858,7 +2919,7 @@ int dspsr_b200_fold_get_profiles (dspsr_b200_fold* f, float* profiles, uint32_t*
     B200_CHECK (ctx, cudaMemcpyAsync (hits, f->hits.ptr, f->nbin * sizeof (unsigned),
                                       cudaMemcpyDeviceToHost, ctx->stream), "download hits");
   B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "get_profiles sync");
-  return DSPSR_B200_OK;
+  return context_waits (ctx);
 }
 
 int dspsr_b200_fold_reset (dspsr_b200_fold* f)
@@ -3077,7 +3138,6 @@ int dspsr_b200_pipeline_destroy (dspsr_b200_pipeline* pl)
     if (pl->host_free[i]) cudaEventDestroy (pl->host_free[i]);
   }
   if (pl->snap_ev) cudaEventDestroy (pl->snap_ev);
-  if (pl->snap_err) cudaFreeHost (pl->snap_err);
   for (auto& u : pl->sub_pending) pl->sub_spare.push_back (u);   // undelivered: dropped
   for (auto& u : pl->sub_spare)
   {
@@ -3280,9 +3340,7 @@ int dspsr_b200_pipeline_get_profiles (dspsr_b200_pipeline* pl, float* profiles, 
     return fail (pl->ctx, DSPSR_B200_ESTATE,
                  "pipeline_get_profiles: the pipeline folds sub-integrations; take them with "
                  "pop_subint or an unloader");
-  int rc = dspsr_b200_fold_get_profiles (&pl->fold, profiles, hits);
-  if (rc) return rc;
-  return pl->conv.status ();
+  return dspsr_b200_fold_get_profiles (&pl->fold, profiles, hits);
 }
 
 int dspsr_b200_pipeline_get_profiles_async (dspsr_b200_pipeline* pl, float* profiles,
@@ -3299,15 +3357,6 @@ int dspsr_b200_pipeline_get_profiles_async (dspsr_b200_pipeline* pl, float* prof
   if (!pl->snap_ev)
     B200_CHECK (ctx, cudaEventCreateWithFlags (&pl->snap_ev, cudaEventDisableTiming),
                 "cudaEventCreate");
-  if (!pl->snap_err)
-  {
-    B200_CHECK (ctx, cudaHostAlloc (&pl->snap_err, sizeof (int), cudaHostAllocDefault),
-                "cudaHostAlloc status");
-    *pl->snap_err = 0;
-  }
-  if (pl->conv.err.ptr)
-    B200_CHECK (ctx, cudaMemcpyAsync (pl->snap_err, pl->conv.err.ptr, sizeof (int),
-                                      cudaMemcpyDeviceToHost, ctx->stream), "read device status");
   if (profiles)
     B200_CHECK (ctx, cudaMemcpyAsync (profiles, f.profiles.ptr,
                                       uint64_t (f.nchan) * f.npol * f.nbin * sizeof (float),
@@ -3324,9 +3373,13 @@ int dspsr_b200_pipeline_wait_profiles (dspsr_b200_pipeline* pl)
   if (!pl) return DSPSR_B200_EINVAL;
   if (pl->snap_ev)
     B200_CHECK (pl->ctx, cudaEventSynchronize (pl->snap_ev), "wait snapshot");
-  if (pl->snap_err && *pl->snap_err)
-    return fail (pl->ctx, DSPSR_B200_ESTATE, "a device-side wait timed out");
-  return DSPSR_B200_OK;
+  return pl->conv.waits.set () ? wait_failed (pl->ctx) : DSPSR_B200_OK;
+}
+
+int dspsr_b200_pipeline_status_word (dspsr_b200_pipeline* pl, int** word)
+{
+  if (!pl) return DSPSR_B200_EINVAL;
+  return dspsr_b200_convolution_status_word (&pl->conv, word);
 }
 
 int dspsr_b200_pipeline_set_unloader (dspsr_b200_pipeline* pl, dspsr_b200_unload_fn fn,

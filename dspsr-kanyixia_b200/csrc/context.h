@@ -4,7 +4,18 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
+#include <mutex>
 #include <string>
+#include <vector>
+
+// Status words of the convolutions made on a context (WaitFlag in capi.cu);
+// shared with them, since an engine may outlive its context
+struct dspsr_b200_wait_words
+{
+  std::mutex lock;
+  std::vector<const volatile int*> words;
+};
 
 struct dspsr_b200_context
 {
@@ -14,6 +25,7 @@ struct dspsr_b200_context
   float* d_lut = nullptr;     // scratch LUT for the standalone unpacker
   float2* d_fb_tab = nullptr; // pass tables of the standalone filterbank's FFT
   unsigned fb_tab_n = 0;      // ... for this transform length
+  std::shared_ptr<dspsr_b200_wait_words> waits = std::make_shared<dspsr_b200_wait_words> ();
 };
 
 struct dspsr_b200_rfi_proposer;

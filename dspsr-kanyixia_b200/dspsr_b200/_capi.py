@@ -202,6 +202,7 @@ SIGNATURES = {
                                                         c_int, c_int, c_uint]),
     "dspsr_b200_convolution_get_response": (c_int, [c_vp, c_fp]),
     "dspsr_b200_convolution_status": (c_int, [c_vp]),
+    "dspsr_b200_convolution_status_word": (c_int, [c_vp, ctypes.POINTER(ctypes.POINTER(c_int))]),
     "dspsr_b200_convolution_set_temporal_apodization": (c_int, [c_vp, c_fp]),
     "dspsr_b200_convolution_set_fft_precision": (c_int, [c_vp, c_int]),
     "dspsr_b200_convolution_perform_noalloc": (c_int, [c_vp, c_vp, c_u64, c_u64, c_uint, c_uint,
@@ -288,6 +289,7 @@ SIGNATURES = {
     "dspsr_b200_pipeline_get_profiles": (c_int, [c_vp, c_fp, c_u32p]),
     "dspsr_b200_pipeline_get_profiles_async": (c_int, [c_vp, c_fp, ctypes.POINTER(ctypes.c_uint32)]),
     "dspsr_b200_pipeline_wait_profiles": (c_int, [c_vp]),
+    "dspsr_b200_pipeline_status_word": (c_int, [c_vp, ctypes.POINTER(ctypes.POINTER(c_int))]),
     "dspsr_b200_pipeline_reset": (c_int, [c_vp]),
     "dspsr_b200_pipeline_info": (c_int, [c_vp, c_u64p]),
     "dspsr_b200_pipeline_profile": (c_int, [c_vp, c_int]),

@@ -81,7 +81,9 @@ int dspsr_b200_context_create (int device, void* stream, dspsr_b200_context** ct
 int dspsr_b200_context_destroy (dspsr_b200_context* ctx);
 int dspsr_b200_context_set_stream (dspsr_b200_context* ctx, void* stream);
 const char* dspsr_b200_last_error (const dspsr_b200_context* ctx);
-/* blocks until all work queued on the context's stream is done */
+/* blocks until all work queued on the context's stream is done; DSPSR_B200_ESTATE
+   when a device-side wait of a convolution made on the context has given up
+   (dspsr_b200_convolution_status) */
 int dspsr_b200_synchronize (dspsr_b200_context* ctx);
 
 /* ---------------------------------------------------------------------- */
@@ -240,10 +242,17 @@ int dspsr_b200_convolution_perform_noalloc (void* stream, const float* d_in, uin
                                             float* d_out, uint64_t out_span, uint64_t* npart,
                                             int* d_status);
 /* Blocks until the engine's queued work is done and returns DSPSR_B200_ESTATE
-   if one of its device-side waits gave up (the tensor-core rows' mbarrier
-   waits, each bounded to about a second; the FP32 kernels have none),
-   DSPSR_B200_OK otherwise. */
+   if one of its device-side waits gave up, after about a second: the waits for
+   the bulk copies of the 4096-point FP32 rows (the default for nfft from 16384
+   to 131072) and for the tensor-core rows' products.  The output is not valid
+   then, and the status stays.  dspsr_b200_synchronize, dspsr_b200_fold_get_profiles
+   and the pipeline's calls that hand out profiles or sub-integrations report it
+   too; a caller that takes perform's output behind a synchronisation of its own
+   asks here, or reads the status word. */
 int dspsr_b200_convolution_status (dspsr_b200_convolution* conv);
+/* The engine's status word, in host memory: 0, or 1 once a wait has given up.
+   It may be read at any time, without waiting, until the engine is destroyed. */
+int dspsr_b200_convolution_status_word (dspsr_b200_convolution* conv, int** word);
 /* copies the response (FFT order) back to host memory, nchan*nfft complex */
 int dspsr_b200_convolution_get_response (dspsr_b200_convolution* conv, float* response);
 /* Convolution::set_temporal_apodization (Convolution.C:144-147, 222-250,
@@ -603,7 +612,8 @@ int dspsr_b200_fold_fold (dspsr_b200_fold* fold, const float* d_in, uint64_t in_
 /* writes the per-sample bin indices of the current plan (for parity checks) */
 int dspsr_b200_fold_binplan (dspsr_b200_fold* fold, uint32_t* d_binplan);
 /* Engine::synch(PhaseSeries*): profiles [chan][pol][bin] floats and hits[bin]
-   into host memory */
+   into host memory; DSPSR_B200_ESTATE (with the arrays filled) when a device-side
+   wait of a convolution on the same context has given up */
 int dspsr_b200_fold_get_profiles (dspsr_b200_fold* fold, float* profiles, uint32_t* hits);
 int dspsr_b200_fold_reset (dspsr_b200_fold* fold);
 
@@ -711,7 +721,9 @@ int dspsr_b200_pipeline_run (dspsr_b200_pipeline* pipe, const void* d_in, uint64
    stream (pinned host memory gives an asynchronous copy). */
 int dspsr_b200_pipeline_run_host (dspsr_b200_pipeline* pipe, const void* h_in,
                                   uint64_t ndat, uint64_t* ndat_folded);
-/* profiles [chan][nout][nbin] and hits[nbin] into host memory */
+/* profiles [chan][nout][nbin] and hits[nbin] into host memory;
+   DSPSR_B200_ESTATE (with the arrays filled) when a device-side wait has given
+   up (dspsr_b200_convolution_status) */
 int dspsr_b200_pipeline_get_profiles (dspsr_b200_pipeline* pipe, float* profiles,
                                       uint32_t* hits);
 /* The same without waiting (PhaseSeries read back while the next block is
@@ -723,6 +735,8 @@ int dspsr_b200_pipeline_get_profiles (dspsr_b200_pipeline* pipe, float* profiles
 int dspsr_b200_pipeline_get_profiles_async (dspsr_b200_pipeline* pipe, float* profiles,
                                             uint32_t* hits);
 int dspsr_b200_pipeline_wait_profiles (dspsr_b200_pipeline* pipe);
+/* the pipeline's status word (dspsr_b200_convolution_status_word) */
+int dspsr_b200_pipeline_status_word (dspsr_b200_pipeline* pipe, int** word);
 int dspsr_b200_pipeline_reset (dspsr_b200_pipeline* pipe);
 /* Per-kernel timing: when enabled, CUDA events are recorded on the context's
    stream around every kernel of the convolution path (column pass, row pass,
@@ -795,7 +809,10 @@ typedef struct
    for the call.  A closed division's copy to the host is queued behind the
    block's kernels and its callback runs in the first later _run, _run_host,
    _run_dada, _set_unloader, _reset or _finish call that finds the copy done;
-   _finish delivers all that remain. */
+   _finish delivers all that remain.  When a device-side wait has given up
+   (dspsr_b200_convolution_status) that call returns DSPSR_B200_ESTATE instead
+   and the waiting sub-integrations are dropped; _pop_subint then returns
+   DSPSR_B200_ESTATE with its arrays filled. */
 typedef void (*dspsr_b200_unload_fn) (void* user, const dspsr_b200_subint* subint,
                                       const float* profiles, const uint32_t* hits);
 int dspsr_b200_pipeline_set_unloader (dspsr_b200_pipeline* pipe, dspsr_b200_unload_fn fn,

@@ -117,6 +117,28 @@ int main ()
     std::vector<float> prof;
     std::vector<uint32_t> hits;
     fold.synch (prof, hits);
+    // a device-side wait of the convolution that gave up stops every call that
+    // hands out results
+    conv.status ();
+    *conv.status_word () = 1;
+    std::vector<float> lost_prof;
+    std::vector<uint32_t> lost_hits;
+    for (int call = 0; call < 3; call++)
+    {
+      bool thrown = false;
+      try
+      {
+        if (call == 0) conv.status ();
+        if (call == 1) ctx.synchronize ();
+        if (call == 2) fold.synch (lost_prof, lost_hits);
+      }
+      catch (b200::Error& e)
+      {
+        thrown = e.code == DSPSR_B200_ESTATE;
+      }
+      CHECK (thrown, "a timed-out wait went unnoticed by call %d", call);
+    }
+    *conv.status_word () = 0;
     std::vector<double> rprof (nbin, 0.0);
     std::vector<uint32_t> rhits (nbin, 0);
     double ph = phi;
