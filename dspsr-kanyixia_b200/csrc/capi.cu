@@ -204,17 +204,37 @@ struct dspsr_b200_convolution
 
   int set_fft_precision (int mode);
 
-  uint64_t budget = 0;        // scratch bytes (parts in flight)
   bool row_fixed = false;     // the caller named the row length
+
+  // A four-step split: its tables, its copy of the response and its batch.
+  // The one in use lies in shape, tw2, tw4, H and max_batch.  An engine whose
+  // arithmetic has been changed keeps the other one here, with its response up
+  // to date: no buffer of either moves or changes its meaning, so that work
+  // captured in a graph before the change stays valid.  The scratch is shared.
+  struct Split
+  {
+    unsigned n1 = 0, n2 = 0, max_batch = 1;
+    DevBuf<float2> tw2, tw4, H;
+    void release ()
+    {
+      tw2.release ();
+      tw4.release ();
+      H.release ();
+    }
+  } other;
 
   // row_len: the four-step row length, 4096 (nfft from 8192 to 131072: then
   // n1 = nfft / 4096 columns), 8192, or 0 for default_row_length
   int init (dspsr_b200_context* c, unsigned nchan, unsigned npol, unsigned nfft,
             unsigned pos, unsigned neg, uint64_t scratch_bytes, unsigned row_len = 0);
-  // n1, n2, their tables, the batch and its scratch
-  int split (unsigned row_len);
-  // changes the row length of an engine in use (its response follows)
-  int resplit (unsigned row_len);
+  // the split of a row length, for batches of at most bmax parts
+  int make_split (Split& s, unsigned row_len, uint64_t bmax);
+  // exchanges the split in use and the other
+  void swap_split ();
+  // changes the row length of an engine in use
+  int use_row_length (unsigned row_len);
+  // copies the response of the split in use to the other split
+  int response_to_other ();
   ConvTables tables () const
   {
     ConvTables t;
@@ -231,6 +251,7 @@ struct dspsr_b200_convolution
   }
   void release ()
   {
+    other.release ();
     tc_dft.release ();
     apod.release ();
     tw2.release ();
@@ -278,87 +299,107 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
   row_fixed = row_len != 0;
   // (1 GiB against 512 MiB: fewer, longer launches -- C1 0.636 against 0.663 ms
   // a block, C2 3.29 against 3.35)
-  budget = scratch_bytes ? scratch_bytes : (uint64_t (1) << 30);
-  const int rc = split (row_len ? row_len : default_row_length (nfft));
+  const uint64_t budget = scratch_bytes ? scratch_bytes : (uint64_t (1) << 30);
+  const uint64_t per_part = uint64_t (nchan) * npol * nfft;
+  const int rc = make_split (other, row_len ? row_len : default_row_length (nfft),
+                             budget / (per_part * sizeof (float2)));
   if (rc) return rc;
-  B200_CHECK (ctx, H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
+  swap_split ();
+  if (shape.n1 > 1) B200_CHECK (ctx, scratch.reserve (max_batch * per_part), "cudaMalloc scratch");
   B200_CHECK (ctx, lut.reserve (256), "cudaMalloc lut");
   B200_CHECK (ctx, waits.create (ctx), "status word");
   return DSPSR_B200_OK;
 }
 
-int dspsr_b200_convolution::split (unsigned row_len)
+int dspsr_b200_convolution::make_split (Split& s, unsigned row_len, uint64_t bmax)
 {
   const unsigned nfft = shape.nfft, nchan = shape.nchan, npol = shape.npol;
   if (row_len == 4096 && nfft >= 8192)
   {
-    shape.n2 = 4096;
-    shape.n1 = nfft / 4096;
+    s.n2 = 4096;
+    s.n1 = nfft / 4096;
   }
   else if (nfft <= 8192)
   {
-    shape.n1 = 1;
-    shape.n2 = nfft;
+    s.n1 = 1;
+    s.n2 = nfft;
   }
   else
   {
-    shape.n2 = 8192;
-    shape.n1 = nfft / 8192;
+    s.n2 = 8192;
+    s.n1 = nfft / 8192;
   }
-  B200_CHECK (ctx, tw2.reserve (shape.n2), "cudaMalloc tw2");
-  std::vector<float2> t2 = make_tw2 (shape.n2);
-  B200_CHECK (ctx, cudaMemcpy (tw2.ptr, t2.data (), t2.size () * sizeof (float2),
+  B200_CHECK (ctx, s.tw2.reserve (s.n2), "cudaMalloc tw2");
+  std::vector<float2> t2 = make_tw2 (s.n2);
+  B200_CHECK (ctx, cudaMemcpy (s.tw2.ptr, t2.data (), t2.size () * sizeof (float2),
                                cudaMemcpyHostToDevice), "copy tw2");
-  if (shape.n1 > 1)
+  B200_CHECK (ctx, s.H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
+  if (s.n1 > 1)
   {
-    B200_CHECK (ctx, tw4.reserve (nfft), "cudaMalloc tw4");
-    std::vector<float2> t4 = make_tw4 (shape.n1, shape.n2);
-    B200_CHECK (ctx, cudaMemcpy (tw4.ptr, t4.data (), t4.size () * sizeof (float2),
+    B200_CHECK (ctx, s.tw4.reserve (nfft), "cudaMalloc tw4");
+    std::vector<float2> t4 = make_tw4 (s.n1, s.n2);
+    B200_CHECK (ctx, cudaMemcpy (s.tw4.ptr, t4.data (), t4.size () * sizeof (float2),
                                  cudaMemcpyHostToDevice), "copy tw4");
     int dev = 0;
     B200_CHECK (ctx, cudaGetDevice (&dev), "cudaGetDevice");
     B200_CHECK (ctx, cudaDeviceGetAttribute (&nsm, cudaDevAttrMultiProcessorCount, dev),
                 "multiprocessor count");
-    // Parts in flight: the scratch stays near the L2 size unless told
-    // otherwise, and the batch is chosen so that its rows spread evenly over
-    // the persistent row kernel's CTAs.
-    const uint64_t per_part = uint64_t (nchan) * npol * nfft * sizeof (float2);
-    const uint64_t bmax = std::max<uint64_t> (1, std::min<uint64_t> (65535, budget / per_part));
-    const uint64_t rows_per_part = uint64_t (shape.n1) * nchan * npol;
+    // Parts in flight: as many as the scratch may hold, the batch chosen so
+    // that its rows spread evenly over the persistent row kernel's CTAs.
+    bmax = std::max<uint64_t> (1, std::min<uint64_t> (65535, bmax));
+    const uint64_t rows_per_part = uint64_t (s.n1) * nchan * npol;
     // (a multiple of the SM count, so also even for the tensor-core rows'
     // one CTA per SM)
-    const uint64_t ctas = uint64_t (nsm) * b200::rows_ctas_per_sm (shape.n2);
-    max_batch = unsigned (bmax);
+    const uint64_t ctas = uint64_t (nsm) * b200::rows_ctas_per_sm (s.n2);
+    s.max_batch = unsigned (bmax);
     for (uint64_t b = bmax; b >= std::max<uint64_t> (1, bmax / 2); b--)
       if ((b * rows_per_part) % ctas == 0)
       {
-        max_batch = unsigned (b);
+        s.max_batch = unsigned (b);
         break;
       }
-    B200_CHECK (ctx, scratch.reserve (uint64_t (max_batch) * nchan * npol * nfft),
-                "cudaMalloc scratch");
   }
   else
-    max_batch = 65535;
+    s.max_batch = 65535;
   return DSPSR_B200_OK;
 }
 
-int dspsr_b200_convolution::resplit (unsigned row_len)
+void dspsr_b200_convolution::swap_split ()
+{
+  std::swap (shape.n1, other.n1);
+  std::swap (shape.n2, other.n2);
+  std::swap (max_batch, other.max_batch);
+  std::swap (tw2, other.tw2);
+  std::swap (tw4, other.tw4);
+  std::swap (H, other.H);
+}
+
+int dspsr_b200_convolution::response_to_other ()
+{
+  B200_CHECK (ctx, tmp.reserve (uint64_t (shape.nchan) * shape.nfft), "cudaMalloc response staging");
+  B200_CHECK (ctx, launch_unpermute_response (tmp.ptr, H.ptr, shape.nchan, shape.n1, shape.n2,
+                                              ctx->stream), "unpermute response");
+  B200_CHECK (ctx, launch_permute_response (other.H.ptr, tmp.ptr, shape.nchan, other.n1, other.n2,
+                                            ctx->stream), "permute response");
+  return DSPSR_B200_OK;
+}
+
+int dspsr_b200_convolution::use_row_length (unsigned row_len)
 {
   if (shape.n1 < 2 || shape.n2 == row_len) return DSPSR_B200_OK;
-  const uint64_t n = uint64_t (shape.nchan) * shape.nfft;
-  if (have_response)
+  if (!other.n2)
   {
-    B200_CHECK (ctx, tmp.reserve (n), "cudaMalloc response staging");
-    B200_CHECK (ctx, launch_unpermute_response (tmp.ptr, H.ptr, shape.nchan, shape.n1, shape.n2,
-                                                ctx->stream), "unpermute response");
+    // the batch that the scratch in place holds (one part at least)
+    int rc = make_split (other, row_len, scratch.n / (uint64_t (shape.nchan) * shape.npol * shape.nfft));
+    if (!rc && have_response) rc = response_to_other ();
+    if (rc)
+    {
+      other.release ();
+      other.n1 = other.n2 = 0;
+      return rc;
+    }
   }
-  B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "sync before the new split");
-  const int rc = split (row_len);
-  if (rc) return rc;
-  if (have_response)
-    B200_CHECK (ctx, launch_permute_response (H.ptr, tmp.ptr, shape.nchan, shape.n1, shape.n2,
-                                              ctx->stream), "permute response");
+  swap_split ();
   return DSPSR_B200_OK;
 }
 
@@ -396,6 +437,11 @@ int build_response (dspsr_b200_convolution* c, const double* freq, double bw, do
                                        sh.nfft, sh.n1, sh.n2, binwidth, 0.5 * chanwidth,
                                        swap_halves, chirp_mode, scale, ctx->stream),
               "build chirp");
+  if (c->other.n2)
+  {
+    const int rc = c->response_to_other ();
+    if (rc) return rc;
+  }
   B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "set_dedispersion sync");
   c->have_response = true;
   return DSPSR_B200_OK;
@@ -2607,6 +2653,11 @@ int dspsr_b200_convolution_copy_response (dspsr_b200_convolution* c, const float
                                     cudaMemcpyHostToDevice, ctx->stream), "upload response");
   B200_CHECK (ctx, launch_permute_response (c->H.ptr, c->tmp.ptr, sh.nchan, sh.n1, sh.n2,
                                             ctx->stream), "permute response");
+  if (c->other.n2)
+  {
+    const int rc = c->response_to_other ();
+    if (rc) return rc;
+  }
   B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "copy_response sync");
   c->have_response = true;
   return DSPSR_B200_OK;
@@ -2701,15 +2752,12 @@ int dspsr_b200_convolution::set_fft_precision (int mode)
     return fail (ctx, DSPSR_B200_EINVAL, "fft precision: unknown mode %d", mode);
   if (mode == DSPSR_B200_FFT_FP32)
   {
-    tc_splits = 0;
-    return row_fixed ? DSPSR_B200_OK : resplit (default_row_length (shape.nfft));
+    const int rc = row_fixed ? DSPSR_B200_OK : use_row_length (default_row_length (shape.nfft));
+    if (!rc) tc_splits = 0;
+    return rc;
   }
-  if (!row_fixed && shape.nfft >= 16384)      // the tensor-core rows are 8192 points long
-  {
-    const int rc = resplit (8192);
-    if (rc) return rc;
-  }
-  if (shape.n1 < 2 || shape.n2 != 8192)
+  // the tensor-core rows are 8192 points long
+  if (shape.nfft < 16384 || (row_fixed && shape.n2 != 8192))
     return fail (ctx, DSPSR_B200_EINVAL,
                  "fft precision: the tensor-core rows need nfft >= 16384 (nfft=%u)", shape.nfft);
   const unsigned ns = mode == DSPSR_B200_FFT_BF16X2 ? 2 : 3;
@@ -2719,8 +2767,9 @@ int dspsr_b200_convolution::set_fft_precision (int mode)
   B200_CHECK (ctx, tc_dft.reserve (img.size ()), "cudaMalloc DFT operands");
   B200_CHECK (ctx, cudaMemcpy (tc_dft.ptr, img.data (), img.size (), cudaMemcpyHostToDevice),
               "copy DFT operands");
-  tc_splits = int (ns);
-  return DSPSR_B200_OK;
+  const int rc = use_row_length (8192);
+  if (!rc) tc_splits = int (ns);
+  return rc;
 }
 
 int dspsr_b200_convolution_set_fft_precision (dspsr_b200_convolution* c, int mode)
@@ -2968,8 +3017,11 @@ int dspsr_b200_pipeline_create (dspsr_b200_context* ctx, const dspsr_b200_pipeli
   // channels the convolution sees
   const unsigned nchan = fb ? cfg->nchan * fb : cfg->nchan;
   pl->rate = std::fabs (cfg->bandwidth_mhz) / double (nchan) * 1e6;
+  // (a pipeline's arithmetic does not change: the tensor-core rows' split at once)
+  const unsigned row_length = !cfg->row_length && cfg->fft_precision != DSPSR_B200_FFT_FP32
+                            ? 8192 : cfg->row_length;
   int rc = pl->conv.init (ctx, nchan, cfg->npol, cfg->nfft, cfg->nfilt_pos, cfg->nfilt_neg,
-                          cfg->scratch_bytes, cfg->row_length);
+                          cfg->scratch_bytes, row_length);
   if (!rc && cfg->fft_precision != DSPSR_B200_FFT_FP32)
     rc = pl->conv.set_fft_precision (cfg->fft_precision);
   if (!rc && cfg->interchannel)

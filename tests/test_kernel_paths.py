@@ -236,6 +236,58 @@ def test_rows_change_with_the_arithmetic(ctx, b2, orc):
     c.close()
 
 
+def test_captured_calls_survive_a_change_of_the_arithmetic(b2, orc):
+    """Graphs captured with one row length replay rightly after the engine has
+    changed to the other, also with a response set in between."""
+    nfft, pos, neg = 1 << 15, 700, 900
+    rng = np.random.default_rng(8)
+    h = np.exp(2j * np.pi * rng.random((2, 1, nfft))).astype(np.complex64) / np.float32(np.sqrt(nfft))
+    nk = nfft - pos - neg
+    ndat = nfft + 40 * nk
+    x = (rng.standard_normal((1, 2, ndat)) + 1j * rng.standard_normal((1, 2, ndat))).astype(np.complex64)
+    ref = [orc.convolve(x.astype(np.complex128), r.astype(np.complex128), nfft, pos, neg) for r in h]
+    st = torch.cuda.Stream()
+    ctx = b2.Context(0, st.cuda_stream)
+    c = b2.Convolution(ctx, 1, 2, nfft, pos, neg)
+    c.copy_response(h[0])
+    d = torch.from_numpy(x.view(np.float32)).cuda()
+    out = torch.zeros((1, 2, 41 * nk), dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+
+    def perform():
+        assert c.perform(d, ndat, ndat, out, 41 * nk) == 41
+
+    def check(what, r):
+        out.zero_()
+        torch.cuda.synchronize()
+        what()
+        torch.cuda.synchronize()
+        assert rel_rms(out.cpu().numpy(), ref[r]) < VOLTAGE_RTOL
+
+    graphs = []
+    for mode in (b2.FFT_FP32, b2.FFT_BF16X3):
+        c.set_fft_precision(mode)
+        check(perform, 0)                  # and what a first call sets up
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            perform()
+        graphs.append(g)
+    for g in graphs:
+        check(g.replay, 0)
+    c.copy_response(h[1])
+    for g in graphs:
+        check(g.replay, 1)
+    c.set_fft_precision(b2.FFT_FP32)
+    check(perform, 1)
+    for g in graphs:
+        check(g.replay, 1)
+    assert np.array_equal(c.get_response(), h[1])
+    c.status()
+    del graphs, g
+    c.close()
+    ctx.close()
+
+
 # spectral kurtosis: 8, 4, 2 and 1 blocks per thread block at the edges of the
 # shared tile, counts that leave the last one partly empty
 SK_EDGES = [(4, 2, 636, 9), (4, 2, 638, 9), (4, 2, 1276, 7), (4, 2, 1278, 7), (4, 2, 2556, 5),
