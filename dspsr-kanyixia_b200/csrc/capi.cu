@@ -224,7 +224,8 @@ struct dspsr_b200_convolution
   } other;
 
   // row_len: the four-step row length, 4096 (nfft from 8192 to 131072: then
-  // n1 = nfft / 4096 columns), 8192, or 0 for default_row_length
+  // n1 = nfft / 4096 columns), 8192, or 0 for default_row_length; scratch_bytes:
+  // the most that the parts in flight may take (one part always fits)
   int init (dspsr_b200_context* c, unsigned nchan, unsigned npol, unsigned nfft,
             unsigned pos, unsigned neg, uint64_t scratch_bytes, unsigned row_len = 0);
   // the split of a row length, for batches of at most bmax parts
@@ -297,12 +298,9 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
     return fail (ctx, DSPSR_B200_EINVAL,
                  "convolution: 4096-point rows need nfft <= 131072 (nfft=%u)", nfft);
   row_fixed = row_len != 0;
-  // (1 GiB against 512 MiB: fewer, longer launches -- C1 0.636 against 0.663 ms
-  // a block, C2 3.29 against 3.35)
-  const uint64_t budget = scratch_bytes ? scratch_bytes : (uint64_t (1) << 30);
   const uint64_t per_part = uint64_t (nchan) * npol * nfft;
   const int rc = make_split (other, row_len ? row_len : default_row_length (nfft),
-                             budget / (per_part * sizeof (float2)));
+                             scratch_bytes / (per_part * sizeof (float2)));
   if (rc) return rc;
   swap_split ();
   if (shape.n1 > 1) B200_CHECK (ctx, scratch.reserve (max_batch * per_part), "cudaMalloc scratch");
@@ -2609,7 +2607,7 @@ int dspsr_b200_convolution_create (dspsr_b200_context* ctx, unsigned nchan, unsi
   *out = nullptr;
   dspsr_b200_convolution* c = new (std::nothrow) dspsr_b200_convolution;
   if (!c) return fail (ctx, DSPSR_B200_ENOMEM, "convolution: out of host memory");
-  int rc = c->init (ctx, nchan, npol, nfft, pos, neg, 0);
+  int rc = c->init (ctx, nchan, npol, nfft, pos, neg, CONVOLUTION_SCRATCH);
   if (rc)
   {
     dspsr_b200_convolution_destroy (c);
@@ -3020,8 +3018,15 @@ int dspsr_b200_pipeline_create (dspsr_b200_context* ctx, const dspsr_b200_pipeli
   // (a pipeline's arithmetic does not change: the tensor-core rows' split at once)
   const unsigned row_length = !cfg->row_length && cfg->fft_precision != DSPSR_B200_FFT_FP32
                             ? 8192 : cfg->row_length;
+  uint64_t scratch = cfg->scratch_bytes;
+  if (!scratch)
+  {
+    size_t free_bytes = 0, total = 0;
+    cudaMemGetInfo (&free_bytes, &total);
+    scratch = pipeline_scratch (free_bytes);
+  }
   int rc = pl->conv.init (ctx, nchan, cfg->npol, cfg->nfft, cfg->nfilt_pos, cfg->nfilt_neg,
-                          cfg->scratch_bytes, row_length);
+                          scratch, row_length);
   if (!rc && cfg->fft_precision != DSPSR_B200_FFT_FP32)
     rc = pl->conv.set_fft_precision (cfg->fft_precision);
   if (!rc && cfg->interchannel)

@@ -21,6 +21,18 @@ struct FoldSegment
 };
 constexpr uint32_t FOLD_SKIP = 0xffffffffu;
 
+// Device scratch (FFT parts in flight) where the caller names no size.  A
+// pipeline takes 1 GiB -- fewer, longer launches: C1 0.636 against 0.663 ms a
+// block, C2 3.29 against 3.35 with 512 MiB -- while that is a sixteenth of the
+// free device memory or less, so that many pipelines, or others on the device,
+// keep room.  A convolution engine's caller has no way to ask for less and
+// gets CONVOLUTION_SCRATCH.
+constexpr uint64_t CONVOLUTION_SCRATCH = uint64_t (512) << 20;
+constexpr uint64_t pipeline_scratch (uint64_t free_bytes)
+{
+  return free_bytes / 16 >= 2 * CONVOLUTION_SCRATCH ? 2 * CONVOLUTION_SCRATCH : CONVOLUTION_SCRATCH;
+}
+
 unsigned smearing_samples (double centre_frequency, double bandwidth, double dm,
                            unsigned nchan, int half);
 unsigned minimum_ndat (unsigned impulse_pos, unsigned impulse_neg);

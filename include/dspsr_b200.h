@@ -184,7 +184,8 @@ int dspsr_b200_unpack16 (dspsr_b200_context* ctx, const void* d_in, uint64_t nda
 /* ---------------------------------------------------------------------- */
 
 /* Engine::prepare(Convolution*): sizes from Convolution::prepare
-   (Convolution.C:316-465).  nfft must be a power of two in [4096, 262144]. */
+   (Convolution.C:316-465).  nfft must be a power of two in [4096, 262144].
+   The parts in flight take up to 512 MiB of device memory. */
 int dspsr_b200_convolution_create (dspsr_b200_context* ctx, unsigned nchan,
                                    unsigned npol, unsigned nfft, unsigned nfilt_pos,
                                    unsigned nfilt_neg, dspsr_b200_convolution** conv);
@@ -649,7 +650,8 @@ typedef struct
   double reference_phase;
   int64_t epoch_day, epoch_sec; double epoch_frac;   /* reference epoch MJD */
   int64_t start_day, start_sec; double start_frac;   /* MJD of input sample 0 */
-  /* tuning: maximum scratch bytes for in-flight FFT parts (0 = default) */
+  /* tuning: maximum scratch bytes for in-flight FFT parts (0 = 1 GiB while
+     16 GiB of device memory are free, else 512 MiB) */
   uint64_t scratch_bytes;
   /* FFT filterbank stage in front of the dedispersion (Filterbank with
      freq_res = 1, Filterbank.C:75-570): channels per input channel, 0 or 1 =

@@ -2,7 +2,9 @@
 include/dspsr_b200.h declares, and its host rules (no GPU needed) agree with
 the oracle's restatement of the reference."""
 import ctypes
+import os
 import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -84,3 +86,33 @@ def test_context_without_gpu_reports_no_device(b2):
     with pytest.raises(b2.B200Error) as e:
         b2.Context(0)
     assert e.value.code == b2._capi.ENODEV
+
+
+def test_default_scratch_leaves_room(tmp_path):
+    """A pipeline's default scratch is 1 GiB only while 16 GiB are free."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = tmp_path / "scratch.cpp"
+    src.write_text("""
+#include "host_rules.h"
+constexpr uint64_t MiB = uint64_t (1) << 20;
+static_assert (b200::pipeline_scratch (178000 * MiB) == 1024 * MiB, "");
+static_assert (b200::pipeline_scratch (16384 * MiB) == 1024 * MiB, "");
+static_assert (b200::pipeline_scratch (16384 * MiB - 1) == 512 * MiB, "");
+static_assert (b200::pipeline_scratch (0) == 512 * MiB, "");
+static_assert (b200::CONVOLUTION_SCRATCH == 512 * MiB, "");
+""")
+    subprocess.run(["g++", "-std=c++17", "-fsyntax-only", "-I",
+                    os.path.join(root, "dspsr-kanyixia_b200", "csrc"), str(src)], check=True)
+
+
+@pytest.mark.gpu
+def test_engine_scratch_stays_within_its_default(ctx, b2):
+    """The engine cannot name a size: 512 MiB and the tables, no more."""
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    c = b2.Convolution(ctx, 1, 2, 1 << 17, 1000, 1000)
+    used = before - torch.cuda.mem_get_info()[0]
+    c.close()
+    # tables and response: 3 MiB, each allocation in steps of 2 MiB
+    assert used <= (512 + 16) << 20, used
