@@ -332,16 +332,16 @@ int dspsr_b200_convolution::make_split (Split& s, unsigned row_len, uint64_t bma
   B200_CHECK (ctx, cudaMemcpy (s.tw2.ptr, t2.data (), t2.size () * sizeof (float2),
                                cudaMemcpyHostToDevice), "copy tw2");
   B200_CHECK (ctx, s.H.reserve (uint64_t (nchan) * nfft), "cudaMalloc response");
+  int dev = 0;
+  B200_CHECK (ctx, cudaGetDevice (&dev), "cudaGetDevice");
+  B200_CHECK (ctx, cudaDeviceGetAttribute (&nsm, cudaDevAttrMultiProcessorCount, dev),
+              "multiprocessor count");
   if (s.n1 > 1)
   {
     B200_CHECK (ctx, s.tw4.reserve (nfft), "cudaMalloc tw4");
     std::vector<float2> t4 = make_tw4 (s.n1, s.n2);
     B200_CHECK (ctx, cudaMemcpy (s.tw4.ptr, t4.data (), t4.size () * sizeof (float2),
                                  cudaMemcpyHostToDevice), "copy tw4");
-    int dev = 0;
-    B200_CHECK (ctx, cudaGetDevice (&dev), "cudaGetDevice");
-    B200_CHECK (ctx, cudaDeviceGetAttribute (&nsm, cudaDevAttrMultiProcessorCount, dev),
-                "multiprocessor count");
     // Parts in flight: as many as the scratch may hold, the batch chosen so
     // that its rows spread evenly over the persistent row kernel's CTAs.
     bmax = std::max<uint64_t> (1, std::min<uint64_t> (65535, bmax));

@@ -198,11 +198,19 @@ k_inv_cols (const float2* __restrict__ scratch, const unsigned n2, const unsigne
 // single-kernel path (n1 == 1): everything in shared memory
 // --------------------------------------------------------------------------
 
-// Groups of T threads take one polarisation each, side by side where 512
-// threads hold them (a call of one or two parts waits for one block's chain of
-// passes: 31 us one after the other, 24 us side by side at 4096 points), one
-// after the other at 8192 points.
-template <int T> B200_CE int fused_groups (unsigned npol) { return 2 * T <= 512 ? npol : 1; }
+// Groups of T threads take one polarisation each, side by side or one after the
+// other.  Side by side (4096 points; 8192 do not fit 512 threads) a block is
+// done sooner but alone on its SM; one after the other two blocks share an SM
+// and overlap each other's barriers.  In blocks per SM, rounded up, and us
+// (voltages of two polarisations, one after the other / side by side): 1:
+// 28.6 / 24.5, 2: 36.9 / 40.9, 3: 61.4 / 57.3 (444 blocks of a fold: 105 / 91),
+// 4: 67.6 / 73.8, 27: 418 / 469.
+template <int T>
+constexpr unsigned fused_groups (unsigned npol, unsigned blocks, unsigned nsm)
+{
+  const unsigned per_sm = (blocks + nsm - 1) / nsm;
+  return 2 * T <= 512 && (per_sm == 1 || per_sm == 3) ? npol : 1;
+}
 
 template <int N, int T, int KIND, int MODE, int NOUT>
 __global__ void __launch_bounds__ (512, 1)
@@ -412,7 +420,8 @@ cudaError_t run_fused_t (const ConvShape& sh, const ConvTables& tb, const InputV
   cudaError_t err = fused_setup<N, KIND, MODE, NOUT> ();
   if (err != cudaSuccess) return err;
   ClockScope cs (clk, KK_FUSED, st);
-  kern<<<dim3 (nbatch, sh.nchan), T * fused_groups<T> (in.npol), smem, st>>> (
+  const unsigned groups = fused_groups<T> (in.npol, nbatch * sh.nchan, unsigned (tb.nsm));
+  kern<<<dim3 (nbatch, sh.nchan), T * groups, smem, st>>> (
       in, tb.lut, tb.tw2, tb.H, sh.nkeep, sh.nfilt_pos, part0, fv, vv, tb.apod);
   return cudaGetLastError ();
 }

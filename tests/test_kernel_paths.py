@@ -213,6 +213,39 @@ def test_fold_runs_of_every_length(ctx, b2, orc, npol, nbin, per_bin):
     assert np.max(np.abs(prof - rprof)[..., hit] / rprof[..., hit]) < 1e-5
 
 
+@pytest.mark.parametrize("npol", [1, 2])
+def test_fused_4096_side_by_side_and_in_turn(ctx, b2, orc, npol):
+    """4096-point parts with one, two, three and five blocks per SM: the same
+    bits however many parts a call has, and right against 64 bits."""
+    nfft, pos, neg = 4096, 300, 211
+    nk = nfft - pos - neg
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    counts = [nsm // 2, 2 * nsm, 2 * nsm + 1, 4 * nsm + 1]
+    total = sum(counts)
+    ndat = total * nk + pos + neg
+    gen = torch.Generator(device="cuda").manual_seed(npol)
+    d = torch.randn((1, npol, ndat, 2), device="cuda", generator=gen)
+    rng = np.random.default_rng(npol)
+    h = np.exp(2j * np.pi * rng.random((1, nfft))).astype(np.complex64) / np.float32(np.sqrt(nfft))
+    c = b2.Convolution(ctx, 1, npol, nfft, pos, neg)
+    c.copy_response(h)
+    whole = torch.zeros((1, npol, total * nk, 2), device="cuda")
+    assert c.perform(d, ndat, ndat, whole, total * nk) == total
+    first = 0
+    for n in counts:
+        part = torch.zeros((1, npol, n * nk, 2), device="cuda")
+        piece = d[:, :, first * nk:first * nk + n * nk + pos + neg].contiguous()
+        assert c.perform(piece, piece.shape[2], piece.shape[2], part, n * nk) == n
+        ctx.synchronize()
+        assert torch.equal(part, whole[:, :, first * nk:(first + n) * nk])
+        first += n
+    c.close()
+    x = d[:, :, :3 * nk + pos + neg].cpu().numpy().astype(np.float64).view(np.complex128)[..., 0]
+    ref = orc.convolve(x, h.astype(np.complex128), nfft, pos, neg)
+    got = whole[:, :, :3 * nk].cpu().numpy().view(np.complex64)[..., 0]
+    assert rel_rms(got, ref) < VOLTAGE_RTOL
+
+
 def test_rows_change_with_the_arithmetic(ctx, b2, orc):
     """An engine with its default rows, then tensor-core rows, then FP32
     again: the response follows the split."""
