@@ -181,10 +181,16 @@ namespace {
 // The four-step row length when the caller names none: 4096-point rows
 // (k_rows64) where they leave columns of at most 32 points, whose passes run a
 // thread or two per column; 8192-point rows above, and the single-kernel
-// transforms below.  Blocks with either: 2^14 x 32 channels 0.357 against
-// 0.420 ms, 2^15 x 1024 (C5) 4.83 against 5.22, 2^16 x 64 (C2) 3.07 against
-// 3.27, 2^17 (C1) 0.620 against 0.655.
-unsigned default_row_length (unsigned nfft) { return nfft >= 16384 && nfft <= 131072 ? 4096 : 8192; }
+// transforms below.  One polarisation keeps the older column kernels, which
+// lose with columns of 16 and 32 what the rows gain: 8192-point rows from 2^16.
+// GPU time of a block (us, 4096 / 8192), 8 M samples, 8-bit, 1024 bins of 1000
+// samples: two polarisations 2^14 195 / 214, 2^15 191 / 224, 2^16 213 / 218,
+// 2^17 225 / 239; one 150 / 167, 166 / 167, 209 / 181, 213 / 222 (2^17 with 256
+// bins 332 / 250).
+unsigned default_row_length (unsigned nfft, unsigned npol)
+{
+  return nfft >= 16384 && nfft <= (npol == 2 ? 131072u : 32768u) ? 4096 : 8192;
+}
 
 } // namespace
 
@@ -299,7 +305,7 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
                  "convolution: 4096-point rows need nfft <= 131072 (nfft=%u)", nfft);
   row_fixed = row_len != 0;
   const uint64_t per_part = uint64_t (nchan) * npol * nfft;
-  const int rc = make_split (other, row_len ? row_len : default_row_length (nfft),
+  const int rc = make_split (other, row_len ? row_len : default_row_length (nfft, npol),
                              scratch_bytes / (per_part * sizeof (float2)));
   if (rc) return rc;
   swap_split ();
@@ -2750,7 +2756,7 @@ int dspsr_b200_convolution::set_fft_precision (int mode)
     return fail (ctx, DSPSR_B200_EINVAL, "fft precision: unknown mode %d", mode);
   if (mode == DSPSR_B200_FFT_FP32)
   {
-    const int rc = row_fixed ? DSPSR_B200_OK : use_row_length (default_row_length (shape.nfft));
+    const int rc = row_fixed ? DSPSR_B200_OK : use_row_length (default_row_length (shape.nfft, shape.npol));
     if (!rc) tc_splits = 0;
     return rc;
   }

@@ -694,7 +694,8 @@ typedef struct
   float sk_std_devs;
   /* tuning: the four-step split's row length, 8192 or 4096 (nfft from 8192 to
      131072, n1 = nfft / 4096 columns; the tensor-core rows need 8192); 0 =
-     4096 for FP32 rows and nfft from 16384 to 131072, else 8192 */
+     4096 for FP32 rows and nfft from 16384 to 131072 (one polarisation: to
+     32768), else 8192 */
   unsigned row_length;
 } dspsr_b200_pipeline_config;
 

@@ -67,6 +67,21 @@ def test_pipeline_paths_match_oracle(ctx, b2, orc, path):
     check(prof, hits, total, rprof, rhits, rtotal, cfg["state"])
 
 
+@pytest.mark.parametrize("npol", [1, 2])
+def test_default_row_lengths(ctx, b2, npol):
+    """The split of each transform length when the caller names no row length."""
+    most = (1 << 15) if npol == 1 else 1 << 17
+    for lg in range(13, 19):
+        nfft = 1 << lg
+        want = 4096 if 1 << 14 <= nfft <= most else 8192
+        for row, n2 in ((0, want), (8192, 8192)):
+            pl = b2.Pipeline(ctx, b2.make_config(1400.0, 16.0, 0.1, 1, npol, nfft, 10, 10, 64, 0.01,
+                                                 row_length=row))
+            info = pl.info()
+            pl.close()
+            assert (info["n1"], info["n2"]) == (nfft // n2, n2), (nfft, row)
+
+
 @pytest.mark.parametrize("nfft,kind", [(1 << 14, "i8"), (1 << 17, "i8"), (1 << 18, "i16")])
 def test_one_polarisation_matches_oracle(ctx, b2, orc, nfft, kind):
     cfg = path_cfg(b2, nfft, 0, 1, kind, b2.INTENSITY, 128, 50.0, npol=1)
