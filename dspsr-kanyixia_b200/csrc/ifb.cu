@@ -208,8 +208,9 @@ k_ifb_stitch (const InputView in, const IfbShape sh, const IfbTables tb, const u
   if (c < sh.nin) stitch_out<LIN, TF> (s, sh, tb, scratch, b, c, p, tid);
 }
 
-// The same for LIN = 128 .. 1024 with 32 points per thread (FbWarp's split
-// LIN = 32 x M: one exchange, warp barriers only).  A block takes
+// The same for LIN = 256 .. 1024 with 32 points per thread (FbWarp's split
+// LIN = 32 x M: one exchange, warp barriers only), where ifb_stitch_by_warps
+// chooses it.  A block takes
 // 8 * (32 / M) slots; TFPD samples are loaded in address order (all slots of a
 // time sample together) and handed over as raw words in the slots' own
 // regions, whose stride of 4 mod 32 words keeps both sides free of bank
@@ -392,23 +393,36 @@ void launch_ifb_stitch_warp (const IfbShape& sh, const IfbTables& tb, const Inpu
                                                                                 scratch);
 }
 
-// 128- to 1024-point transforms fit a warp with 32 points per thread
-template <int LIN>
-void launch_ifb_stitch_w (const IfbShape& sh, const IfbTables& tb, const InputView& in,
-                          uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
+// Whether the transforms of lin points run 32 points per thread.  That spends
+// less on the transform and shared memory, but leaves half the threads to place
+// the bins: a response or a spectral window, loaded bin by bin, then costs more
+// than the transform gains, except for float samples, and so do 128-point
+// transforms, which make the most slots.  Calls of 64 M samples, 16 points per
+// thread / 32 (us): 1024 x 256 int16 1322 / 1218, with a response 1478 / 1433;
+// 1024 x 64 int16, one polarisation 634 / 626, with a response 656 / 683;
+// 256 x 128 int16 640 / 632, with a response 648 / 712, int8 1276 / 1307;
+// 128 x 256 float 655 / 683.
+bool ifb_stitch_by_warps (unsigned lin, int kind, bool windows)
 {
-  if (in.kind == IN_INT8)
-    launch_ifb_stitch_warp<LIN, IN_INT8> (sh, tb, in, part0, nbatch, scratch, st);
-  else if (in.kind == IN_INT16)
-    launch_ifb_stitch_warp<LIN, IN_INT16> (sh, tb, in, part0, nbatch, scratch, st);
-  else
-    launch_ifb_stitch_warp<LIN, IN_FLOAT> (sh, tb, in, part0, nbatch, scratch, st);
+  if (lin == 256) return kind != IN_INT8 && !windows;
+  return (lin == 512 || lin == 1024) && (kind == IN_FLOAT || !windows);
 }
 
 template <int LIN>
 void launch_ifb_stitch_k (const IfbShape& sh, const IfbTables& tb, const InputView& in,
                           uint64_t part0, unsigned nbatch, float2* scratch, cudaStream_t st)
 {
+  if constexpr (LIN >= 256 && LIN <= 1024)
+    if (ifb_stitch_by_warps (LIN, in.kind, tb.response || tb.spectral))
+    {
+      if (in.kind == IN_INT16)
+        launch_ifb_stitch_warp<LIN, IN_INT16> (sh, tb, in, part0, nbatch, scratch, st);
+      else if (in.kind == IN_FLOAT)
+        launch_ifb_stitch_warp<LIN, IN_FLOAT> (sh, tb, in, part0, nbatch, scratch, st);
+      else if constexpr (LIN >= 512)
+        launch_ifb_stitch_warp<LIN, IN_INT8> (sh, tb, in, part0, nbatch, scratch, st);
+      return;
+    }
   if (in.kind == IN_INT8)
     launch_ifb_stitch<LIN, IN_INT8> (sh, tb, in, part0, nbatch, scratch, st);
   else if (in.kind == IN_INT16)
@@ -464,10 +478,10 @@ cudaError_t launch_inverse_filterbank (const IfbShape& sh, const IfbTables& tb,
     switch (sh.lin)
     {
       case 64: launch_ifb_stitch_k<64> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 128: launch_ifb_stitch_w<128> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 256: launch_ifb_stitch_w<256> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 512: launch_ifb_stitch_w<512> (sh, tb, in, part0, nbatch, scratch, st); break;
-      case 1024: launch_ifb_stitch_w<1024> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 128: launch_ifb_stitch_k<128> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 256: launch_ifb_stitch_k<256> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 512: launch_ifb_stitch_k<512> (sh, tb, in, part0, nbatch, scratch, st); break;
+      case 1024: launch_ifb_stitch_k<1024> (sh, tb, in, part0, nbatch, scratch, st); break;
       case 2048: launch_ifb_stitch_k<2048> (sh, tb, in, part0, nbatch, scratch, st); break;
       case 4096: launch_ifb_stitch_k<4096> (sh, tb, in, part0, nbatch, scratch, st); break;
       default: return cudaErrorInvalidValue;

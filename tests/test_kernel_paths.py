@@ -207,6 +207,40 @@ def test_inverse_filterbank_sizes(ctx, b2, orc, lin, kind, npol):
     assert rel_rms(out.cpu().numpy().view(np.complex64)[..., 0], ref) < VOLTAGE_RTOL
 
 
+@pytest.mark.parametrize("lin,nin,npol", [(64, 512, 1), (128, 256, 2), (256, 128, 1), (512, 128, 2),
+                                          (1024, 256, 1), (1024, 64, 2), (2048, 16, 2)])
+@pytest.mark.parametrize("kind", ["i16", "f"])
+def test_inverse_filterbank_windows(ctx, b2, orc, lin, nin, npol, kind):
+    """Response and both windows, with rows of the stitched spectra shorter and
+    longer than the threads of a transform, both splits of the transforms."""
+    disc = nin * 3
+    rng = np.random.default_rng(lin + nin)
+    ifb = b2.InverseFilterbank(ctx, nin, 1, nin, npol, lin, os=(4, 3), output_discard=(disc, disc))
+    info = ifb.info
+    lout = info["lout"]
+    resp = (np.exp(2j * np.pi * rng.random((1, lout))) * rng.uniform(0.5, 1.5, (1, lout))).astype(np.complex64)
+    temporal = b2.apodization(b2.APOD_TUKEY, lin, info["in_discard_pos"], info["in_discard_neg"])
+    spectral = b2.apodization(b2.APOD_HANNING, lout, swap_halves=True)
+    ifb.copy_response(resp)
+    ifb.set_apodization(temporal, spectral)
+    ndat = 2 * info["in_step"] + info["in_discard_pos"] + info["in_discard_neg"]
+    raw = np.clip(np.round(rng.standard_normal((ndat, nin, npol, 2)) * 3000), -32768, 32767).astype(np.int16)
+    v = (raw + np.float32(0.5)).astype(np.float32)
+    x = np.ascontiguousarray(np.moveaxis(v, 0, 2)).view(np.complex64)[..., 0]
+    data = raw if kind == "i16" else x.view(np.float32)
+    cfg = dict(input_nchan=nin, output_nchan=1, pfb_nchan=nin, npol=npol, input_fft_length=lin,
+               os_num=4, os_den=3, output_discard_pos=disc, output_discard_neg=disc,
+               pfb_dc_chan=1, pfb_all_chan=1, dual_sideband=1)
+    ref = orc.inverse_filterbank(x, cfg, response=resp, temporal=temporal, spectral=spectral, fp64=True)
+    n = 2 * info["out_step"]
+    out = torch.zeros((1, npol, n, 2), device="cuda")
+    assert ifb.perform(torch.from_numpy(data).cuda(), ndat, out, n,
+                       input_kind=b2.INT16_TFPD if kind == "i16" else b2.FLOAT_FPT) == 2
+    ctx.synchronize()
+    assert rel_rms(out.cpu().numpy().view(np.complex64)[..., 0], ref) < VOLTAGE_RTOL
+    ifb.close()
+
+
 @pytest.mark.parametrize("npol,nbin,per_bin", [(1, 64, 700.0), (2, 500, 0.3), (3, 100, 9.0),
                                                (4, 128, 9.0), (4, 32, 3000.0), (5, 64, 1.0)])
 def test_fold_runs_of_every_length(ctx, b2, orc, npol, nbin, per_bin):
