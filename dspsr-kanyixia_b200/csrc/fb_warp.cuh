@@ -16,7 +16,8 @@ namespace {
 // block's 8 * (32 / M) consecutive output samples of one polarisation are
 // written together, so that every channel gets runs of 64 bytes and more.
 // Persistent blocks keep the twiddle table.  Bound by HBM (8 or fewer bytes
-// in, 8 out per value): 480 shared-memory clocks and 260 FP32 clocks per
+// in, 8 out per value; TFPD samples of many channels by the 32-byte sector that
+// each of them fetches from L2): 480 shared-memory clocks and 260 FP32 clocks per
 // 1024 points against 730 of copying.  16 points per thread in three passes
 // with block barriers took 1435 us for C5's block (134 M samples, 1024 channels,
 // float), this 1033 us,
@@ -69,8 +70,13 @@ k_filterbank_warp (const InputView in, const float* __restrict__ lut, const uint
   const uint64_t rowv = uint64_t (in.nchan) * npol;      // TFPD values per time sample
   for (uint64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x)
   {
-    const unsigned row = unsigned (tile / tiles_per_row);          // input channel * npol + pol
-    const uint64_t blk0 = tile % tiles_per_row * F::NB;
+    // input channel * npol + pol: outermost for FPT rows, innermost for TFPD
+    // samples, whose sectors hold several rows: blocks at work together then
+    // share them through L2 (32 dual-polarisation int8 channels into 512 each,
+    // 64 M values: 491 us, with the row outermost 768; into 128 each 668, 1350)
+    const uint64_t nrow = uint64_t (in.nchan) * npol;
+    const unsigned row = unsigned (KIND == IN_FLOAT ? tile / tiles_per_row : tile % nrow);
+    const uint64_t blk0 = (KIND == IN_FLOAT ? tile % tiles_per_row : tile / nrow) * F::NB;
     const bool live = blk0 + slot < nblk;
     const uint64_t t0 = (blk0 + slot) * NSUB + t;
     CP v[32];

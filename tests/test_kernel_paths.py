@@ -140,7 +140,8 @@ def test_fused_filterbank_row_lengths(ctx, b2, orc, row, kind):
 
 
 @pytest.mark.parametrize("nsub", [128, 256, 512, 1024, 2048])
-@pytest.mark.parametrize("kind,npol,nchan", [("f", 2, 2), ("i8", 2, 1), ("i16", 1, 3)])
+@pytest.mark.parametrize("kind,npol,nchan", [("f", 2, 2), ("i8", 2, 1), ("i16", 1, 3), ("i16", 2, 5),
+                                             ("i8", 1, 12)])
 def test_filterbank_sizes(ctx, b2, nsub, kind, npol, nchan):
     """Output lengths around a tile's, against a 64-bit FFT."""
     kinds = dict(i8=b2.INT8_TFPD, i16=b2.INT16_TFPD, f=b2.FLOAT_FPT)
