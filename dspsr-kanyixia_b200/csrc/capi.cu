@@ -312,6 +312,7 @@ int dspsr_b200_convolution::init (dspsr_b200_context* c, unsigned nchan, unsigne
   if (shape.n1 > 1) B200_CHECK (ctx, scratch.reserve (max_batch * per_part), "cudaMalloc scratch");
   B200_CHECK (ctx, lut.reserve (256), "cudaMalloc lut");
   B200_CHECK (ctx, waits.create (ctx), "status word");
+  B200_CHECK (ctx, convolution_kernel_setup (), "kernel set-up");
   return DSPSR_B200_OK;
 }
 
@@ -1593,6 +1594,7 @@ int dspsr_b200_inverse_filterbank::init (dspsr_b200_context* c, const dspsr_b200
   shape.out_step = lout - cfg.output_discard_pos - cfg.output_discard_neg;
   shape.out_discard_pos = cfg.output_discard_pos;
   shape.dual_sideband = cfg.dual_sideband;
+  B200_CHECK (ctx, inverse_filterbank_kernel_setup (), "kernel set-up");
   B200_CHECK (ctx, map.reserve (nin), "cudaMalloc stitch map");
   B200_CHECK (ctx, cudaMemcpy (map.ptr, m.data (), nin * sizeof (int4), cudaMemcpyHostToDevice),
               "copy stitch map");
@@ -1877,6 +1879,7 @@ int dspsr_b200_filterbank_during::init (dspsr_b200_context* c, const dspsr_b200_
   max_batch = unsigned (std::max<uint64_t> (1, std::min<uint64_t> (65535, budget / per_part)));
   B200_CHECK (ctx, scratch.reserve (uint64_t (max_batch) * s.nchan_in * s.npol * N),
               "cudaMalloc scratch");
+  B200_CHECK (ctx, during_kernel_setup (), "kernel set-up");
   B200_CHECK (ctx, H.reserve (uint64_t (s.nchan_in) * s.nsub * s.freq_res), "cudaMalloc response");
   return DSPSR_B200_OK;
 }

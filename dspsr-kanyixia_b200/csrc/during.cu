@@ -664,6 +664,13 @@ cudaError_t launch_window_response (float2* out, const float2* in, const float* 
   return cudaGetLastError ();
 }
 
+// (its kernels' shared-memory opt-in goes with each launch)
+cudaError_t during_kernel_setup ()
+{
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes (&a, k_window_response);
+}
+
 bool during_supported (unsigned nsub, unsigned freq_res)
 {
   if (nsub < 2 || nsub > 128 || (nsub & (nsub - 1))) return false;

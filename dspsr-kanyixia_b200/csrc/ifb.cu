@@ -456,6 +456,20 @@ bool ifb_supported_lin (unsigned lin)
          lin == 4096;
 }
 
+cudaError_t inverse_filterbank_kernel_setup ()
+{
+  static std::atomic<unsigned> done {0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice (&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned bit = dev < 32 ? 1u << dev : 0u;    // devices past 32: set every time
+  if (bit && (done.load () & bit)) return cudaSuccess;
+  e = set_rows_smem<8192, false> ();
+  if (e == cudaSuccess) e = set_rows_smem<4096, false> ();
+  if (e == cudaSuccess) done.fetch_or (bit);
+  return e;
+}
+
 cudaError_t launch_inverse_filterbank (const IfbShape& sh, const IfbTables& tb,
                                        const InputView& in, uint64_t part0, unsigned nbatch,
                                        float2* scratch, const VoltView& vv, cudaStream_t st,
@@ -463,15 +477,9 @@ cudaError_t launch_inverse_filterbank (const IfbShape& sh, const IfbTables& tb,
 {
   if (nbatch == 0) return cudaSuccess;
   if (sh.n2 != 8192 && sh.n2 != 4096) return cudaErrorInvalidValue;
-  static unsigned attr_done = 0;
-  int dev = 0;
-  cudaGetDevice (&dev);
-  if (dev < 32 && !(attr_done & (1u << dev)))
   {
-    cudaError_t e = set_rows_smem<8192, false> ();
-    if (e == cudaSuccess) e = set_rows_smem<4096, false> ();
+    const cudaError_t e = inverse_filterbank_kernel_setup ();
     if (e != cudaSuccess) return e;
-    attr_done |= 1u << dev;
   }
   {
     ClockScope cs (clk, KK_FWD_COLS, st);

@@ -168,8 +168,12 @@ cudaError_t launch_zeroed_fold (const float2* v, uint64_t span, uint64_t ndat, u
                                 const KernelClock* clock = nullptr);
 
 // Per-device set-up of the four-step convolution kernels (their shared-memory
-// opt-in) on the current device; launch_convolution calls it itself.
+// opt-in) on the current device; launch_convolution calls it itself.  An engine
+// calls its path's set-up when it is made, so that the first block does not
+// wait for the path's module to be loaded (20 to 30 ms).
 cudaError_t convolution_kernel_setup ();
+cudaError_t during_kernel_setup ();
+cudaError_t inverse_filterbank_kernel_setup ();
 
 // Runs parts [part0, part0 + nbatch) of one block.  scratch holds
 // nbatch*nchan*npol*nfft complex values (unused when n1 == 1).
