@@ -755,7 +755,7 @@ struct dspsr_b200_pipeline
   DevBuf<uint8_t> sk_pmask;
   DevBuf<float2> fbbuf;             // filterbank output, FPT
   DevBuf<uint8_t> aligned_in;       // a misaligned block of the fused filterbank, copied
-  float2* fb_tab = nullptr;         // pass tables of the filterbank FFT (fb_nsub >= 128)
+  float2* fb_tab = nullptr;         // pass tables of the filterbank FFT (filterbank_uses_tables)
   size_t fb_tab_cap = 0;
   // run_host folds a block in pieces: the first piece that folds starts the
   // block's phase with Fold::get_phase, later pieces go on with the block's
@@ -2720,7 +2720,7 @@ int dspsr_b200_filterbank (dspsr_b200_context* ctx, int input_kind, const void* 
   if (!is_pow2 (nsub) || nsub < 4 || nsub > 4096)
     return fail (ctx, DSPSR_B200_EINVAL, "filterbank: nsub=%u not a power of two in [4, 4096]",
                  nsub);
-  if (nsub >= 128 && ctx->fb_tab_n != nsub)
+  if (filterbank_uses_tables (nsub) && ctx->fb_tab_n != nsub)
   {
     size_t cap = ctx->fb_tab_n ? pass_tables_count (ctx->fb_tab_n) : 0;
     B200_CHECK (ctx, cudaStreamSynchronize (ctx->stream), "sync before table upload");
@@ -3016,7 +3016,7 @@ int dspsr_b200_pipeline_create (dspsr_b200_context* ctx, const dspsr_b200_pipeli
                  "pipeline: filterbank_nchan=%u not a power of two in [4, 4096]", fb);
   }
   pl->fb_nsub = fb;
-  if (fb >= 128 && upload_pass_tables (fb, &pl->fb_tab, &pl->fb_tab_cap) != cudaSuccess)
+  if (filterbank_uses_tables (fb) && upload_pass_tables (fb, &pl->fb_tab, &pl->fb_tab_cap) != cudaSuccess)
   {
     delete pl;
     return fail (ctx, DSPSR_B200_ECUDA, "pipeline: filterbank tables");

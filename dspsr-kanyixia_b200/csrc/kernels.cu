@@ -1107,9 +1107,9 @@ cudaError_t launch_filterbank (const InputView& in, const float* d_lut, unsigned
   if (nblk == 0) return cudaSuccess;
   // up to 64 channels the one-thread-per-block register transform is faster;
   // 128 to 1024 fit a warp with 32 points per thread, more need the block
+  if (filterbank_uses_tables (nsub) && !ptab) return cudaErrorInvalidValue;
   if (nsub >= 128)
   {
-    if (!ptab) return cudaErrorInvalidValue;
     switch (nsub)
     {
       case 128: return run_filterbank_warp<128> (in, d_lut, nblk, scale, out, out_span, st, clk);

@@ -198,8 +198,9 @@ cudaError_t launch_unpermute_response (float2* dst, const float2* H, unsigned nc
 
 // FFT filterbank, freq_res = 1: nsub a power of two in [4, 4096]; nblk blocks
 // of nsub input samples per (input channel, pol); output FPT with channel
-// cin*nsub + k, span out_span.  nsub >= 128 runs the transforms in shared
-// memory and needs the per-pass tables of the nsub-point FFT (ptab).
+// cin*nsub + k, span out_span.  Above 1024 channels the transforms run in shared
+// memory and need the per-pass tables of the nsub-point FFT (ptab).
+inline bool filterbank_uses_tables (unsigned nsub) { return nsub > 1024; }
 cudaError_t launch_filterbank (const InputView& in, const float* d_lut, unsigned nsub,
                                uint64_t nblk, float scale, float2* out, uint64_t out_span,
                                cudaStream_t stream, const KernelClock* clock = nullptr,

@@ -172,6 +172,33 @@ def test_filterbank_sizes(ctx, b2, nsub, kind, npol, nchan):
         assert rel_rms(g, ref) < VOLTAGE_RTOL
 
 
+def test_filterbank_captured_at_its_first_call(b2):
+    """Up to 1024 channels a call sets nothing up: its first one, at a length
+    other than the last call's, can be captured."""
+    st = torch.cuda.Stream()
+    ctx = b2.Context(0, st.cuda_stream)
+    ndat = 1 << 15
+    d = torch.randn((1, 2, ndat, 2), device="cuda")
+    out = torch.zeros((1024, 2, 300, 2), device="cuda")
+    torch.cuda.synchronize()
+    for nsub in (2048, 256, 1024, 128):
+        want = torch.zeros_like(out)
+        got = torch.zeros_like(out)
+        torch.cuda.synchronize()
+        if nsub > 1024:
+            ctx.filterbank(b2.FLOAT_FPT, d, ndat, 1, 2, nsub, out, 300, in_span=ndat)
+            ctx.synchronize()
+            continue
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            ctx.filterbank(b2.FLOAT_FPT, d, ndat, 1, 2, nsub, got, 300, in_span=ndat)
+        g.replay()
+        ctx.filterbank(b2.FLOAT_FPT, d, ndat, 1, 2, nsub, want, 300, in_span=ndat)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and bool((want != 0).any())
+    ctx.close()
+
+
 @pytest.mark.parametrize("lin", [64, 128, 256, 512, 1024, 2048])
 @pytest.mark.parametrize("kind,npol", [("i16", 2), ("i8", 1), ("f", 2)])
 def test_inverse_filterbank_sizes(ctx, b2, orc, lin, kind, npol):
