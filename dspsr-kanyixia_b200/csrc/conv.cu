@@ -292,8 +292,8 @@ void launch_inv (const ConvShape& sh, dim3 grid, float2* scratch, uint64_t part0
   // 2 M samples in 20.7 us against 25.0
   if constexpr (N1 >= 8 && NPOL == 2 && MODE != OUT_VOLTAGE)
   {
-    launch_inv_split<N1, MODE, NOUT> (scratch, {sh.n2, sh.n2, sh.nchan, sh.nkeep, sh.nfilt_pos},
-                                      part0, grid.y, tb.tw4, tb.nsm, fv, vv, st);
+    launch_inv_split<N1, NOUT> (scratch, {sh.n2, sh.n2, sh.nchan, sh.nkeep, sh.nfilt_pos}, part0,
+                                grid.y, tb.tw4, tb.nsm, fv, st);
     return;
   }
   else

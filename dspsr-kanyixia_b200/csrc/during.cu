@@ -476,9 +476,12 @@ void launch_inv_during (const DuringShape& sh, dim3 grid, const float2* scratch,
                         const DuringTables& tb, const FoldView& fv, const VoltView& vv,
                         cudaStream_t st)
 {
-  if constexpr (N1 >= 8 && N1 <= 32 && NPOL == 2)
-    launch_inv_split<N1, MODE, NOUT> (scratch, {sh.n2, sh.seg, sh.nchan_in, sh.nkeep, sh.nfilt_pos},
-                                      part0, grid.y, tb.twd, tb.nsm, fv, vv, st);
+  // voltages need no exchange of the polarisations (calls of 8 M samples, int8,
+  // split / a thread per column: 64 x 4096 206.9 / 198.7 us, 64 x 2048 194.6 /
+  // 191.5, 32 x 2048 183.3 / 180.3)
+  if constexpr (N1 >= 8 && N1 <= 32 && NPOL == 2 && MODE != OUT_VOLTAGE)
+    launch_inv_split<N1, NOUT> (scratch, {sh.n2, sh.seg, sh.nchan_in, sh.nkeep, sh.nfilt_pos},
+                                part0, grid.y, tb.twd, tb.nsm, fv, st);
   else
     k_inv_cols_during<N1, NPOL, MODE, NOUT><<<grid, 128, 0, st>>> (scratch, sh, part0, tb.twd, fv,
                                                                    vv);

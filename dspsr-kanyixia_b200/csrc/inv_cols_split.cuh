@@ -26,9 +26,9 @@ template <int N1> B200_CE int ivs_cols () { return 128 / ivs_split<N1> (); }
 // resident blocks per SM that the registers are sized for
 template <int N1> B200_CE int ivs_blocks () { return N1 == 8 ? 10 : 8; }
 
-// K3 for two polarisations and n1 = 8, 16 or 32.  A thread transforms one
-// polarisation of one column (at n1 = 32 the even or the odd rows of it), so
-// that it needs 64 registers or less and 32 warps and more keep loads in
+// K3 with detection and fold, for two polarisations and n1 = 8, 16 or 32.  A
+// thread transforms one polarisation of one column (at n1 = 32 the even or the
+// odd rows of it), so that it needs 64 registers or less and 32 warps and more keep loads in
 // flight: the pass waits for HBM and for the latency of the fold's shuffles,
 // and a thread per column with both polarisations (128 to 168 registers, 11
 // to 16 warps per SM) left 60 % of the issue slots empty.  The values are
@@ -39,11 +39,10 @@ template <int N1> B200_CE int ivs_blocks () { return N1 == 8 ? 10 : 8; }
 // + gridDim.y, ...).  Before and now: 239 and 162 us at n1 = 16 (10.5 M samples,
 // long bins), 174 and 99 us at n1 = 32, and for the filterbank with a response
 // (n1 = 32) 615 and 363 us.
-template <int N1, int MODE, int NOUT, bool LONG>
+template <int N1, int NOUT, bool LONG>
 __global__ void __launch_bounds__ (128, ivs_blocks<N1> ())
 k_inv_cols_split (const float2* __restrict__ scratch, const InvColsShape sh, const uint64_t part0,
-                  const unsigned nbatch, const float2* __restrict__ tw, const FoldView fv,
-                  const VoltView vv)
+                  const unsigned nbatch, const float2* __restrict__ tw, const FoldView fv)
 {
   constexpr int HS = N1 == 32 ? 2 : 1;            // halves of a column
   constexpr int V = N1 / HS;                      // values per thread
@@ -77,16 +76,13 @@ k_inv_cols_split (const float2* __restrict__ scratch, const InvColsShape sh, con
     for (int m = 0; m < V; m++) v[m] = __ldcs (src + uint64_t (HS * m + h) * sh.n2);
     // the profile columns of the samples, asked for with the values: waited for
     // one after another in the fold they were most of the pass's time
-    unsigned fcol[MODE == OUT_FOLD ? R : 1];
-    if constexpr (MODE == OUT_FOLD)
-    {
+    unsigned fcol[R];
 #pragma unroll
-      for (int r = 0; r < R; r++)
-      {
-        const uint64_t tl = uint64_t (sample (r)) * sh.seg + t2;
-        const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
-        fcol[r] = fold_column (fv, ok, tbase + (tl - sh.nfilt_pos));
-      }
+    for (int r = 0; r < R; r++)
+    {
+      const uint64_t tl = uint64_t (sample (r)) * sh.seg + t2;
+      const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
+      fcol[r] = fold_column (fv, ok, tbase + (tl - sh.nfilt_pos));
     }
     __syncthreads ();                  // the twiddles are there; the last part's reads are done
 #pragma unroll
@@ -119,21 +115,8 @@ k_inv_cols_split (const float2* __restrict__ scratch, const InvColsShape sh, con
     }
     __syncthreads ();
     const auto emit = [&] (int r, float2 p, float2 q) {
-      if constexpr (MODE == OUT_VOLTAGE)
-      {
-        const uint64_t tl = uint64_t (sample (r)) * sh.seg + t2;
-        if (tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep)
-        {
-          float2* o = vv.out + uint64_t (c) * 2 * vv.span + tbase + (tl - sh.nfilt_pos);
-          o[0] = p;
-          o[vv.span] = q;
-        }
-      }
-      else
-      {
-        detect_row<LONG> (rf, fv.state, 2, fcol[r], p, q);
-        if (LONG && (r + 1) % RF::ROWS == 0) rf.flush ();
-      }
+      detect_row<LONG> (rf, fv.state, 2, fcol[r], p, q);
+      if (LONG && (r + 1) % RF::ROWS == 0) rf.flush ();
     };
     if constexpr (HS == 1)
     {
@@ -161,22 +144,20 @@ k_inv_cols_split (const float2* __restrict__ scratch, const InvColsShape sh, con
   }
 }
 
-template <int N1, int MODE, int NOUT>
+template <int N1, int NOUT>
 void launch_inv_split (const float2* scratch, const InvColsShape& sh, uint64_t part0,
                        unsigned nbatch, const float2* tw, int nsm, const FoldView& fv,
-                       const VoltView& vv, cudaStream_t st)
+                       cudaStream_t st)
 {
   const unsigned gx = sh.n2 / ivs_cols<N1> ();
   // about four blocks of work per resident block, then parts per block
   const unsigned resident = unsigned (nsm) * ivs_blocks<N1> ();
   const unsigned want = std::max (1u, 4 * resident / std::max (1u, gx * sh.nchan_in));
   const dim3 grid (gx, std::min (nbatch, want), sh.nchan_in);
-  if (MODE == OUT_FOLD && fv.long_bins)
-    k_inv_cols_split<N1, MODE, NOUT, MODE == OUT_FOLD><<<grid, 128, 0, st>>> (scratch, sh, part0,
-                                                                             nbatch, tw, fv, vv);
+  if (fv.long_bins)
+    k_inv_cols_split<N1, NOUT, true><<<grid, 128, 0, st>>> (scratch, sh, part0, nbatch, tw, fv);
   else
-    k_inv_cols_split<N1, MODE, NOUT, false><<<grid, 128, 0, st>>> (scratch, sh, part0, nbatch, tw,
-                                                                   fv, vv);
+    k_inv_cols_split<N1, NOUT, false><<<grid, 128, 0, st>>> (scratch, sh, part0, nbatch, tw, fv);
 }
 
 } // namespace
