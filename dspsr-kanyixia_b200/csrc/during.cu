@@ -242,22 +242,20 @@ constexpr int COLW = 16;
 template <int N1, int CW = COLW>
 B200_CE int colbig_stride () { return spad_size (N1) + (CW >= 16 ? 1 : 2); }
 
-template <int N1, int NPOL>
+template <int N1>
 constexpr size_t colbig_smem ()
 {
-  return size_t (NPOL * COLW * colbig_stride<N1> () + pass_tables_size (N1)) * sizeof (float2);
+  return size_t (COLW * colbig_stride<N1> () + pass_tables_size (N1)) * sizeof (float2);
 }
 
-// columns per CTA of the inverse pass: 8 for 512-point columns, so that both
-// polarisations (72 KB) leave room for a second CTA on the SM
+// columns per CTA of the inverse pass
 template <int N1>
 B200_CE int inv_colw () { return N1 >= 512 ? 8 : COLW; }
 
-template <int N1, int NPOL>
+template <int N1>
 constexpr size_t colbig_inv_smem ()
 {
-  return size_t (NPOL * inv_colw<N1> () * colbig_stride<N1, inv_colw<N1> ()> ()
-                 + pass_tables_size (N1))
+  return size_t (inv_colw<N1> () * colbig_stride<N1, inv_colw<N1> ()> () + pass_tables_size (N1))
          * sizeof (float2);
 }
 
@@ -377,12 +375,13 @@ k_fwd_cols_big (const InputView in, const float* __restrict__ lut, const uint64_
   }
 }
 
-// Inverse columns of the During filterbank for N1 = 64 .. 512: the 16
-// columns of a CTA lie in one output channel's segment (seg >= 64); both
-// polarisations are loaded with the conjugate twiddle exp(+2 pi i k1 t2 /
-// freq_res), transformed, and read back in time order (16 consecutive
-// samples per row) for the discard and the voltages or detection + fold.
-template <int N1, int NPOL, int MODE, int NOUT>
+// Inverse columns of the During filterbank for N1 = 64 .. 512 and one
+// polarisation (two: k_inv_cols_big_pair): the columns of a CTA lie in one output
+// channel's segment (seg >= 64); they are loaded with the conjugate twiddle
+// exp(+2 pi i k1 t2 / freq_res), transformed, and read back in time order (16
+// consecutive samples per row) for the discard and the voltages or detection
+// + fold.
+template <int N1, int MODE>
 __global__ void __launch_bounds__ (inv_colw<N1> () * stockham_threads (N1), 1024 / N1)
 k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
                        const uint64_t part0, const float2* __restrict__ twd,
@@ -393,7 +392,7 @@ k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
   constexpr int SP = colbig_stride<N1, CW> ();
   constexpr int TAB = pass_tables_size (N1);
   extern __shared__ __align__ (16) float2 s_cb[];
-  float2* tab = s_cb + NPOL * CW * SP;
+  float2* tab = s_cb + CW * SP;
   for (int i = threadIdx.x; i < TAB; i += T) tab[i] = __ldg (ptab_col + i);
   const unsigned c0 = blockIdx.x * CW;
   const unsigned b = blockIdx.y;
@@ -403,31 +402,24 @@ k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
   const unsigned c = cin * sh.nsub + cs;
   // thread (kk, j) takes rows k1 = kk + m KSTEP of column c0 + j
   constexpr int KSTEP = T / CW;
-  const int j = threadIdx.x % CW, kk = threadIdx.x / CW;
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
   {
-    const float2* src = scratch + ((uint64_t (b) * sh.nchan_in + cin) * NPOL + p) * N + c0 + j
+    const int j = threadIdx.x % CW, kk = threadIdx.x / CW;
+    const float2* src = scratch + (uint64_t (b) * sh.nchan_in + cin) * N + c0 + j
                         + uint64_t (kk) * sh.n2;
     const float2* tw = twd + uint64_t (kk) * sh.seg + t20 + j;
-    float2* col = s_cb + p * CW * SP + j * SP;
     const uint64_t sstep = uint64_t (KSTEP) * sh.n2, tstep = uint64_t (KSTEP) * sh.seg;
     for (int k1 = kk; k1 < N1; k1 += KSTEP, src += sstep, tw += tstep)
     {
       float2 x = *src;
       if (k1) x = cmulc (x, __ldg (tw));
-      col[spad (k1)] = x;
+      s_cb[j * SP + spad (k1)] = x;
     }
   }
   __syncthreads ();
-#pragma unroll
-  for (int p = 0; p < NPOL; p++)
-    colbig_fft<N1, +1, SP> (s_cb + p * CW * SP, tab);
+  colbig_fft<N1, +1, SP> (s_cb, tab);
   __syncthreads ();                    // the fold below reads across columns' groups
   const uint64_t tbase = (part0 + b) * sh.nkeep;
-  const float2* c0p = s_cb;
-  const float2* c1p = s_cb + (NPOL - 1) * CW * SP;
-  float* prof = fv.profiles + uint64_t (c) * NOUT * fv.stride;
+  float* prof = fv.profiles + uint64_t (c) * fv.stride;
   unsigned* hits = c == 0 ? fv.hits : nullptr;
   for (int e = threadIdx.x; e < CW * N1; e += T)
   {
@@ -435,18 +427,13 @@ k_inv_cols_during_big (const float2* __restrict__ scratch, const DuringShape sh,
     const uint64_t tl = uint64_t (t1) * sh.seg + t20 + j;
     const bool ok = tl >= sh.nfilt_pos && tl < sh.nfilt_pos + sh.nkeep;
     const uint64_t t = tbase + (tl - sh.nfilt_pos);
-    const float2 pv = c0p[j * SP + spad (t1)];
-    const float2 qv = c1p[j * SP + spad (t1)];
+    const float2 v = s_cb[j * SP + spad (t1)];
     if constexpr (MODE == OUT_VOLTAGE)
     {
-      if (ok)
-      {
-        vv.out[(uint64_t (c) * NPOL) * vv.span + t] = pv;
-        if (NPOL == 2) vv.out[(uint64_t (c) * NPOL + 1) * vv.span + t] = qv;
-      }
+      if (ok) vv.out[uint64_t (c) * vv.span + t] = v;
     }
     else
-      detect_fold<NOUT> (fv, NPOL, fold_column (fv, ok, t), pv, qv, prof, hits);
+      detect_fold<1> (fv, 1, fold_column (fv, ok, t), v, v, prof, hits);
   }
 }
 
@@ -569,11 +556,11 @@ cudaError_t launch_inv_during_big (const DuringShape& sh, dim3 grid, const float
       return launch_inv_big_pair<N1, OUT_FOLD, 2> (sh, tb, part0, grid.y, scratch, fv, vv, st);
     return launch_inv_big_pair<N1, OUT_FOLD, 4> (sh, tb, part0, grid.y, scratch, fv, vv, st);
   }
-  constexpr size_t smem = colbig_inv_smem<N1, 1> ();
+  constexpr size_t smem = colbig_inv_smem<N1> ();
   constexpr int T = inv_colw<N1> () * stockham_threads (N1);
   grid.x = sh.n2 / inv_colw<N1> ();
-  auto k = mode == OUT_VOLTAGE ? k_inv_cols_during_big<N1, 1, OUT_VOLTAGE, 1>
-                               : k_inv_cols_during_big<N1, 1, OUT_FOLD, 1>;
+  auto k = mode == OUT_VOLTAGE ? k_inv_cols_during_big<N1, OUT_VOLTAGE>
+                               : k_inv_cols_during_big<N1, OUT_FOLD>;
   const cudaError_t e = cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               int (smem));
   if (e != cudaSuccess) return e;
@@ -587,11 +574,11 @@ cudaError_t run_during_big (const DuringShape& sh, const DuringTables& tb, const
                             const FoldView& fv, const VoltView& vv, cudaStream_t st,
                             const KernelClock* clk)
 {
-  static_assert (colbig_inv_smem<N1, 1> () <= 227u * 1024u, "column kernel shared memory");
+  static_assert (colbig_inv_smem<N1> () <= 227u * 1024u, "column kernel shared memory");
   const dim3 gcol (sh.n2 / COLW, nbatch, sh.nchan_in);
   {
     ClockScope cs (clk, KK_FWD_COLS, st);
-    constexpr size_t smem = colbig_smem<N1, 1> ();
+    constexpr size_t smem = colbig_smem<N1> ();
     if (in.npol == 2 && fwd_pair_aligned (in))
     {
       const cudaError_t e = launch_fwd_big_pair<N1> (sh, tb, in, part0, nbatch, scratch, st);
