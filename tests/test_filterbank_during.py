@@ -301,3 +301,79 @@ def test_during_fold_matches_its_voltages(ctx, b2, orc, state, npol, nsub, fr):
     assert rel_rms(prof, rprof) < 1e-5, rel_rms(prof, rprof)
     f.close()
     fbd.close()
+
+
+# shapes whose big transforms have n1 = 2 .. 512 columns, products, input kind
+COLUMN_SHAPES = [(16, 1024, 0, "float"), (16, 2048, 1, "int8"), (32, 2048, 3, "int16"),
+                 (16, 8192, 0, "int8"), (64, 4096, 2, "int8"), (8, 65536, 1, "int16"),
+                 (64, 16384, 3, "float"), (32, 65536, 0, "int8"), (64, 65536, 3, "int8")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nsub,fr,state,kind", COLUMN_SHAPES)
+def test_during_columns_and_folds(ctx, b2, orc, nsub, fr, state, kind):
+    """Every column pass for two polarisations: voltages against the 64-bit
+    oracle, and the fused folds, with bins much longer and shorter than a
+    sample, against detection and fold of those voltages; hits bit-exact."""
+    torch = pytest.importorskip("torch")
+    nfilt, npart = (fr // 20 + 3, fr // 16), 2
+    fbd = b2.FilterbankDuring(ctx, 1, 2, nsub, fr, nfilt)
+    assert fbd.info["n1"] == nsub * fr // 8192
+    rng = np.random.default_rng(nsub + fr)
+    resp = (np.exp(2j * np.pi * rng.random((nsub, fr))) * rng.uniform(0.5, 1.5, (nsub, fr))
+            / np.sqrt(float(nsub) * fr * fr)).astype(np.complex64)
+    fbd.copy_response(resp)
+    nkeep = fbd.info["nkeep"]
+    ndat = npart * nsub * nkeep + sum(nfilt) * nsub + 3
+    raw, x, ik, lut = _input(rng, 1, 2, ndat, kind, b2)
+    d_in = torch.from_numpy(np.ascontiguousarray(raw).view(np.float32) if kind == "float" else raw).cuda()
+    span = npart * nkeep
+    d_v = torch.zeros((nsub, 2, span, 2), device="cuda")
+    kw = dict(input_kind=ik, lut=lut)
+    assert fbd.perform(d_in, ndat, d_v, span, **kw) == npart
+    ctx.synchronize()
+    v = d_v.cpu().numpy().view(np.complex64)[..., 0]
+    ref = orc.filterbank_during(x.astype(np.complex128), nsub, fr, nfilt, resp.astype(np.complex128))
+    assert rel_rms(v, ref) < DURING_RTOL_FP64, rel_rms(v, ref)
+    det = orc.detect(v.astype(np.complex128), state)
+    for nbin, per_bin in ((128, 0.4), (16, 150.0)):
+        phi, pps = 0.3, 1.0 / (nbin * per_bin)
+        plan = orc.fold_binplan(phi, pps, span, nbin)
+        rprof, rhits = orc.fold_accumulate(det, plan, nbin)
+        f = b2.Fold(ctx, nbin, nsub, det.shape[1])
+        f.set_bins(phi, pps, span)
+        assert fbd.perform_fold(d_in, ndat, f, state, **kw) == npart
+        prof, hits = f.get_profiles()
+        f.close()
+        assert np.array_equal(hits, rhits)
+        assert rel_rms(prof, rprof) < 1e-5, rel_rms(prof, rprof)
+    fbd.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nsub,fr", [(16, 2048), (64, 4096), (8, 65536), (64, 65536)])
+@pytest.mark.parametrize("kind,offset", [("int8", 2), ("int16", 4)])
+def test_during_blocks_between_words(ctx, b2, nsub, fr, kind, offset):
+    """A block at an address that is no multiple of a dual-polarisation
+    sample's gives the voltages of the same block aligned."""
+    torch = pytest.importorskip("torch")
+    nfilt = (fr // 16, fr // 16)
+    fbd = b2.FilterbankDuring(ctx, 1, 2, nsub, fr, nfilt)
+    rng = np.random.default_rng(nsub + offset)
+    fbd.copy_response((np.exp(2j * np.pi * rng.random((nsub, fr))) / np.sqrt(float(nsub) * fr * fr)
+                       ).astype(np.complex64))
+    nkeep = fbd.info["nkeep"]
+    ndat = nsub * nkeep + sum(nfilt) * nsub
+    raw, _, ik, lut = _input(rng, 1, 2, ndat, kind, b2)
+    raw = raw.view(np.uint8)
+    whole = torch.zeros(raw.size + 16, dtype=torch.uint8, device="cuda")
+    whole[offset:offset + raw.size] = torch.from_numpy(raw).cuda()
+    out = []
+    for d in (torch.from_numpy(raw).cuda(), whole[offset:]):
+        o = torch.zeros((nsub, 2, nkeep, 2), device="cuda")
+        assert fbd.perform(d, ndat, o, nkeep, input_kind=ik, lut=lut) == 1
+        ctx.synchronize()
+        out.append(o.cpu().numpy().view(np.complex64)[..., 0])
+    fbd.close()
+    # two kernels of the same precision
+    assert rel_rms(out[1], out[0]) < DURING_RTOL
