@@ -25,8 +25,8 @@ def rel_rms(a, b):
     return float(np.sqrt(np.mean(np.abs(a - b) ** 2) / np.mean(np.abs(b) ** 2)))
 
 
-# nfft, row length, channels, input kind (8-bit: affine table or not), state,
-# nbin, samples per bin
+# nfft, row length (0: the default, 4096 up to 2^17 points and 8192 above),
+# channels, input kind (8-bit: affine table or not), state, nbin, samples per bin
 PATHS = [
     (1 << 14, 4096, 1, "i8", 3, 64, 2000.0),      # n1 4, one column per row of samples
     (1 << 14, 8192, 2, "i8", 1, 512, 0.4),        # n1 2, bins shorter than a sample
@@ -36,7 +36,8 @@ PATHS = [
     (1 << 16, 0, 3, "i16", 3, 256, 11.0),         # n1 16, channels that do not tile
     (1 << 16, 0, 8, "i8", 0, 64, 900.0),          # n1 16, transposing load
     (1 << 16, 8192, 1, "f", 2, 333, 3.0),         # n1 8 with 8192-point rows
-    (1 << 17, 0, 1, "i8", 3, 256, 33.0),          # n1 16, 8192-point rows
+    (1 << 17, 8192, 1, "i8", 3, 256, 33.0),       # n1 16, 8192-point rows
+    (1 << 17, 0, 8, "i8", 2, 256, 90.0),          # n1 32, transposing load
     (1 << 17, 4096, 1, "i16", 1, 256, 100.0),     # n1 32, 4096-point rows
     (1 << 18, 0, 2, "lut", 3, 1024, 11.0),        # n1 32
     (1 << 18, 0, 1, "f", 0, 64, 5000.0),
@@ -62,7 +63,9 @@ def test_pipeline_paths_match_oracle(ctx, b2, orc, path):
     nk = nfft - cfg["pos"] - cfg["neg"]
     # the second block starts with a carried prefix that parts straddle
     blocks = make_blocks(rng, cfg, [nfft + nk + 777, 2 * nk + 12345])
-    prof, hits, total, _ = run_pipeline(ctx, b2, blocks, cfg)
+    prof, hits, total, info = run_pipeline(ctx, b2, blocks, cfg)
+    n2 = path[1] or (4096 if nfft <= 1 << 17 else 8192)
+    assert (info["n1"], info["n2"]) == (nfft // n2, n2)
     rprof, rhits, rtotal = oracle_chain(orc, b2, blocks, cfg)
     check(prof, hits, total, rprof, rhits, rtotal, cfg["state"])
 
