@@ -26,6 +26,44 @@ using namespace b200;
 
 #include "context.h"
 
+int* dspsr_b200_wait_words::take ()
+{
+  std::lock_guard<std::mutex> g (lock);
+  if (spare.empty ())
+  {
+    int* page = nullptr;
+    if (cudaHostAlloc (&page, PER_PAGE * sizeof (int), cudaHostAllocMapped) != cudaSuccess)
+      return nullptr;
+    pages.push_back (page);
+    for (int i = PER_PAGE - 1; i >= 0; i--) spare.push_back (page + i);
+  }
+  int* word = spare.back ();
+  spare.pop_back ();
+  *word = 0;
+  used.push_back (word);
+  return word;
+}
+
+void dspsr_b200_wait_words::give (int* word)
+{
+  std::lock_guard<std::mutex> g (lock);
+  used.erase (std::find (used.begin (), used.end (), word));
+  spare.push_back (word);
+}
+
+bool dspsr_b200_wait_words::any_set ()
+{
+  std::lock_guard<std::mutex> g (lock);
+  for (const volatile int* w : used)
+    if (*w) return true;
+  return false;
+}
+
+dspsr_b200_wait_words::~dspsr_b200_wait_words ()
+{
+  for (int* p : pages) cudaFreeHost (p);
+}
+
 namespace {
 
 int fail (dspsr_b200_context* ctx, int code, const char* fmt, ...)
@@ -62,27 +100,14 @@ struct WaitFlag
   int* dev = nullptr;
   cudaError_t create (dspsr_b200_context* ctx)
   {
-    const cudaError_t e = cudaHostAlloc (&host, sizeof (int), cudaHostAllocMapped);
-    if (e != cudaSuccess)
-    {
-      host = nullptr;
-      return e;
-    }
-    *host = 0;
     owner = ctx->waits;
-    std::lock_guard<std::mutex> g (owner->lock);
-    owner->words.push_back (host);
-    return cudaHostGetDevicePointer (&dev, host, 0);
+    host = owner->take ();
+    return host ? cudaHostGetDevicePointer (&dev, host, 0) : cudaErrorMemoryAllocation;
   }
   bool set () const { return host && *static_cast<const volatile int*> (host); }
   void release ()
   {
-    if (!host) return;
-    {
-      std::lock_guard<std::mutex> g (owner->lock);
-      owner->words.erase (std::find (owner->words.begin (), owner->words.end (), host));
-    }
-    cudaFreeHost (host);
+    if (host) owner->give (host);
     host = dev = nullptr;
   }
 };
@@ -96,10 +121,7 @@ int wait_failed (dspsr_b200_context* ctx)
 // caller has synchronised with the work that it asks about
 int context_waits (dspsr_b200_context* ctx)
 {
-  std::lock_guard<std::mutex> g (ctx->waits->lock);
-  for (const volatile int* w : ctx->waits->words)
-    if (*w) return wait_failed (ctx);
-  return DSPSR_B200_OK;
+  return ctx->waits->any_set () ? wait_failed (ctx) : DSPSR_B200_OK;
 }
 
 // Per-pass Stockham tables of an n-point transform uploaded into a device

@@ -9,12 +9,21 @@
 #include <string>
 #include <vector>
 
-// Status words of the convolutions made on a context (WaitFlag in capi.cu);
-// shared with them, since an engine may outlive its context
+// Status words of the convolutions made on a context (WaitFlag in capi.cu):
+// host memory that the device can write, a page at a time (an allocation per
+// engine took 1.3 ms of its creation).  Shared with the engines, which may
+// outlive their context; the pages go with the last of them.
 struct dspsr_b200_wait_words
 {
+  static constexpr int PER_PAGE = 1024;
   std::mutex lock;
-  std::vector<const volatile int*> words;
+  std::vector<int*> pages, spare, used;
+  // a word that reads 0, or null when no page can be had
+  int* take ();
+  void give (int* word);
+  // whether any word in use is set
+  bool any_set ();
+  ~dspsr_b200_wait_words ();
 };
 
 struct dspsr_b200_context

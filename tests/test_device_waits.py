@@ -141,3 +141,27 @@ def test_pipeline_status_reaches_subints(own, b2):
             assert len(got) == seen
         pl.close()
     own.synchronize()
+
+
+@pytest.mark.gpu
+def test_status_words_are_each_engines_own(own, b2):
+    """Engines that come and go: each word starts at 0 and is seen by its own
+    engine alone, also where another engine's set word was handed back."""
+    engines = [b2.Convolution(own, 1, 2, 4096, 10, 10) for _ in range(1100)]
+    words = [word_of(own, own._lib.dspsr_b200_convolution_status_word, c.handle) for c in engines]
+    assert len({ctypes.addressof(w.contents) for w in words}) == len(engines)
+    assert all(w[0] == 0 for w in words)
+    words[7][0] = words[1050][0] = 1
+    for i in (6, 8, 1049, 1051):
+        engines[i].status()
+    for i in (7, 1050):
+        with gave_up(b2):
+            engines[i].status()
+        engines[i].close()
+    own.synchronize()
+    again = [b2.Convolution(own, 1, 2, 4096, 10, 10) for _ in range(3)]
+    for c in again:
+        c.status()
+        assert word_of(own, own._lib.dspsr_b200_convolution_status_word, c.handle)[0] == 0
+    for c in engines[:7] + engines[8:1050] + engines[1051:] + again:
+        c.close()
