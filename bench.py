@@ -79,7 +79,8 @@ CONFIGS = {
         kind="ifb",
         workload=("inverse filterbank stage of C5 alone: 256 PFB channels int16 dual-pol, "
                   "1024-point input FFTs, 196608-point output spectra, 1 s of 800 MHz"),
-        nin=256, npol=2, lin=1024, disc=12288, ndat=4166784),
+        nin=256, npol=2, lin=1024, disc=12288, ndat=4166784, cf=1400.0, bw=800.0, dm=1000.0,
+        period=1.6e-3),
     "c2d": dict(
         kind="fbd",
         workload=("filterbank with the dedispersion inside it (-F 64:D): 256 MHz complex "
