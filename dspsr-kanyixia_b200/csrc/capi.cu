@@ -492,7 +492,7 @@ struct dspsr_b200_fold
   static constexpr size_t INITIAL_SEGMENTS = 16384;
   DevBuf<FoldSegment> d_segs[NRING];
   // the column of each sample is computed once per block (k_colplan: one
-  // segment search per 1024 samples) instead of by a search per warp in every
+  // segment search per 512 samples) instead of by a search per warp in every
   // channel's epilogue; with one channel it still pays (C1: 0.867 -> 0.827 ms
   // per block)
   bool use_cols = false;
@@ -2593,7 +2593,7 @@ int dspsr_b200_sk_mask (dspsr_b200_context* ctx, const uint8_t* d_mask, const fl
   return DSPSR_B200_OK;
 }
 
-// ---- unpack ----------------------------------------------------------------// ---- unpack ----------------------------------------------------------------
+// ---- unpack ----------------------------------------------------------------
 
 int dspsr_b200_unpack8 (dspsr_b200_context* ctx, const void* d_in, uint64_t ndat,
                         unsigned nchan, unsigned npol, unsigned ndim, const float* lut256,

@@ -240,9 +240,9 @@ __device__ __forceinline__ void fold_runs (unsigned hm, unsigned col, const floa
 // flush() finds the rows that have one column -- most of them -- and has 1 to
 // 8 lanes sum each (row, product), 32 values in eight 16-byte loads, one atomic
 // each; the others go to fold_runs in one rolled loop.  Against fold_runs for
-// every row (5 x NOUT shuffles) C1's inverse columns went from 239 to 162 us
-// with the rest of the pass; with 11 samples a bin (C2) the detour through
-// shared memory is slower, 803 against 664 us at n1 = 8.  Rows of 36 words: the
+// every row (5 x NOUT shuffles) C1's inverse columns (n1 = 16) went from 239 to
+// 162 us with the rest of the pass; with 11 samples a bin (C2) the detour
+// through shared memory is slower, 803 against 664 us at n1 = 8.  Rows of 36 words: the
 // row-wise accesses and the 16-byte loads of 8 lanes fall in distinct banks.
 template <int NOUT, int K>
 struct RowFold

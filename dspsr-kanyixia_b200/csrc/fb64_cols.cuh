@@ -42,10 +42,11 @@ namespace {
 // distinct bank pairs.  The pass is bound by the passes of its global and
 // shared accesses through L1: with 4-byte raw loads (eight lines a warp each)
 // and runs of 32 bytes (eight rows a warp) they were 640 per warp and column
-// at n1 = 8, now 430: 922 us before, 895 us now for 134 M two-polarisation points at
-// n1 = 8 and 985 us at n1 = 16 (the block's barriers are the largest stall).  An 8-bit table that is not affine is one 1 KB copy in
-// shared memory (eight interleaved copies measured 10 % slower: the occupancy
-// they cost outweighs the bank conflicts they remove).
+// at n1 = 8, now 430: 922 us before, 895 us now for 134 M two-polarisation
+// points at n1 = 8 and 985 us at n1 = 16 (the block's barriers are the largest
+// stall).  An 8-bit table that is not affine is one 1 KB copy in shared memory
+// (eight interleaved copies measured 10 % slower: the occupancy they cost
+// outweighs the bank conflicts they remove).
 
 constexpr int FBC_THREADS = 256;
 constexpr int FBC_COLS = FBC_THREADS / 32;      // columns per block, one per warp

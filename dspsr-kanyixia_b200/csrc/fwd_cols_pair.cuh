@@ -98,7 +98,8 @@ template <int N1, bool TILE> B200_CE int fwp_blocks () { return N1 == 16 ? (TILE
 // thread by thread each sector would be fetched once per channel.
 // Bound by HBM (4 or 8 B in, 16 B out per point of both polarisations) and by
 // issue.  Against a thread per polarisation: 10.5 M samples of one channel at
-// n1 = 16 172 us before, 108 us now; 32 channels at n1 = 2 180 and 82 us;
+// n1 = 16 172 us before, 108 us now (119 us at n1 = 32, where 2^17 points go
+// with 4096-point rows); 32 channels at n1 = 2 180 and 82 us;
 // 2^18-point transforms of int16 at n1 = 32 (below) 76 and 46 us.
 template <int N1, int KIND, bool AFFINE, bool TILE>
 __global__ void __launch_bounds__ (fwp_threads<TILE> (), fwp_blocks<N1, TILE> ())

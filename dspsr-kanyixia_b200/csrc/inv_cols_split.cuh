@@ -28,17 +28,18 @@ template <int N1> B200_CE int ivs_blocks () { return N1 == 8 ? 10 : 8; }
 
 // K3 with detection and fold, for two polarisations and n1 = 8, 16 or 32.  A
 // thread transforms one polarisation of one column (at n1 = 32 the even or the
-// odd rows of it), so that it needs 64 registers or less and 32 warps and more keep loads in
-// flight: the pass waits for HBM and for the latency of the fold's shuffles,
+// odd rows of it), so that it needs 64 registers or less and 32 warps and more
+// keep loads in flight: the pass waits for HBM and for the latency of the fold's shuffles,
 // and a thread per column with both polarisations (128 to 168 registers, 11
 // to 16 warps per SM) left 60 % of the issue slots empty.  The values are
 // exchanged through shared memory, after which every thread has both
 // polarisations of n1 / 2 (8, 16) or eight (32) of the column's samples; the
 // last radix-2 step of n1 = 32 is taken there.  The twiddles of the block's
 // columns stay in shared memory for all its parts (b = blockIdx.y,
-// + gridDim.y, ...).  Before and now: 239 and 162 us at n1 = 16 (10.5 M samples,
-// long bins), 174 and 99 us at n1 = 32, and for the filterbank with a response
-// (n1 = 32) 615 and 363 us.
+// + gridDim.y, ...).  A thread per column and now: 239 and 162 us at n1 = 16
+// (10.5 M samples of one channel, long bins; 192 us at n1 = 32, where 2^17
+// points go with 4096-point rows), 174 and 99 us at n1 = 32 (2^18 points), and
+// for the filterbank with a response (n1 = 32) 615 and 363 us.
 template <int N1, int NOUT, bool LONG>
 __global__ void __launch_bounds__ (128, ivs_blocks<N1> ())
 k_inv_cols_split (const float2* __restrict__ scratch, const InvColsShape sh, const uint64_t part0,
