@@ -44,7 +44,10 @@ struct FbWarp
   static_assert (NB * RS % 2 == 0 && RS % 2 == 0, "16-byte aligned regions");
 };
 
-template <int NSUB, int KIND>
+// TWO: both polarisations of TFPD samples in a tile, so that one load
+// instruction takes them from the same sectors (a warp's first transforms are of
+// one, the others of the other; the regions of one lie together)
+template <int NSUB, int KIND, bool TWO>
 __global__ void __launch_bounds__ (FBW_WARPS * 32, 2)
 k_filterbank_warp (const InputView in, const float* __restrict__ lut, const uint64_t nblk,
                    const float scale, float2* __restrict__ out, const uint64_t out_span,
@@ -64,19 +67,24 @@ k_filterbank_warp (const InputView in, const float* __restrict__ lut, const uint
   }
   __syncthreads ();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = lane % M, slot = warp * F::G + lane / M;
-  float2* s = s_fbw + slot * F::RS;
   const unsigned npol = in.npol;
   const uint64_t rowv = uint64_t (in.nchan) * npol;      // TFPD values per time sample
+  static_assert (!TWO || (KIND != IN_FLOAT && F::G >= 2), "two transforms of a warp");
+  constexpr int G = TWO ? F::G / 2 : F::G, NBT = FBW_WARPS * G;        // output samples: warp, tile
+  const int t = lane % M, grp = lane / M;
+  const int spol = TWO ? grp / G : 0, slot = warp * G + (TWO ? grp % G : grp);
+  float2* s = s_fbw + (spol * NBT + slot) * F::RS;
   for (uint64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x)
   {
-    // input channel * npol + pol: outermost for FPT rows, innermost for TFPD
+    // input channel and polarisation: outermost for FPT rows, innermost for TFPD
     // samples, whose sectors hold several rows: blocks at work together then
     // share them through L2 (32 dual-polarisation int8 channels into 512 each,
-    // 64 M values: 491 us, with the row outermost 768; into 128 each 668, 1350)
-    const uint64_t nrow = uint64_t (in.nchan) * npol;
-    const unsigned row = unsigned (KIND == IN_FLOAT ? tile / tiles_per_row : tile % nrow);
-    const uint64_t blk0 = (KIND == IN_FLOAT ? tile % tiles_per_row : tile / nrow) * F::NB;
+    // 64 M values: 768 us with the row outermost, 491 innermost, 352 with both
+    // polarisations in a tile; into 128 each 1350, 668 and 483)
+    const uint64_t nrow = TWO ? uint64_t (in.nchan) : rowv;
+    const unsigned trow = unsigned (KIND == IN_FLOAT ? tile / tiles_per_row : tile % nrow);
+    const uint64_t blk0 = (KIND == IN_FLOAT ? tile % tiles_per_row : tile / nrow) * NBT;
+    const unsigned row = TWO ? 2 * trow + spol : trow;
     const bool live = blk0 + slot < nblk;
     const uint64_t t0 = (blk0 + slot) * NSUB + t;
     CP v[32];
@@ -115,7 +123,7 @@ k_filterbank_warp (const InputView in, const float* __restrict__ lut, const uint
     {
       // the transform this lane's slot takes next starts on its way to L2
       const uint64_t nt = tile + gridDim.x;
-      const uint64_t nb0 = nt % tiles_per_row * F::NB + slot;
+      const uint64_t nb0 = nt % tiles_per_row * NBT + slot;
       if (t == 0 && nt < ntile && nb0 < nblk)
         prefetch_l2_span (static_cast<const float2*> (in.main)
                               + nt / tiles_per_row * in.main_span + nb0 * NSUB, NSUB * 8);
@@ -143,17 +151,18 @@ k_filterbank_warp (const InputView in, const float* __restrict__ lut, const uint
       for (int p = 0; p < M; p++) s[t + M * i + 32 * p] = v[i * M + p].z;
     }
     __syncthreads ();
-    const unsigned nb = unsigned (min (uint64_t (F::NB), nblk - blk0));
-    const unsigned cin = row / npol, p = row % npol;
-    float2* o = out + (uint64_t (cin) * NSUB * npol + p) * out_span + blk0;
+    const unsigned nb = unsigned (min (uint64_t (NBT), nblk - blk0));
+    const unsigned cin = TWO ? trow : row / npol, p0 = TWO ? 0 : row % npol;
+    float2* o = out + (uint64_t (cin) * NSUB * npol + p0) * out_span + blk0;
 #pragma unroll 8
     for (unsigned e = threadIdx.x; e < unsigned (F::NB * NSUB); e += FBW_WARPS * 32)
     {
-      const unsigned b = e % F::NB, k = e / F::NB;
-      const float2 y = s_fbw[b * F::RS + k];
+      const unsigned b = e % unsigned (NBT), k = e / unsigned (TWO ? F::NB : NBT);
+      const unsigned p = TWO ? e / unsigned (NBT) % 2 : 0;
+      const float2 y = s_fbw[(TWO ? p * NBT + b : b) * F::RS + k];
       if (b < nb)
-        o[uint64_t (k) * npol * out_span + b] = make_float2 (__fmul_rn (scale, y.x),
-                                                             __fmul_rn (scale, y.y));
+        o[(TWO ? uint64_t (k) * 2 + p : uint64_t (k) * npol) * out_span + b] =
+            make_float2 (__fmul_rn (scale, y.x), __fmul_rn (scale, y.y));
     }
     __syncthreads ();                  // the regions are free again
   }

@@ -1027,22 +1027,22 @@ cudaError_t sm_count (int* n)
   return e;
 }
 
-template <int NSUB, int KIND>
+template <int NSUB, int KIND, bool TWO>
 cudaError_t run_filterbank_warp_t (const InputView& in, const float* d_lut, uint64_t nblk,
                                    float scale, float2* out, uint64_t out_span, cudaStream_t st)
 {
   using F = FbWarp<NSUB>;
+  auto kern = k_filterbank_warp<NSUB, KIND, TWO>;
   int nsm = 0;
   cudaError_t e = sm_count (&nsm);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute (k_filterbank_warp<NSUB, KIND>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, int (F::SMEM));
+    e = cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int (F::SMEM));
   if (e != cudaSuccess) return e;
-  const uint64_t per_row = (nblk + F::NB - 1) / F::NB;
-  const uint64_t ntile = per_row * in.nchan * in.npol;
+  const unsigned pols = TWO ? 2 : 1, nbt = F::NB / pols;
+  const uint64_t per_row = (nblk + nbt - 1) / nbt;
+  const uint64_t ntile = per_row * in.nchan * in.npol / pols;
   const unsigned grid = unsigned (std::min<uint64_t> (ntile, 2 * uint64_t (nsm)));
-  k_filterbank_warp<NSUB, KIND><<<grid, FBW_WARPS * 32, F::SMEM, st>>> (
-      in, d_lut, nblk, scale, out, out_span, per_row, ntile);
+  kern<<<grid, FBW_WARPS * 32, F::SMEM, st>>> (in, d_lut, nblk, scale, out, out_span, per_row, ntile);
   return cudaGetLastError ();
 }
 
@@ -1052,11 +1052,16 @@ cudaError_t run_filterbank_warp (const InputView& in, const float* d_lut, uint64
                                  const KernelClock* clk)
 {
   ClockScope cs (clk, KK_FILTERBANK, st);
+  if constexpr (NSUB <= 512)
+    if (in.npol == 2 && in.kind != IN_FLOAT)
+      return in.kind == IN_INT8
+             ? run_filterbank_warp_t<NSUB, IN_INT8, true> (in, d_lut, nblk, scale, out, out_span, st)
+             : run_filterbank_warp_t<NSUB, IN_INT16, true> (in, d_lut, nblk, scale, out, out_span, st);
   if (in.kind == IN_INT8)
-    return run_filterbank_warp_t<NSUB, IN_INT8> (in, d_lut, nblk, scale, out, out_span, st);
+    return run_filterbank_warp_t<NSUB, IN_INT8, false> (in, d_lut, nblk, scale, out, out_span, st);
   if (in.kind == IN_INT16)
-    return run_filterbank_warp_t<NSUB, IN_INT16> (in, d_lut, nblk, scale, out, out_span, st);
-  return run_filterbank_warp_t<NSUB, IN_FLOAT> (in, d_lut, nblk, scale, out, out_span, st);
+    return run_filterbank_warp_t<NSUB, IN_INT16, false> (in, d_lut, nblk, scale, out, out_span, st);
+  return run_filterbank_warp_t<NSUB, IN_FLOAT, false> (in, d_lut, nblk, scale, out, out_span, st);
 }
 
 template <int NSUB>
