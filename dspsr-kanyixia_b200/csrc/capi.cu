@@ -419,6 +419,12 @@ int dspsr_b200_convolution::use_row_length (unsigned row_len)
     // the batch that the scratch in place holds (one part at least)
     int rc = make_split (other, row_len, scratch.n / (uint64_t (shape.nchan) * shape.npol * shape.nfft));
     if (!rc && have_response) rc = response_to_other ();
+    // the next call may run on another stream
+    if (!rc)
+    {
+      const cudaError_t e = cudaStreamSynchronize (ctx->stream);
+      if (e != cudaSuccess) rc = cuda_fail (ctx, e, "sync the second split");
+    }
     if (rc)
     {
       other.release ();

@@ -349,6 +349,33 @@ def test_rows_change_with_the_arithmetic(ctx, b2, orc):
     c.close()
 
 
+def test_change_of_the_arithmetic_then_of_the_stream(b2, orc):
+    """The second split's response is in place before a call on another stream."""
+    nfft, nchan = 1 << 16, 64
+    rng = np.random.default_rng(9)
+    h = np.exp(2j * np.pi * rng.random((nchan, nfft))).astype(np.complex64) / np.float32(np.sqrt(nfft))
+    x = (rng.standard_normal((nchan, 2, nfft)) + 1j * rng.standard_normal((nchan, 2, nfft))).astype(np.complex64)
+    ref = orc.convolve(x.astype(np.complex128), h.astype(np.complex128), nfft, 100, 100)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    ctx = b2.Context(0, streams[0].cuda_stream)
+    c = b2.Convolution(ctx, nchan, 2, nfft, 100, 100)
+    c.copy_response(h)
+    d = torch.from_numpy(x.view(np.float32)).cuda()
+    out = torch.zeros((nchan, 2, nfft - 200), dtype=torch.complex64, device="cuda")
+    busy = torch.zeros(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        for _ in range(20):
+            busy.add_(1.0)
+    c.set_fft_precision(b2.FFT_BF16X3)
+    ctx.set_stream(streams[1].cuda_stream)
+    assert c.perform(d, nfft, nfft, out, nfft - 200) == 1
+    torch.cuda.synchronize()
+    assert rel_rms(out.cpu().numpy(), ref) < VOLTAGE_RTOL
+    c.close()
+    ctx.close()
+
+
 def test_captured_calls_survive_a_change_of_the_arithmetic(b2, orc):
     """Graphs captured with one row length replay rightly after the engine has
     changed to the other, also with a response set in between."""
