@@ -31,6 +31,17 @@ int* dspsr_b200_wait_words::take ()
   std::lock_guard<std::mutex> g (lock);
   if (spare.empty ())
   {
+    // room for every word in both lists first: nothing below throws
+    try
+    {
+      pages.reserve (pages.size () + 1);
+      spare.reserve ((pages.size () + 1) * PER_PAGE);
+      used.reserve ((pages.size () + 1) * PER_PAGE);
+    }
+    catch (const std::bad_alloc&)
+    {
+      return nullptr;
+    }
     int* page = nullptr;
     if (cudaHostAlloc (&page, PER_PAGE * sizeof (int), cudaHostAllocMapped) != cudaSuccess)
       return nullptr;
@@ -2194,8 +2205,17 @@ int dspsr_b200_context_create (int device, void* stream, dspsr_b200_context** ou
     return DSPSR_B200_ENODEV;
   if (device < 0 || device >= ndev) return DSPSR_B200_EINVAL;
   if (cudaSetDevice (device) != cudaSuccess) return DSPSR_B200_ECUDA;
-  dspsr_b200_context* ctx = new (std::nothrow) dspsr_b200_context;
-  if (!ctx) return DSPSR_B200_ENOMEM;
+  dspsr_b200_context* ctx = nullptr;
+  try
+  {
+    ctx = new dspsr_b200_context;
+    ctx->waits = std::make_shared<dspsr_b200_wait_words> ();
+  }
+  catch (const std::bad_alloc&)
+  {
+    delete ctx;
+    return DSPSR_B200_ENOMEM;
+  }
   ctx->device = device;
   ctx->stream = static_cast<cudaStream_t> (stream);
   if (cudaMalloc (&ctx->d_lut, 256 * sizeof (float)) != cudaSuccess)

@@ -34,7 +34,7 @@ struct dspsr_b200_context
   float* d_lut = nullptr;     // scratch LUT for the standalone unpacker
   float2* d_fb_tab = nullptr; // pass tables of the standalone filterbank's FFT
   unsigned fb_tab_n = 0;      // ... for this transform length
-  std::shared_ptr<dspsr_b200_wait_words> waits = std::make_shared<dspsr_b200_wait_words> ();
+  std::shared_ptr<dspsr_b200_wait_words> waits;
 };
 
 struct dspsr_b200_rfi_proposer;
